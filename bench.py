@@ -68,10 +68,9 @@ FLOPS_STEP1 = 25.0
 FLOPS_LEAP = 26.0
 FLOPS_STEP2 = 8.0
 FLOPS_DIRECT = 8.0  # FP64 direct Mandelbrot step
-# Double-double Burning Ship step, CPU profile (csrc/ap_dd.cuh with the Dekker
-# product): two squares (2 x 26), |Z|^2 (1), dd_sub (14), dd_mul of |zx|,|zy| (27),
-# doubling (2), dd_add (14), dd_sub (14)                                           -> 124
-FLOPS_DD_SHIP = 124.0
+# Double-double Burning Ship step (dd_quad_orbit of csrc/ap_dd.cuh, a fused multiply-add as 2):
+# 2 z_x, 2 z_y (2), two squares (2 x 8), the product (10), three sums (3 x 11)        -> 61
+FLOPS_DD_SHIP = 61.0
 # FloatExp perturbation step (FP64 mantissa): the FP64-delta step (25) plus the
 # exponent-scaled Z terms and the renormalisation test (10)                          -> 35
 FLOPS_STEP1_FEXP = 35.0

@@ -17,7 +17,7 @@ namespace ap {
 // one long-lived pixel of a 16 x 16 tile.
 constexpr int kTile = 8;
 
-template <int TIER, int ARITH>
+template <int TIER, int ARITH, bool MULTI>
 __device__ __forceinline__ SampleOut sample_at(const ApFrameParams& p, const ApFrameBuffers& b,
                                                double sub_i, double sub_j) {
     if constexpr (TIER == AP_TIER_FP64) {
@@ -31,7 +31,7 @@ __device__ __forceinline__ SampleOut sample_at(const ApFrameParams& p, const ApF
         }
         return fp64_sample<ARITH>(x, y, p);
     } else if constexpr (TIER == AP_TIER_DD) {
-        return dd_sample_at<ARITH>(p, sub_i, sub_j);
+        return dd_sample_at<ARITH, MULTI>(p, sub_i, sub_j);
     } else if constexpr (TIER == AP_TIER_PERTURB) {
         return perturb_sample_at<ARITH>(p, b, sub_i, sub_j);
     } else {
@@ -43,7 +43,7 @@ __device__ __forceinline__ SampleOut sample_at(const ApFrameParams& p, const ApF
 //   (math_core/cuda_kernels.py:1615-1917);
 // hist_resolve = 1: ssaa_resolve_hist_*_kernel semantics
 //   (math_core/cuda_kernels.py:2038-2234).
-template <int TIER, int ARITH>
+template <int TIER, int ARITH, bool MULTI>
 __global__ void __launch_bounds__(kTile * kTile) render_pass_kernel(const ApFrameParams p,
                                                           const ApFrameBuffers b,
                                                           const int hist_resolve) {
@@ -65,7 +65,7 @@ __global__ void __launch_bounds__(kTile * kTile) render_pass_kernel(const ApFram
 
     if (mode == AP_MODE_COARSE) {
         const double sub_offset = ((double)f - 1.0) * 0.5;
-        const SampleOut o = sample_at<TIER, ARITH>(p, b, (double)(i * f) + sub_offset,
+        const SampleOut o = sample_at<TIER, ARITH, MULTI>(p, b, (double)(i * f) + sub_offset,
                                                    (double)(j * f) + sub_offset);
         b.iter_map[idx] = o.s;
         if (b.kmap) b.kmap[idx] = o.k;
@@ -88,7 +88,7 @@ __global__ void __launch_bounds__(kTile * kTile) render_pass_kernel(const ApFram
     for (int sy = 0; sy < f; ++sy) {
         for (int sx = 0; sx < f; ++sx) {
             const SampleOut o =
-                sample_at<TIER, ARITH>(p, b, (double)(i * f + sx), (double)(j * f + sy));
+                sample_at<TIER, ARITH, MULTI>(p, b, (double)(i * f + sx), (double)(j * f + sy));
             last = o;
             iters += o.iters;
             leaps += o.leaps;
@@ -122,7 +122,10 @@ template <int TIER, int ARITH>
 static int launch_pass(const ApFrameParams& p, const ApFrameBuffers& b, int hist_resolve,
                        cudaStream_t st) {
     dim3 grid((p.width + kTile - 1) / kTile, (p.height + kTile - 1) / kTile);
-    render_pass_kernel<TIER, ARITH><<<grid, kTile * kTile, 0, st>>>(p, b, hist_resolve);
+    if (TIER == AP_TIER_DD && p.fractal_type == 4)
+        render_pass_kernel<TIER, ARITH, TIER == AP_TIER_DD><<<grid, kTile * kTile, 0, st>>>(p, b, hist_resolve);
+    else
+        render_pass_kernel<TIER, ARITH, false><<<grid, kTile * kTile, 0, st>>>(p, b, hist_resolve);
     return check_launch("render_pass_kernel");
 }
 

@@ -184,7 +184,8 @@ __global__ void __launch_bounds__(kStrictThreads) strict_eval_kernel(
     if (r < 0 || r >= p.height || c < 0 || c >= p.width) return;
     float s;
     if (v.tier == AP_STRICT_DD) {
-        s = dd_sample_at<AP_ARITH_REF_CUDA>(p, (double)c, (double)r).s;
+        s = p.fractal_type == 4 ? dd_sample_at<AP_ARITH_REF_CUDA, true>(p, (double)c, (double)r).s
+                                : dd_sample_at<AP_ARITH_REF_CUDA, false>(p, (double)c, (double)r).s;
     } else if (v.tier == AP_STRICT_FP64) {
         const double x = p.x_min_hi + (double)c * p.dx_hi;
         const double y = p.y_max_hi - (double)r * p.dy_hi;
