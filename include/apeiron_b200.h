@@ -121,7 +121,8 @@ typedef struct ApFrameBuffers {
     double* s64;               /* optional [H, W]: smooth value in float64, -1 = interior */
     int32_t* counters;         /* optional [H, W, 4]: work done for the pixel by this pass, summed
                                   over its sub-samples: [0] iterations stepped one at a time
-                                  (direct tiers; perturbation stage 1), [1] BLA leaps taken,
+                                  (direct tiers; perturbation stage 1; those of an orbit found to
+                                  repeat for ever are not run and not counted), [1] BLA leaps taken,
                                   [2] perturbation stage-2 (direct) steps, [3] rebases
                                   (AP_FLAG_REBASE coarse passes on packed inputs; otherwise zero).  16-byte aligned;
                                   written only for pixels the pass evaluates. */
