@@ -54,13 +54,15 @@ inline __device__ ApFrameBuffers tile_buffers(const ApTileDesc* t) {
 // A stage-2 pixel keeps z itself where a stage-1 pixel keeps its delta; a one-pass
 // pixel keeps its reference index m where a single-reference pixel keeps the step
 // at which it entered stage 2.  The finished sample is not kept: a pixel that has
-// not finished holds the interior sample.  64 bytes a slot (32 KiB for 512 slots).
+// not finished holds the interior sample.  64 bytes a slot, and 28 of the FP64 forms'
+// cycle detection (46 KiB for 512 slots).
 struct BatchSlots {
     double zx[kBatchThreads], zy[kBatchThreads];
     double dcx[kBatchThreads], dcy[kBatchThreads];
     int idx[kBatchThreads], k[kBatchThreads], k0[kBatchThreads], k2m[kBatchThreads];
     int leaps[kBatchThreads], skipped[kBatchThreads], rebases[kBatchThreads];
     int tag[kBatchThreads];  // tile << 3 | stage << 1 | glitch
+    CycleStore<kBatchThreads> cycles;
 };
 
 __device__ __forceinline__ void slot_store(BatchSlots& S, int q, const PixelRun& s, int tile, bool rebase) {
@@ -77,6 +79,7 @@ __device__ __forceinline__ void slot_store(BatchSlots& S, int q, const PixelRun&
     S.skipped[q] = s.skipped;
     S.rebases[q] = s.rebases;
     S.tag[q] = (tile << 3) | (s.stage << 1) | (s.glitch ? 1 : 0);
+    S.cycles.visits[q] = 0;
 }
 
 // What a round reads: everything but the pixel index and its first step, which only
@@ -127,9 +130,9 @@ __device__ __noinline__ bool slot_run(const ApTileDesc* __restrict__ t, BatchSlo
     PixelRun s;
     slot_load_run(S, q, s, REBASE);
     if (REBASE)
-        rebase_advance<ARITH, FT, BLA, true>(t->p, b, s, quantum);
+        rebase_advance<ARITH, FT, BLA, true>(t->p, b, s, quantum, S.cycles, q);
     else
-        pixel_advance<ARITH, FT, BLA, true>(t->p, b, s, quantum);
+        pixel_advance<ARITH, FT, BLA, true>(t->p, b, s, quantum, S.cycles, q);
     if (s.stage == 3) {
         s.idx = S.idx[q];
         s.k0 = S.k0[q];
@@ -356,18 +359,22 @@ __global__ void __launch_bounds__(kBatchThreads, MINB * 256 / kBatchThreads) bat
             pos += (w < warp) ? warp_live[w] : 0;
             now += warp_live[w];
         }
-        double zx = 0.0, zy = 0.0, dcx = 0.0, dcy = 0.0;
-        int w0 = 0, w1 = 0, w2 = 0, w3 = 0, w4 = 0, w5 = 0, w6 = 0, w7 = 0;
+        double zx = 0.0, zy = 0.0, dcx = 0.0, dcy = 0.0, cyx = 0.0, cyy = 0.0;
+        int w0 = 0, w1 = 0, w2 = 0, w3 = 0, w4 = 0, w5 = 0, w6 = 0, w7 = 0, w8 = 0, w9 = 0, w10 = 0;
         if (running) {
             zx = S.zx[tid], zy = S.zy[tid], dcx = S.dcx[tid], dcy = S.dcy[tid];
             w0 = S.idx[tid], w1 = S.k[tid], w2 = S.k0[tid], w3 = S.k2m[tid];
             w4 = S.leaps[tid], w5 = S.skipped[tid], w6 = S.rebases[tid], w7 = S.tag[tid];
+            cyx = S.cycles.x[tid], cyy = S.cycles.y[tid];
+            w8 = S.cycles.k[tid], w9 = S.cycles.m[tid], w10 = S.cycles.visits[tid];
         }
         __syncthreads();
         if (running && pos != tid) {
             S.zx[pos] = zx, S.zy[pos] = zy, S.dcx[pos] = dcx, S.dcy[pos] = dcy;
             S.idx[pos] = w0, S.k[pos] = w1, S.k0[pos] = w2, S.k2m[pos] = w3;
             S.leaps[pos] = w4, S.skipped[pos] = w5, S.rebases[pos] = w6, S.tag[pos] = w7;
+            S.cycles.x[pos] = cyx, S.cycles.y[pos] = cyy;
+            S.cycles.k[pos] = w8, S.cycles.m[pos] = w9, S.cycles.visits[pos] = w10;
         }
         if (tid == 0) {
             live_s = now;

@@ -6,10 +6,62 @@
 
 namespace ap {
 
+// The periodic tail of an orbit of n values, for the kernels' cycle detection: the smallest
+// period p <= 4095 with Z_k = Z_{k-p} (bit for bit up to the sign of a zero) for every k from
+// s0 + p to n - 2, the tail holding at least two periods and 64 steps; returned as 4096 s0 + p,
+// 0 when there is none.  One block.  An orbit that escaped has none (its last value tells, at
+// the cost of one load); the search compares 8 values per candidate and walks the tail of a
+// bounded reference once.
+constexpr int kTailMaxPeriod = 4095;
+__device__ double find_orbit_tail(const double* __restrict__ re, const double* __restrict__ im, int n) {
+    __shared__ int period_s, start_s;
+    const int last = n - 2;  // the record at n - 1 is the orbit's end, never a step
+    const double ex = re[n - 1], ey = im[n - 1];
+    if (last < 128 || !(ex * ex + ey * ey <= kBailout)) return 0.0;
+    const int t = threadIdx.x;
+    if (t == 0) period_s = kTailMaxPeriod + 1;
+    __syncthreads();
+    for (int p0 = 1; p0 <= kTailMaxPeriod; p0 += blockDim.x) {
+        const int p = p0 + t;
+        bool same = p <= kTailMaxPeriod && 2 * (long long)p < last;
+        for (int j = 0; j < 8 && same; ++j) {
+            const int k = last - j;
+            same = k - p >= 0 && re[k] == re[k - p] && im[k] == im[k - p];
+        }
+        if (same) atomicMin(&period_s, p);
+        __syncthreads();
+        const bool found = period_s <= kTailMaxPeriod;
+        __syncthreads();
+        if (found) break;
+    }
+    const int p = period_s;
+    if (p > kTailMaxPeriod) return 0.0;
+    if (t == 0) start_s = -1;
+    __syncthreads();
+    // the largest k with Z_k != Z_{k-p}, chunks of 4 values a thread from the end
+    for (int hi = last; hi >= p; hi -= 4 * blockDim.x) {
+        int bad = -1;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int k = hi - j * (int)blockDim.x - t;
+            if (k >= p && !(re[k] == re[k - p] && im[k] == im[k - p])) bad = max(bad, k);
+        }
+        if (bad >= 0) atomicMax(&start_s, bad);
+        __syncthreads();
+        const bool found = start_s >= 0;
+        __syncthreads();
+        if (found) break;
+    }
+    const int s0 = start_s < 0 ? 0 : start_s + 1 - p;
+    return last - s0 >= max(2 * p, 64) ? 4096.0 * (double)s0 + (double)p : 0.0;
+}
+
 __global__ void __launch_bounds__(256) pack_orbit_kernel(const double* __restrict__ re,
                                                          const double* __restrict__ im, int n,
                                                          double4* __restrict__ out) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    // the last block (it writes the last record) also looks for the orbit's periodic tail
+    const double tail = blockIdx.x == gridDim.x - 1 ? find_orbit_tail(re, im, n) : 0.0;
     if (k >= n) return;
     const double rx = re[k], ry = im[k];
     const double r_mag2 = rx * rx + ry * ry;
@@ -25,8 +77,9 @@ __global__ void __launch_bounds__(256) pack_orbit_kernel(const double* __restric
     s = fmin(s, rz * (1.0 - 1e-12) * 0.5 * (1.0 - 1e-7));
     s = s > 0.0 ? s : 0.0;
     if (k == n - 1) s = 0.0;  // the orbit's end is never a safe step (the rebase kernels rely on it)
-    // slot 3: the level-0 BLA radius, written by ap_pack_bla (0: no leap)
-    out[k] = make_double4(rx, ry, s * s * (1.0 - 1e-12), 0.0);
+    // slot 3: the level-0 BLA radius, written by ap_pack_bla (0: no leap); in the last record,
+    // which no leap starts from, the negated periodic tail
+    out[k] = make_double4(rx, ry, s * s * (1.0 - 1e-12), k == n - 1 ? -tail : 0.0);
 }
 
 __global__ void __launch_bounds__(256) pack_bla_kernel(const double* __restrict__ T, int levels,

@@ -28,7 +28,8 @@ __global__ void __launch_bounds__(kCoarseThreads, (REBASE ? AP_REBASE_MIN_BLOCKS
     const int i = blockIdx.x * kCoarseTile + (w % kWarpsPerRow) * 8 + (l & 7);
     const int j = row0 + blockIdx.y * kCoarseTile + (w / kWarpsPerRow) * 4 + (l >> 3);
     if (i >= p.width || j >= row_end) return;
-    coarse_pixel<ARITH, FT, BLA, REBASE>(p, b, i, j);
+    __shared__ CycleStore<kCoarseThreads> cycles;
+    coarse_pixel<ARITH, FT, BLA, REBASE>(p, b, i, j, cycles, threadIdx.x);
 }
 
 template <int ARITH, int FT>
