@@ -292,7 +292,11 @@ __device__ __noinline__ bool slot_begin(const ApTileDesc* __restrict__ t, int ti
 }
 
 // Pixel u of the batch (patches of 256 pixels, numbered tile after tile; row-major in a
-// patch) -> its tile and its (i, j); false when it falls outside the tile.
+// patch) -> its tile and its (i, j); false when it falls outside the tile.  Within a tile the
+// queue runs through the groups of 32 pixels in a scattered order (a multiplier coprime to
+// their number): the long-lived pixels of a tile lie together, and blocks that took them as
+// they lie kept a few SMs busy long after the others had run out of work (one 504x504 Multibrot
+// n = 5 tile 18.7 ms, 12.2 scattered).
 __device__ __forceinline__ bool batch_pixel_at(const ApTileDesc* __restrict__ tiles,
                                                const int64_t* __restrict__ first, int n, int patch_w,
                                                int patch_h, long long u, int* tile, int* i, int* j) {
@@ -306,11 +310,35 @@ __device__ __forceinline__ bool batch_pixel_at(const ApTileDesc* __restrict__ ti
     }
     *tile = lo;
     const ApTileDesc* t = tiles + lo;
-    const long long local = item - first[lo];
+    const long long patches = first[lo + 1] - first[lo];
+    const unsigned groups = (unsigned)(patches * 8);  // below 2^31 (a tile has fewer than 2^31 pixels)
+    unsigned g = (unsigned)((item - first[lo]) * 8) + (unsigned)(q >> 5);
+    if (patches % 7919) g = (unsigned)(g * 7919ull % groups);  // 7919 is an odd prime
+    const long long local = g >> 3;
+    const int w = (int)(g & 7) * 32 + (q & 31);
     const int px = (t->p.width + patch_w - 1) / patch_w;
-    *i = (int)(local % px) * patch_w + q % patch_w;
-    *j = (int)(local / px) * patch_h + q / patch_w;
+    *i = (int)(local % px) * patch_w + w % patch_w;
+    *j = (int)(local / px) * patch_h + w / patch_w;
     return *i < t->p.width && *j < t->p.height;
+}
+
+// The variant a pixel of tile t runs (what batch_run dispatches on), 0..7, as the key that
+// keeps the pixels of one variant together when they are compacted.
+__device__ __forceinline__ int batch_class(const ApTileDesc* t) {
+    const int ft = t->p.fractal_type;
+    const int formula = ft == 4 ? 2 : (ft & 1);
+    return formula + (t->p.tier == AP_TIER_FLOATEXP32 ? 3 : 0);
+}
+constexpr int kBatchClasses = 6;
+
+// Loop steps of a round for tile t: `quantum` of the dearest step (Multibrot n = 5, 58 FP64
+// operations), more of a cheaper one, so that the warps of a block, which wait for one
+// another at the end of a round, take about as long whatever they run (21 mixed tiles 42.6 ->
+// 35.5 ms; blocks of 64, 128 and 256 threads 46, 41 and 36 ms).
+__device__ __forceinline__ int batch_quantum(const ApTileDesc* t, int quantum) {
+    const int ft = t->p.fractal_type;
+    const int cost = ft == 4 ? max(12, min(58, 12 * t->p.gen_n - 2)) : (ft & 1) ? 16 : 12;
+    return quantum * 58 / cost;
 }
 
 template <int ARITH, int MINB>
@@ -320,8 +348,8 @@ __global__ void __launch_bounds__(kBatchThreads, MINB * 256 / kBatchThreads) bat
                                                                     int quantum,
                                                                     unsigned long long* head) {
     __shared__ BatchSlots S;
-    __shared__ int warp_live[kBatchThreads / 32];
-    __shared__ int live_s, drained_s;
+    __shared__ int class_live[kBatchClasses][kBatchThreads / 32];
+    __shared__ int live_s, drained_s, want_s;
     __shared__ unsigned long long base_s;
     const unsigned full = 0xffffffffu;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -335,29 +363,46 @@ __global__ void __launch_bounds__(kBatchThreads, MINB * 256 / kBatchThreads) bat
         // the slots past the live pixels take the next pixels of the queue
         const int live = live_s;
         const bool take = !drained_s && live < kBatchThreads;
-        if (tid == 0 && take) base_s = atomicAdd(head, (unsigned long long)(kBatchThreads - live));
+        if (tid == 0 && take) {
+            // all free slots while the queue is long; towards its end an even share of what is
+            // left, in whole warps, so that the last pixels spread over every block
+            const unsigned long long seen = *(volatile unsigned long long*)head;
+            const unsigned long long left = seen < (unsigned long long)total ? (unsigned long long)total - seen : 0;
+            const unsigned long long share = (left / gridDim.x + 31) / 32 * 32;
+            want_s = (int)min((unsigned long long)(kBatchThreads - live), max(share, 32ull));
+            base_s = atomicAdd(head, (unsigned long long)want_s);
+        }
         __syncthreads();
         bool running = false;
         int tile = 0;
         if (tid < live) {
             tile = S.tag[tid] >> 3;
             running = true;
-        } else if (take) {
+        } else if (take && tid < live + want_s) {
             const long long u = (long long)base_s + (tid - live);
             int i = 0, j = 0;
             if (u < total && batch_pixel_at(tiles, first, n, patch_w, patch_h, u, &tile, &i, &j))
                 running = slot_begin<ARITH>(tiles + tile, tile, S, tid, i, j);
         }
-        if (running) running = batch_run<ARITH>(tiles + tile, S, tid, quantum);
-        // compact the unfinished pixels into the first slots, in order
-        const unsigned bal = __ballot_sync(full, running);
-        if (lane == 0) warp_live[warp] = __popc(bal);
-        __syncthreads();
-        int pos = __popc(bal & ((1u << lane) - 1u)), now = 0;
+        if (running) running = batch_run<ARITH>(tiles + tile, S, tid, batch_quantum(tiles + tile, quantum));
+        // compact the unfinished pixels into the first slots, by variant and in order within
+        // one: a warp whose lanes run different variants runs them one after the other
+        const int cls = running ? batch_class(tiles + tile) : -1;
+        int pos = 0;
 #pragma unroll
-        for (int w = 0; w < kBatchThreads / 32; ++w) {
-            pos += (w < warp) ? warp_live[w] : 0;
-            now += warp_live[w];
+        for (int c = 0; c < kBatchClasses; ++c) {
+            const unsigned bal = __ballot_sync(full, cls == c);
+            if (lane == 0) class_live[c][warp] = __popc(bal);
+            if (cls == c) pos = __popc(bal & ((1u << lane) - 1u));
+        }
+        __syncthreads();
+        int now = 0;
+#pragma unroll 1
+        for (int c = 0; c < kBatchClasses; ++c) {
+            int mine = lane < kBatchThreads / 32 ? class_live[c][lane] : 0;
+            const int before = __reduce_add_sync(full, lane < warp ? mine : 0);
+            if (cls == c) pos += now + before;
+            now += __reduce_add_sync(full, mine);
         }
         double zx = 0.0, zy = 0.0, dcx = 0.0, dcy = 0.0, cyx = 0.0, cyy = 0.0;
         int w0 = 0, w1 = 0, w2 = 0, w3 = 0, w4 = 0, w5 = 0, w6 = 0, w7 = 0, w8 = 0, w9 = 0, w10 = 0;
@@ -378,7 +423,7 @@ __global__ void __launch_bounds__(kBatchThreads, MINB * 256 / kBatchThreads) bat
         }
         if (tid == 0) {
             live_s = now;
-            if (take && base_s + (unsigned long long)(kBatchThreads - live) >= (unsigned long long)total)
+            if (take && base_s + (unsigned long long)want_s >= (unsigned long long)total)
                 drained_s = 1;
         }
         __syncthreads();
@@ -463,7 +508,7 @@ extern "C" int ap_render_batch(const ApTileDesc* tiles, const int64_t* first_pat
         ap::set_error("ap_render_batch: memset: %s", cudaGetErrorString(e));
         return AP_E_CUDA;
     }
-    const int grid = sms * blocks_per_sm;
+    const int grid = sms * blocks_per_sm * (512 / ap::kBatchThreads);  // blocks_per_sm counts 512 threads
 #define AP_BATCH_LAUNCH(A, M)                                                                              \
     ap::batch_kernel<A, M><<<grid, ap::kBatchThreads, 0, st>>>(tiles, first_patch, n, patch_w, patch_h, \
                                                                quantum, queue_head)
