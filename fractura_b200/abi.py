@@ -33,6 +33,7 @@ AP_FLAG_ITER_LAST_SUB = 8
 AP_FLAG_MAP_FUSED = 16
 AP_FLAG_HIST_COLOUR = 32
 AP_FLAG_REBASE = 64
+AP_FLAG_SPANS = 128
 
 
 class ApFrameParams(C.Structure):

@@ -149,7 +149,7 @@ def _tile_inputs(t, ref, arith, bla_form, torch, stream, L, scratch):
     """Packed records, BLA rows, outputs and parameters of one tile around its
     reference `ref` (find_optimal_reference_orbit's result), as the coarse pass of
     render_perturbation_frame sets them (factor 1, one reference)."""
-    from .perturbation import max_delta_c
+    from .perturbation import max_delta_c, spans_allowed
     cpu_sem = arith == "ref_cpu"
     fp32 = t.delta_form == "fp32"
     pw = Decimal(t.width)
@@ -200,6 +200,8 @@ def _tile_inputs(t, ref, arith, bla_form, torch, stream, L, scratch):
         raise NotImplementedError("one-pass rebasing serves Mandelbrot, Burning Ship and Multibrot tiles")
     if rebase:
         flags |= abi.AP_FLAG_REBASE
+    if use_bla and spans_allowed(t.fractal_type, ACCURATE_BLA_EPS if bla_form == "accurate" else float(t.bla_tol)):
+        flags |= abi.AP_FLAG_SPANS
     p = abi.new_params(width=t.W, height=t.H, factor=1, max_iter=int(t.max_iter),
                        fractal_type=int(t.fractal_type),
                        tier=abi.AP_TIER_FLOATEXP32 if fp32 else abi.AP_TIER_PERTURB,

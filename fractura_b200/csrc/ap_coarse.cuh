@@ -18,6 +18,7 @@
 #pragma once
 
 #include "ap_common.cuh"
+#include "ap_fp64.cuh"
 
 namespace ap {
 
@@ -39,11 +40,22 @@ __device__ __forceinline__ void for_powers(int n, F&& power) {
     }
 }
 
-// 32-byte record through the read-only path (two 16-byte loads).
+// |Z + dz| - |Z| of one component, given z = Z + dz and a = 2 Z + dz (each rounded): the
+// reference's s dz where z keeps the sign s of Z and -s a where it does not.  s is Z's sign bit,
+// so the test and the products by s = +-1 are integer operations on the high words (they were
+// 5 of the 12 FP64-pipe operations a component took).  z = 0 passes for either sign: then
+// dz = -Z and a = Z, and both forms give s dz.
+__device__ __forceinline__ double fold_delta(double Z, double z, double dz, double a) {
+    const int s = __double2hiint(Z);
+    const double v = (__double2hiint(z) ^ s) >= 0 ? dz : -a;
+    return __hiloint2double(__double2hiint(v) ^ (s & 0x80000000), __double2loint(v));
+}
+
+// 32-byte record (32-byte aligned) through the read-only path, as one 256-bit load.
 __device__ __forceinline__ double4 ldg4(const double4* p) {
-    const double2* q = reinterpret_cast<const double2*>(p);
-    const double2 a = __ldg(q), c = __ldg(q + 1);
-    return make_double4(a.x, a.y, c.x, c.y);
+    double4 r;
+    asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(r.x), "=d"(r.y), "=d"(r.z), "=d"(r.w) : "l"(p));
+    return r;
 }
 
 // Cycle detection.  A bounded pixel mostly settles on an exact cycle: its state returns bit for
@@ -89,7 +101,7 @@ template <int N>
 __device__ __forceinline__ int cycle_visit(CycleStore<N>& C, int q, double x, double y, int k, int m) {
     const int visits = C.visits[q];
     if (visits > 0 && C.x[q] == x && C.y[q] == y) {
-        const int km = C.k[q], mm = C.m[q];
+        const int km = C.k[q], mm = C.m[q];  // m = -1: z itself, past the reference (stage 2)
         if (m == mm || (m > 0 && mm > 0 && m - mm == k - km)) return k - km;
     }
     if ((visits & (visits - 1)) == 0) {
@@ -170,10 +182,153 @@ __device__ __forceinline__ bool pixel_begin(const ApFrameParams& p, const ApFram
     return true;
 }
 
+// The largest admissible level of a leap: the levels whose radius covers |dz| are a prefix
+// 0..lo (radii never increase with the level), so lo is a count.  Two rounds of three
+// independent loads: the quarter of the row, then the level in it.
+__device__ __forceinline__ int leap_level(const double* __restrict__ row, double dz_mag2, int hi) {
+    int quarter = 0;
+#pragma unroll
+    for (int t = 1; t <= 3; ++t) quarter += (4 * t <= hi && dz_mag2 < __ldg(row + 4 * t)) ? 1 : 0;
+    int lo = 4 * quarter;
+#pragma unroll
+    for (int t = 1; t <= 3; ++t) {
+        const int d = 4 * quarter + t;
+        lo += (d <= hi && dz_mag2 < __ldg(row + d)) ? 1 : 0;
+    }
+    return lo;
+}
+
+__device__ __forceinline__ bool not_finite(double v) {
+    return (__double2hiint(v) & 0x7ff00000) == 0x7ff00000;
+}
+
+// A leap dz <- A dz + B dc.
+template <bool CPU>
+__device__ __forceinline__ void leap_delta(const double4 e, double& dzx, double& dzy, double dcx, double dcy) {
+    double nx, ny;
+    if (CPU) {
+        nx = (e.x * dzx - e.y * dzy) + (e.z * dcx - e.w * dcy);
+        ny = (e.x * dzy + e.y * dzx) + (e.z * dcy + e.w * dcx);
+    } else {
+        nx = fma(e.x, dzx, fma(-e.y, dzy, fma(e.z, dcx, -e.w * dcy)));
+        ny = fma(e.x, dzy, fma(e.y, dzx, fma(e.z, dcy, e.w * dcx)));
+    }
+    dzx = nx;
+    dzy = ny;
+}
+
+// One step of the delta at the orbit value (rx, ry), in the profile's operations.
+template <int ARITH, int FT>
+__device__ __forceinline__ void delta_step(const ApFrameParams& p, double rx, double ry, double& dzx, double& dzy,
+                                           double dcx, double dcy) {
+    constexpr bool kCpu = (ARITH == AP_ARITH_REF_CPU);
+    constexpr bool kFast = (ARITH == AP_ARITH_FAST);
+    if (FT == kFtQuad) {
+        double nx, ny;
+        if (kFast) {  // (2Z + dz) dz + dc with a = 2Z + dz rounded once
+            const double ax = fma(2.0, rx, dzx), ay = fma(2.0, ry, dzy);
+            nx = fma(ax, dzx, fma(-ay, dzy, dcx));
+            ny = fma(ax, dzy, fma(ay, dzx, dcy));
+        } else if (kCpu) {
+            nx = (2.0 * rx + dzx) * dzx - (2.0 * ry + dzy) * dzy + dcx;
+            ny = 2.0 * ((rx + dzx) * dzy + ry * dzx) + dcy;
+        } else {
+            nx = fma(2.0 * rx + dzx, dzx, fma(-(2.0 * ry + dzy), dzy, dcx));
+            ny = fma(2.0, fma(rx + dzx, dzy, ry * dzx), dcy);
+        }
+        dzx = nx;
+        dzy = ny;
+    } else if (FT == kFtShip) {
+        const double zx = rx + dzx, zy = ry + dzy;
+        if (kFast) {  // 2Z + dz rounded once (2Z is exact); products fused into the sums
+            const double ax = fma(2.0, rx, dzx), ay = fma(2.0, ry, dzy);
+            const double nx = fma(ax, dzx, fma(-ay, dzy, dcx));
+            const double ddx = fold_delta(rx, zx, dzx, ax), ddy = fold_delta(ry, zy, dzy, ay);
+            dzy = fma(2.0, fma(fabs(rx), ddy, fma(fabs(ry), ddx, ddx * ddy)), -dcy);
+            dzx = nx;
+        } else {
+            const double ax = 2.0 * rx + dzx, ay = 2.0 * ry + dzy;
+            const double nx = ax * dzx - ay * dzy + dcx;
+            const double ddx = fold_delta(rx, zx, dzx, ax), ddy = fold_delta(ry, zy, dzy, ay);
+            dzy = 2.0 * (fabs(rx) * ddy + fabs(ry) * ddx + ddx * ddy) - dcy;
+            dzx = nx;
+        }
+    } else if (kFast) {
+        // (Z + dz)^n - Z^n by P_{j+1} = P_j Z + (P_j + Z^j) dz, each complex product
+        // sum as one chain of fused multiply-adds, then + k dz + dc
+        double pr = dzx, pi = dzy, qr = rx, qi = ry;
+        for_powers(p.gen_n, [&]() {
+            const double sr = pr + qr, si = pi + qi;
+            const double npr = fma(pr, rx, fma(-pi, ry, fma(sr, dzx, -si * dzy)));
+            const double npi = fma(pr, ry, fma(pi, rx, fma(sr, dzy, si * dzx)));
+            const double nqr = fma(qr, rx, -qi * ry), nqi = fma(qr, ry, qi * rx);
+            pr = npr;
+            pi = npi;
+            qr = nqr;
+            qi = nqi;
+        });
+        const double ox = dzx, oy = dzy;
+        dzx = fma(p.gen_kr, ox, fma(-p.gen_ki, oy, pr + dcx));
+        dzy = fma(p.gen_kr, oy, fma(p.gen_ki, ox, pi + dcy));
+    } else {
+        double pr = dzx, pi = dzy, qr = rx, qi = ry;
+        for_powers(p.gen_n, [&]() {
+            const double t1r = pr * rx - pi * ry, t1i = pr * ry + pi * rx;
+            const double sr = pr + qr, si = pi + qi;
+            const double t2r = sr * dzx - si * dzy, t2i = sr * dzy + si * dzx;
+            pr = t1r + t2r;
+            pi = t1i + t2i;
+            const double nqr = qr * rx - qi * ry, nqi = qr * ry + qi * rx;
+            qr = nqr;
+            qi = nqi;
+        });
+        const double kzr = p.gen_kr * dzx - p.gen_ki * dzy;
+        const double kzi = p.gen_kr * dzy + p.gen_ki * dzx;
+        dzx = pr + kzr + dcx;
+        dzy = pi + kzi + dcy;
+    }
+}
+
+// Whether the kSpan steps from here on are plain (ap_pack.cu's orbit_window, the low word of the
+// record's third slot): |dz|^2's exponent in the record's window, and |dc|^2's at least 60 below it
+// (dc_exp60: that exponent plus 60; a |dc|^2 that underflows has exponent 0, and is covered; no
+// exponent reaches 4096, which turns spans off).
+template <bool BLA>
+__device__ __forceinline__ bool span_fits(int dz_mag2_hi, const double4 rec, int dc_exp60) {
+    const int e = dz_mag2_hi >> 20, w = __double2loint(rec.z);
+    return e < (w & 0xffff) && e >= dc_exp60 && (!BLA || e >= (__double2hiint(rec.w) >> 20) + (w >> 16));
+}
+
+// kSpan steps from record `rec` on without a test: 7 instructions a step where a tested one takes
+// about 28.  Lanes that do not fit wait for those that do; taking a span only where most lanes fit
+// measured slower (1920x1080 Mandelbrot at 1e-160, one-pass rebasing, a frame: 1.58 ms without
+// spans, 1.50 with, 1.67 with that vote), and the Burning Ship, whose lanes disagree more, loses
+// (a 167x167 tile at depth 65541 18.8 ms without spans, 28 with): it takes none.
+template <int ARITH, int FT>
+__device__ __forceinline__ void span_steps(const ApFrameParams& p, const double4* __restrict__ rec, double& dzx,
+                                           double& dzy, double dcx, double dcy) {
+#pragma unroll
+    for (int j = 0; j < kSpan; ++j) {
+        const double2 Z = __ldg(reinterpret_cast<const double2*>(rec + j));
+        delta_step<ARITH, FT>(p, Z.x, Z.y, dzx, dzy, dcx, dcy);
+    }
+}
+
+// What a lane does at the end of a loop iteration.  The loops below decide it in the branches of
+// their tests and act on it afterwards.  For Multibrot, whose step is 30 to 60 FP64 operations,
+// the decision goes through value_barrier, so that all lanes that step do so together: with the
+// branches threaded to their ends (a jump from a test to the loop's head) the lanes that passed a
+// test and those that skipped it ran the step one after the other, and a step's FP64 instructions
+// were issued 1.7 times (a 399x399 tile with n = 4: 8.0 ms, 5.9 with the barrier).  The cheaper
+// steps lose more by the barrier than by that (a 1920x1080 Mandelbrot view 1.58 -> 1.78 ms).
+enum { kActStep = 0, kActMoved = 1, kActEscaped = 2, kActNotFinite = 3 };
+__device__ __forceinline__ void value_barrier(int& v) { asm volatile("" : "+r"(v)); }
+
 template <int ARITH, int FT, bool BLA, bool BUDGET, int N>
 __device__ __forceinline__ void pixel_advance(const ApFrameParams& p, const ApFrameBuffers& b, PixelRun& s,
                                               int budget, CycleStore<N>& C, int q) {
     constexpr bool kCpu = (ARITH == AP_ARITH_REF_CPU);
+    constexpr bool kMerge = (FT == kFtMulti);
     const bool julia = (p.fractal_type == 2 || p.fractal_type == 3);
     const int ref_len = p.ref_len, max_iter = p.max_iter;
     const double4* __restrict__ orb = reinterpret_cast<const double4*>(b.orbit_packed);
@@ -190,7 +345,11 @@ __device__ __forceinline__ void pixel_advance(const ApFrameParams& p, const ApFr
         const double4* __restrict__ AB =
             reinterpret_cast<const double4*>(b.bla_packed + (size_t)ref_len * 16);
         const int max_level = p.bla_levels - 1;
-        bool finished = false, paused = false;
+        bool paused = false;
+        int act = kActStep;
+        double esc_mag2 = 0.0;
+        const int dc_exp60 = BLA && !(p.flags & AP_FLAG_SPANS)
+                                 ? 4096 : (__double2hiint(dcpx * dcpx + dcpy * dcpy) >> 20) + 60;
         // the loop runs to `bound`: the orbit's end, or the next visited step of its tail
         // (past step 15, from which on the Pauldelbrot test looks at every step)
         int bound = min(ref_len, max(k, max(16, orbit_tail(orb, ref_len).s0)));
@@ -209,7 +368,6 @@ __device__ __forceinline__ void pixel_advance(const ApFrameParams& p, const ApFr
                     gap = tail_gap(C, q, tail, k, true);
                 }
                 bound = gap < ref_len - k ? k + gap : ref_len;
-                continue;
             }
             if (BUDGET && --budget < 0) {
                 paused = true;
@@ -217,107 +375,56 @@ __device__ __forceinline__ void pixel_advance(const ApFrameParams& p, const ApFr
             }
             const double4 Z = ldg4(orb + k);
             const double rx = Z.x, ry = Z.y;
-            const double zx = rx + dzx, zy = ry + dzy;
             const double dz_mag2 = dzx * dzx + dzy * dzy;
+            const int dz_hi = __double2hiint(dz_mag2);
+            if (FT == kFtQuad && k + kSpan <= bound && span_fits<BLA>(dz_hi, Z, dc_exp60)) {
+                span_steps<ARITH, FT>(p, orb + k, dzx, dzy, dcpx, dcpy);
+                k += kSpan;
+                if (BUDGET) budget -= kSpan - 1;
+                continue;
+            }
             // One branch on the common path: inside the safe radius (no test can fire)
             // and outside the level-0 BLA radius (no leap), the step runs straight
             // through.  The packed radii are 0 wherever k + 2^d >= ref_len, so no level
             // is admissible at the last step without a separate bound check.
-            const bool unsafe = !(dz_mag2 < Z.z);
+            const bool unsafe = dz_hi >= __double2hiint(Z.z);
             const bool leap = BLA && (dz_mag2 < Z.w);
+            act = kActStep;
             if (unsafe || leap) {
                 if (unsafe) {
+                    const double zx = rx + dzx, zy = ry + dzy;
                     const double mag2 = zx * zx + zy * zy;
                     const double r_mag2 = rx * rx + ry * ry;
                     if (mag2 > kBailout) {
                         if (esc_glitch && strict && k > 15 && r_mag2 < 4.0) glitch = 1;
-                        o = escaped_sample(k, mag2, inv_ln);
-                        finished = true;
-                        break;
+                        esc_mag2 = mag2;
+                        act = kActEscaped;
+                    } else {
+                        // the Pauldelbrot threshold, as the reference forms it
+                        const double thr = r_mag2 > 1e-8 ? 1e-6 * r_mag2 : -1.0;
+                        if (strict && k > 15 && mag2 < thr) glitch = 1;
                     }
-                    // the Pauldelbrot threshold, as the reference forms it
-                    const double thr = r_mag2 > 1e-8 ? 1e-6 * r_mag2 : -1.0;
-                    if (strict && k > 15 && mag2 < thr) glitch = 1;
                 }
-                if (leap) {
-                    const double* row = R + (size_t)k * 16;
+                if (leap && act == kActStep) {
                     int hi = max_level;
                     if (dz_mag2 == 0.0 && (dzx != 0.0 || dzy != 0.0)) hi = min(hi, 8);
-                    // The admissible levels are a prefix 0..lo (radii never increase
-                    // with the level), so lo is a count.  Two rounds of three
-                    // independent loads: the quarter of the row, then the level in it.
-                    int quarter = 0;
-#pragma unroll
-                    for (int t = 1; t <= 3; ++t)
-                        quarter += (4 * t <= hi && dz_mag2 < __ldg(row + 4 * t)) ? 1 : 0;
-                    int lo = 4 * quarter;
-#pragma unroll
-                    for (int t = 1; t <= 3; ++t) {
-                        const int d = 4 * quarter + t;
-                        lo += (d <= hi && dz_mag2 < __ldg(row + d)) ? 1 : 0;
+                    const int lo = leap_level(R + (size_t)k * 16, dz_mag2, hi);
+                    leap_delta<kCpu>(ldg4(AB + (size_t)k * 16 + lo), dzx, dzy, dcpx, dcpy);
+                    act = kActNotFinite;
+                    if (!not_finite(dzx) && !not_finite(dzy)) {
+                        act = kActMoved;
+                        k += 1 << lo;
+                        ++leaps;
+                        skipped += 1 << lo;
                     }
-                    const double4 e = ldg4(AB + (size_t)k * 16 + lo);
-                    double nx, ny;
-                    if (kCpu) {
-                        nx = (e.x * dzx - e.y * dzy) + (e.z * dcpx - e.w * dcpy);
-                        ny = (e.x * dzy + e.y * dzx) + (e.z * dcpy + e.w * dcpx);
-                    } else {
-                        nx = fma(e.x, dzx, fma(-e.y, dzy, fma(e.z, dcpx, -e.w * dcpy)));
-                        ny = fma(e.x, dzy, fma(e.y, dzx, fma(e.z, dcpy, e.w * dcpx)));
-                    }
-                    dzx = nx;
-                    dzy = ny;
-                    if (isnan(dzx) || isnan(dzy) || isinf(dzx) || isinf(dzy)) {
-                        o = interior_sample();
-                        o.s = (float)k;
-                        o.s64 = (double)k;
-                        o.k = k;
-                        glitch = 1;
-                        finished = true;
-                        break;
-                    }
-                    k += 1 << lo;
-                    ++leaps;
-                    skipped += 1 << lo;
-                    continue;
                 }
             }
-            if (FT == kFtQuad) {
-                double nx, ny;
-                if (kCpu) {
-                    nx = (2.0 * rx + dzx) * dzx - (2.0 * ry + dzy) * dzy + dcpx;
-                    ny = 2.0 * (zx * dzy + ry * dzx) + dcpy;
-                } else {
-                    nx = fma(2.0 * rx + dzx, dzx, fma(-(2.0 * ry + dzy), dzy, dcpx));
-                    ny = fma(2.0, fma(zx, dzy, ry * dzx), dcpy);
-                }
-                dzx = nx;
-                dzy = ny;
-            } else if (FT == kFtShip) {
-                const double nx = (2.0 * rx + dzx) * dzx - (2.0 * ry + dzy) * dzy + dcpx;
-                const double sx = rx >= 0.0 ? 1.0 : -1.0, sy = ry >= 0.0 ? 1.0 : -1.0;
-                const double ddx = zx * sx >= 0.0 ? sx * dzx : -sx * (2.0 * rx + dzx);
-                const double ddy = zy * sy >= 0.0 ? sy * dzy : -sy * (2.0 * ry + dzy);
-                dzy = 2.0 * (fabs(rx) * ddy + fabs(ry) * ddx + ddx * ddy) - dcpy;
-                dzx = nx;
-            } else {
-                double pr = dzx, pi = dzy, qr = rx, qi = ry;
-                for_powers(p.gen_n, [&]() {
-                    const double t1r = pr * rx - pi * ry, t1i = pr * ry + pi * rx;
-                    const double sr = pr + qr, si = pi + qi;
-                    const double t2r = sr * dzx - si * dzy, t2i = sr * dzy + si * dzx;
-                    pr = t1r + t2r;
-                    pi = t1i + t2i;
-                    const double nqr = qr * rx - qi * ry, nqi = qr * ry + qi * rx;
-                    qr = nqr;
-                    qi = nqi;
-                });
-                const double kzr = p.gen_kr * dzx - p.gen_ki * dzy;
-                const double kzi = p.gen_kr * dzy + p.gen_ki * dzx;
-                dzx = pr + kzr + dcpx;
-                dzy = pi + kzi + dcpy;
+            if (kMerge) value_barrier(act);
+            if (act >= kActEscaped) break;
+            if (act == kActStep) {
+                delta_step<ARITH, FT>(p, rx, ry, dzx, dzy, dcpx, dcpy);
+                ++k;
             }
-            ++k;
         }
         if (paused) {
             s.dzx = dzx;
@@ -328,7 +435,16 @@ __device__ __forceinline__ void pixel_advance(const ApFrameParams& p, const ApFr
             s.skipped = skipped;
             return;
         }
-        if (finished) {
+        if (act >= kActEscaped) {
+            if (act == kActEscaped) {
+                o = escaped_sample(k, esc_mag2, inv_ln);
+            } else {
+                o = interior_sample();
+                o.s = (float)k;
+                o.s64 = (double)k;
+                o.k = k;
+                glitch = 1;
+            }
             s.stage = 3;
         } else {
             // Stage 2: past the end of the reference orbit, iterate z directly.
@@ -348,11 +464,38 @@ __device__ __forceinline__ void pixel_advance(const ApFrameParams& p, const ApFr
         const double cy = julia ? p.julia_cy_hi : p.ref_cy + s.dcy;
         const bool nan_guard = (p.flags & AP_FLAG_NAN_GUARD) != 0;
         bool paused = false;
+        constexpr int kKind = FT == kFtQuad ? kKindQuad : FT == kFtShip ? kKindShip : kKindMulti;
+        const bool growing = fp64_growing(kKind, cx, cy, p.gen_n, p.gen_kr, p.gen_ki);
+        int tested = 0;  // steps to test one by one before the next block
         while (k < max_iter) {
             if (BUDGET && --budget < 0) {
                 paused = true;
                 break;
             }
+            // blocks tested at their end only, as in direct iteration (fp64_orbit, ap_fp64.cuh)
+            if (growing && tested == 0 && k + kBlock <= max_iter) {
+                const double bx = zx, by = zy;
+                for_degree(kKind, p.gen_n, [&](auto n) {
+#pragma unroll
+                    for (int t = 0; t < kBlock; ++t)
+                        fp64_step<AP_ARITH_REF_CUDA, kKind, n()>(zx, zy, zx * zx, zy * zy, cx, cy, p.gen_n, p.gen_kr,
+                                                                 p.gen_ki);
+                });
+                if (zx * zx + zy * zy <= kBailout) {
+                    k += kBlock;
+                    if (BUDGET) budget -= kBlock - 1;
+                    if (cycle_visit(C, q, zx, zy, k, -1) > 0) {  // it repeats: never escapes
+                        s.k2 += max_iter - k;
+                        skipped += max_iter - k;
+                        k = max_iter;
+                    }
+                    continue;
+                }
+                zx = bx;
+                zy = by;
+                tested = kBlock + 1;
+            }
+            if (tested > 0) --tested;
             const double zx2 = zx * zx, zy2 = zy * zy;
             const double mag2 = zx2 + zy2;
             if (nan_guard && (isnan(mag2) || isinf(mag2))) {
@@ -415,9 +558,9 @@ __device__ __forceinline__ void rebase_advance(const ApFrameParams& p, const ApF
                                                int budget, CycleStore<N>& C, int q) {
     constexpr bool kCpu = (ARITH == AP_ARITH_REF_CPU);
     constexpr bool kFast = (ARITH == AP_ARITH_FAST);
+    constexpr bool kMerge = (FT == kFtMulti);
     const int ref_len = p.ref_len, max_iter = p.max_iter;
     const double4* __restrict__ orb = reinterpret_cast<const double4*>(b.orbit_packed);
-    const double inv_ln = inv_ln_for(p.fractal_type, p.gen_n);
     const double* __restrict__ R = b.bla_packed;
     const double4* __restrict__ AB = reinterpret_cast<const double4*>(b.bla_packed + (size_t)ref_len * 16);
     const int max_level = p.bla_levels - 1;
@@ -426,10 +569,17 @@ __device__ __forceinline__ void rebase_advance(const ApFrameParams& p, const ApF
     // restart moves only m, so k = m + (max_iter - lim) with lim moved at each restart,
     // and the loop runs while m < lim (k < max_iter).
     int m = s.m, lim = max_iter - s.k + s.m;
-    int glitch = s.glitch, leaps = s.leaps, skipped = s.skipped, rebases = s.rebases;
+    int leaps = s.leaps, skipped = s.skipped, rebases = s.rebases;
     double dzx = s.dzx, dzy = s.dzy;
-    SampleOut o = s.o;
     bool paused = false;
+    int act = kActStep;
+    double esc_mag2 = 0.0;
+    const int dc_exp60 = BLA && !(p.flags & AP_FLAG_SPANS)
+                             ? 4096 : (__double2hiint(dcpx * dcpx + dcpy * dcpy) >> 20) + 60;
+    // A restart at an orbit that starts at 0, without a leap there, needs no test at m = 0: z = dz
+    // has just been tested.  It goes straight to the step.
+    const double4 Zstart = ldg4(orb);
+    const bool zero_start = Zstart.x == 0.0 && Zstart.y == 0.0 && !(Zstart.w > 0.0);
     // the loop runs to `bound`: lim, or the next visited step of the reference's tail
     const int tail_s0 = max(1, orbit_tail(orb, ref_len).s0);
     int bound = min(lim, max(m, tail_s0));
@@ -454,49 +604,40 @@ __device__ __forceinline__ void rebase_advance(const ApFrameParams& p, const ApF
                 gap = tail_gap(C, q, tail, m, true);
             }
             bound = gap < lim - m ? m + gap : lim;
-            continue;
+            if (m >= lim) break;
         }
         if (BUDGET && --budget < 0) {
             paused = true;
             break;
         }
         const double4 Z = ldg4(orb + m);
-        const double rx = Z.x, ry = Z.y;
-        // z itself: every step but the fused Mandelbrot one uses it; that one forms it
-        // only where a test can fire
-        constexpr bool kLateZ = kFast && FT == kFtQuad;
-        double zx = 0.0, zy = 0.0;
-        if (!kLateZ) {
-            zx = rx + dzx;
-            zy = ry + dzy;
-        }
+        double rx = Z.x, ry = Z.y;
         const double dz_mag2 = kFast ? fma(dzx, dzx, dzy * dzy) : dzx * dzx + dzy * dzy;
+        const int dz_hi = __double2hiint(dz_mag2);
+        if (FT == kFtQuad && m + kSpan <= bound && span_fits<BLA>(dz_hi, Z, dc_exp60)) {
+            span_steps<ARITH, FT>(p, orb + m, dzx, dzy, dcpx, dcpy);
+            m += kSpan;
+            if (BUDGET) budget -= kSpan - 1;
+            continue;
+        }
         // ap_pack_orbit leaves the orbit's last record (m == ref_len) with safe radius 0,
         // so the end of the reference takes this branch without a test of its own
-        const bool unsafe = !(dz_mag2 < Z.z);
+        const bool unsafe = dz_hi >= __double2hiint(Z.z);
         const bool leap = BLA && (dz_mag2 < Z.w);
+        act = kActStep;
         if (unsafe || leap) {
+            bool may_leap = leap;
             if (unsafe) {
-                if (kLateZ) {
-                    zx = rx + dzx;
-                    zy = ry + dzy;
-                }
+                const double zx = rx + dzx, zy = ry + dzy;
                 const double mag2 = kFast ? fma(zx, zx, zy * zy) : zx * zx + zy * zy;
-                if (!(mag2 <= kBailout)) {
-                    const int k = m + (max_iter - lim);
-                    if (isnan(mag2)) {
-                        o = interior_sample();
-                        o.s = (float)k;
-                        o.s64 = (double)k;
-                        o.k = k;
-                        glitch = 1;
-                    } else {
-                        o = escaped_sample(k, mag2, inv_ln);
-                    }
-                    s.stage = 3;
-                    break;
-                }
-                if (mag2 < dz_mag2 || (m == ref_len && m > 0)) {
+                // high words decide most: neither test fires where |z|^2's lies above |dz|^2's
+                // and below the bailout's (NaN lies above it)
+                const int mag_hi = __double2hiint(mag2);
+                if (mag_hi > dz_hi && mag_hi < 0x40f00000 && m != ref_len) {
+                } else if (!(mag2 <= kBailout)) {
+                    esc_mag2 = mag2;
+                    act = kActEscaped;
+                } else if (mag2 < dz_mag2 || (m == ref_len && m > 0)) {
                     dzx = zx;
                     dzy = zy;
                     lim -= m;
@@ -509,128 +650,54 @@ __device__ __forceinline__ void rebase_advance(const ApFrameParams& p, const ApF
                         skipped += jump;
                     }
                     bound = min(lim, tail_s0);
-                    continue;
+                    act = zero_start && lim > 0 ? kActStep : kActMoved;
+                    rx = 0.0;
+                    ry = 0.0;
+                    may_leap = false;
                 }
             }
-            if (leap) {
-                const double* row = R + (size_t)m * 16;
+            if (may_leap && act == kActStep) {
                 int hi = max_level;
                 if (dz_mag2 == 0.0 && (dzx != 0.0 || dzy != 0.0)) hi = min(hi, 8);
                 hi = min(hi, 31 - __clz(lim - m));  // k + 2^lo <= max_iter
-                int quarter = 0;
-#pragma unroll
-                for (int t = 1; t <= 3; ++t)
-                    quarter += (4 * t <= hi && dz_mag2 < __ldg(row + 4 * t)) ? 1 : 0;
-                int lo = 4 * quarter;
-#pragma unroll
-                for (int t = 1; t <= 3; ++t) {
-                    const int d = 4 * quarter + t;
-                    lo += (d <= hi && dz_mag2 < __ldg(row + d)) ? 1 : 0;
+                const int lo = leap_level(R + (size_t)m * 16, dz_mag2, hi);
+                leap_delta<kCpu>(ldg4(AB + (size_t)m * 16 + lo), dzx, dzy, dcpx, dcpy);
+                act = kActNotFinite;
+                if (!not_finite(dzx) && !not_finite(dzy)) {
+                    act = kActMoved;
+                    m += 1 << lo;
+                    ++leaps;
+                    skipped += 1 << lo;
                 }
-                const double4 e = ldg4(AB + (size_t)m * 16 + lo);
-                double nx, ny;
-                if (kCpu) {
-                    nx = (e.x * dzx - e.y * dzy) + (e.z * dcpx - e.w * dcpy);
-                    ny = (e.x * dzy + e.y * dzx) + (e.z * dcpy + e.w * dcpx);
-                } else {
-                    nx = fma(e.x, dzx, fma(-e.y, dzy, fma(e.z, dcpx, -e.w * dcpy)));
-                    ny = fma(e.x, dzy, fma(e.y, dzx, fma(e.z, dcpy, e.w * dcpx)));
-                }
-                dzx = nx;
-                dzy = ny;
-                if (isnan(dzx) || isnan(dzy) || isinf(dzx) || isinf(dzy)) {
-                    const int k = m + (max_iter - lim);
-                    o = interior_sample();
-                    o.s = (float)k;
-                    o.s64 = (double)k;
-                    o.k = k;
-                    glitch = 1;
-                    s.stage = 3;
-                    break;
-                }
-                m += 1 << lo;
-                ++leaps;
-                skipped += 1 << lo;
-                continue;
             }
         }
-        if (FT == kFtQuad) {
-            double nx, ny;
-            if (kFast) {  // (2Z + dz) dz + dc with a = 2Z + dz rounded once
-                const double ax = fma(2.0, rx, dzx), ay = fma(2.0, ry, dzy);
-                nx = fma(ax, dzx, fma(-ay, dzy, dcpx));
-                ny = fma(ax, dzy, fma(ay, dzx, dcpy));
-            } else if (kCpu) {
-                nx = (2.0 * rx + dzx) * dzx - (2.0 * ry + dzy) * dzy + dcpx;
-                ny = 2.0 * (zx * dzy + ry * dzx) + dcpy;
-            } else {
-                nx = fma(2.0 * rx + dzx, dzx, fma(-(2.0 * ry + dzy), dzy, dcpx));
-                ny = fma(2.0, fma(zx, dzy, ry * dzx), dcpy);
-            }
-            dzx = nx;
-            dzy = ny;
-        } else if (FT == kFtShip) {
-            const double sx = rx >= 0.0 ? 1.0 : -1.0, sy = ry >= 0.0 ? 1.0 : -1.0;
-            if (kFast) {  // 2Z + dz rounded once (2Z is exact); products fused into the sums
-                const double ax = fma(2.0, rx, dzx), ay = fma(2.0, ry, dzy);
-                const double nx = fma(ax, dzx, fma(-ay, dzy, dcpx));
-                const double ddx = zx * sx >= 0.0 ? sx * dzx : -sx * ax;
-                const double ddy = zy * sy >= 0.0 ? sy * dzy : -sy * ay;
-                dzy = fma(2.0, fma(fabs(rx), ddy, fma(fabs(ry), ddx, ddx * ddy)), -dcpy);
-                dzx = nx;
-            } else {
-                const double nx = (2.0 * rx + dzx) * dzx - (2.0 * ry + dzy) * dzy + dcpx;
-                const double ddx = zx * sx >= 0.0 ? sx * dzx : -sx * (2.0 * rx + dzx);
-                const double ddy = zy * sy >= 0.0 ? sy * dzy : -sy * (2.0 * ry + dzy);
-                dzy = 2.0 * (fabs(rx) * ddy + fabs(ry) * ddx + ddx * ddy) - dcpy;
-                dzx = nx;
-            }
-        } else if (kFast) {
-            // (Z + dz)^n - Z^n by P_{j+1} = P_j Z + (P_j + Z^j) dz, each complex product
-            // sum as one chain of fused multiply-adds, then + k dz + dc
-            double pr = dzx, pi = dzy, qr = rx, qi = ry;
-            for_powers(p.gen_n, [&]() {
-                const double sr = pr + qr, si = pi + qi;
-                const double npr = fma(pr, rx, fma(-pi, ry, fma(sr, dzx, -si * dzy)));
-                const double npi = fma(pr, ry, fma(pi, rx, fma(sr, dzy, si * dzx)));
-                const double nqr = fma(qr, rx, -qi * ry), nqi = fma(qr, ry, qi * rx);
-                pr = npr;
-                pi = npi;
-                qr = nqr;
-                qi = nqi;
-            });
-            const double ox = dzx, oy = dzy;
-            dzx = fma(p.gen_kr, ox, fma(-p.gen_ki, oy, pr + dcpx));
-            dzy = fma(p.gen_kr, oy, fma(p.gen_ki, ox, pi + dcpy));
-        } else {
-            double pr = dzx, pi = dzy, qr = rx, qi = ry;
-            for_powers(p.gen_n, [&]() {
-                const double t1r = pr * rx - pi * ry, t1i = pr * ry + pi * rx;
-                const double sr = pr + qr, si = pi + qi;
-                const double t2r = sr * dzx - si * dzy, t2i = sr * dzy + si * dzx;
-                pr = t1r + t2r;
-                pi = t1i + t2i;
-                const double nqr = qr * rx - qi * ry, nqi = qr * ry + qi * rx;
-                qr = nqr;
-                qi = nqi;
-            });
-            const double kzr = p.gen_kr * dzx - p.gen_ki * dzy;
-            const double kzi = p.gen_kr * dzy + p.gen_ki * dzx;
-            dzx = pr + kzr + dcpx;
-            dzy = pi + kzi + dcpy;
+        if (kMerge) value_barrier(act);
+        if (act >= kActEscaped) break;
+        if (act == kActStep) {
+            delta_step<ARITH, FT>(p, rx, ry, dzx, dzy, dcpx, dcpy);
+            ++m;
         }
-        ++m;
     }
-    if (!paused) s.stage = 3;
+    const int k = m + (max_iter - lim);
+    if (!paused) {
+        s.stage = 3;
+        if (act == kActEscaped && !isnan(esc_mag2)) {
+            s.o = escaped_sample(k, esc_mag2, inv_ln_for(p.fractal_type, p.gen_n));
+        } else if (act >= kActEscaped) {
+            s.o = interior_sample();
+            s.o.s = (float)k;
+            s.o.s64 = (double)k;
+            s.o.k = k;
+            s.glitch = 1;
+        }
+    }
     s.dzx = dzx;
     s.dzy = dzy;
-    s.k = m + (max_iter - lim);
+    s.k = k;
     s.m = m;
-    s.glitch = glitch;
     s.leaps = leaps;
     s.skipped = skipped;
     s.rebases = rebases;
-    s.o = o;
 }
 
 __device__ __forceinline__ void pixel_finish(const ApFrameParams& p, const ApFrameBuffers& b, const PixelRun& s) {

@@ -93,6 +93,10 @@ __host__ __device__ __forceinline__ double inv_ln_for(int fractal_type, int gen_
     return kInvLn2;
 }
 
+// Steps of a span: consecutive steps of a packed orbit that the coarse kernels take without a
+// test where the delta lies in the window stored in the record (orbit_window, ap_pack.cu).
+constexpr int kSpan = 8;
+
 // ---------------------------------------------------------------- colouring
 // Transfer functions of math_core/cuda_kernels.py:157-259, evaluated in
 // float64 on the float32 smooth value.

@@ -14,6 +14,23 @@ namespace ap {
 
 constexpr int kKindQuad = 0, kKindShip = 1, kKindMulti = 4;
 
+// Calls f with the Multibrot degree as a compile-time constant for 2..5, else (and for the
+// quadratic kinds) with 0.
+template <int N>
+struct Degree {
+    __host__ __device__ constexpr int operator()() const { return N; }
+};
+template <typename F>
+__device__ __forceinline__ void for_degree(int kind, int n, F&& f) {
+    switch (kind == kKindMulti ? n : 0) {
+    case 2: f(Degree<2>()); break;
+    case 3: f(Degree<3>()); break;
+    case 4: f(Degree<4>()); break;
+    case 5: f(Degree<5>()); break;
+    default: f(Degree<0>());
+    }
+}
+
 // One step of z in the profile's operations; zx2, zy2 the squares (quadratic kinds).  N: the
 // Multibrot degree where it is known at compile time (2..5, the powers unrolled), else 0.
 template <int ARITH, int KIND, int N>
@@ -80,6 +97,12 @@ __device__ __forceinline__ double fp64_mag2(double zx, double zy) {
 // 1283x721 Julia frame with 2x SSAA 772 us, blocks of 16 take 726; leads of 4, 8 and 16 time alike.
 constexpr int kLead = 8;
 constexpr int kBlock = 16;
+
+// Whether an orbit that has passed the bailout keeps growing (see fp64_orbit).
+__device__ __forceinline__ bool fp64_growing(int kind, double cx, double cy, int n, double kr, double ki) {
+    return fabs(cx) <= 1000.0 && fabs(cy) <= 1000.0 &&
+           (kind != kKindMulti || (n >= 2 && fabs(kr) <= 100.0 && fabs(ki) <= 100.0));
+}
 
 // The orbit of z: escape step and |z|^2 as testing every step gives them.  A step's test is on the
 // step's dependent chain (square, add, compare, branch) and takes two of its FP64 operations, so
@@ -169,26 +192,18 @@ __device__ __forceinline__ SampleOut fp64_sample(double x, double y, const ApFra
     const double cx = julia ? p.julia_cx_hi : x, cy = julia ? p.julia_cy_hi : y;
     const int n = p.gen_n;
     const double kr = p.gen_kr, ki = p.gen_ki;
-    bool growing = fabs(cx) <= 1000.0 && fabs(cy) <= 1000.0;
-    if (ft == 4) growing = growing && n >= 2 && fabs(kr) <= 100.0 && fabs(ki) <= 100.0;
+    const bool growing = fp64_growing(ft == 4 ? kKindMulti : kKindQuad, cx, cy, n, kr, ki);
     double mag2 = 0.0;
     int steps = 0, k;
-#define AP_FP64_ORBIT(KIND, N) \
-    fp64_orbit<ARITH, KIND, N>(zx, zy, cx, cy, p.max_iter, growing, n, kr, ki, mag2, steps)
     if (ft == 4) {
-        switch (n) {
-        case 2: k = AP_FP64_ORBIT(kKindMulti, 2); break;
-        case 3: k = AP_FP64_ORBIT(kKindMulti, 3); break;
-        case 4: k = AP_FP64_ORBIT(kKindMulti, 4); break;
-        case 5: k = AP_FP64_ORBIT(kKindMulti, 5); break;
-        default: k = AP_FP64_ORBIT(kKindMulti, 0);
-        }
+        for_degree(kKindMulti, n, [&](auto degree) {
+            k = fp64_orbit<ARITH, kKindMulti, degree()>(zx, zy, cx, cy, p.max_iter, growing, n, kr, ki, mag2, steps);
+        });
     } else if (ft & 1) {
-        k = AP_FP64_ORBIT(kKindShip, 0);
+        k = fp64_orbit<ARITH, kKindShip, 0>(zx, zy, cx, cy, p.max_iter, growing, n, kr, ki, mag2, steps);
     } else {
-        k = AP_FP64_ORBIT(kKindQuad, 0);
+        k = fp64_orbit<ARITH, kKindQuad, 0>(zx, zy, cx, cy, p.max_iter, growing, n, kr, ki, mag2, steps);
     }
-#undef AP_FP64_ORBIT
     if (k >= 0) return escaped_sample(k, mag2, inv_ln_for(ft, n));
     return interior_after(steps);
 }

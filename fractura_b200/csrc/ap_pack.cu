@@ -6,6 +6,41 @@
 
 namespace ap {
 
+// The radius below which no test of a step at |Z| = rz can fire (see pack_orbit_kernel).
+__device__ __forceinline__ double safe_radius(double rz) {
+    const double s = fmin(256.0 * (1.0 - 1e-12) - rz * (1.0 + 1e-12), rz * (1.0 - 1e-12) * 0.5 * (1.0 - 1e-7));
+    return s > 0.0 ? s : 0.0;
+}
+
+// The window of |dz| at step k in which the next kSpan steps of z^2 + c are plain: no test of
+// theirs can fire and none of them leaps.  While |dz_j| is below step j's
+// safe radius it is at most |Z_j| / 2, so
+//     1.5 |Z_j| |dz_j| - |dc|  <=  |dz_{j+1}|  <=  2.5 |Z_j| |dz_j| + |dc|
+// (|dz'| = |2 Z + dz| |dz| up to dc).  With the factors widened to 1.49 and 2.51, which cover
+// every rounding and a |dc| up to 2^-29 |dz_0| (the kernels check that) as long as the lower
+// products stay above 2^-20, the window is |dz_0| < h = min_j s_j / prod_{i<j} 2.51 |Z_i| and,
+// with leaps, |dz_0| >= max_j r_j / prod_{i<j} 1.49 |Z_i|.  The level-0 radii r_j of ap_build_bla
+// and ap_build_bla_dc are proportional to |Z_j|, so that bound is r_k times a number of the orbit
+// alone.  Kept: h^2's biased exponent (0: no window) and, above it, two more than the exponent of
+// that number squared, which the kernels add to r_k^2's.
+__device__ __forceinline__ unsigned orbit_window(const double* __restrict__ re, const double* __restrict__ im, int k,
+                                                 int n) {
+    if (k == 0 || k + kSpan >= n) return 0u;  // step 0 may have radius 0 next to 0
+    double up = 1.0, down = 1.0, h = 256.0, l = 0.0, rk = 0.0;
+    for (int j = 0; j < kSpan; ++j) {
+        const double rz = sqrt(re[k + j] * re[k + j] + im[k + j] * im[k + j]);
+        if (j == 0) rk = rz;
+        if (!(down >= 0x1p-20) || !(rk > 0.0)) return 0u;
+        h = fmin(h, safe_radius(rz) / (up * (1.0 + 1e-9)));
+        l = fmax(l, rz / rk * (1.0 + 1e-9) / down);
+        up *= 2.51 * rz;
+        down *= 1.49 * rz;
+    }
+    const unsigned end = (unsigned)__double2hiint(h * h) >> 20;
+    const unsigned first = ((unsigned)__double2hiint(l * l) >> 20) - 1023u + 2u;  // l >= 1
+    return end > 0u && first < 0x8000u ? (first << 16) | end : 0u;
+}
+
 // The periodic tail of an orbit of n values, for the kernels' cycle detection: the smallest
 // period p <= 4095 with Z_k = Z_{k-p} (bit for bit up to the sign of a zero) for every k from
 // s0 + p to n - 2, the tail holding at least two periods and 64 steps; returned as 4096 s0 + p,
@@ -72,14 +107,15 @@ __global__ void __launch_bounds__(256) pack_orbit_kernel(const double* __restric
     // and 1e-6 |Z|^2 < s^2 covers the Pauldelbrot threshold.  The 1e-12 margins
     // cover the roundings of |Z|, of Z + dz and of the squares.  Stored as
     // s^2 (1 - 1e-12) to be compared with the rounded |dz|^2.
-    const double rz = sqrt(r_mag2);
-    double s = 256.0 * (1.0 - 1e-12) - rz * (1.0 + 1e-12);
-    s = fmin(s, rz * (1.0 - 1e-12) * 0.5 * (1.0 - 1e-7));
-    s = s > 0.0 ? s : 0.0;
+    // The kernels compare high words (one unit down: a delta just below the radius takes the tests
+    // too); the low word holds the record's span window.
+    double s = safe_radius(sqrt(r_mag2));
     if (k == n - 1) s = 0.0;  // the orbit's end is never a safe step (the rebase kernels rely on it)
+    const int safe_hi = __double2hiint(s * s * (1.0 - 1e-12)) - 1;
+    const double safe = safe_hi > 0 ? __hiloint2double(safe_hi, (int)orbit_window(re, im, k, n)) : 0.0;
     // slot 3: the level-0 BLA radius, written by ap_pack_bla (0: no leap); in the last record,
     // which no leap starts from, the negated periodic tail
-    out[k] = make_double4(rx, ry, s * s * (1.0 - 1e-12), k == n - 1 ? -tail : 0.0);
+    out[k] = make_double4(rx, ry, safe, k == n - 1 ? -tail : 0.0);
 }
 
 __global__ void __launch_bounds__(256) pack_bla_kernel(const double* __restrict__ T, int levels,

@@ -214,6 +214,11 @@ def max_delta_c(ref_px, ref_py, w_sub, h_sub, dx, dy):
     return float(np.hypot(ex, ey)) * (1.0 + 1e-6)
 
 
+def spans_allowed(fractal_type, tol):
+    """Whether AP_FLAG_SPANS holds for a table built at ``tol``: z^2 + c, radii below their cap."""
+    return fractal_type in (0, 2) and 0.0 < tol <= 1e-4
+
+
 def _pack_orbit(L, d_re, d_im, ref_len, slot, tag, stream_h):
     from .engine import get_scratch_device_array_1d
     n = 6 * (ref_len + 1)  # FP64 records, then the FP32 copy of the FP32 FloatExp tier
@@ -413,6 +418,8 @@ def render_perturbation_frame(p, fr, lut, stream_h, st, *, W, H, factor, max_ite
     # BLA variant (NaN guard), their histogram resolve passes the plain one (escape glitch).
     unified_flags = (abi.AP_FLAG_ESCAPE_GLITCH | abi.AP_FLAG_NAN_GUARD) if cpu_sem else abi.AP_FLAG_NAN_GUARD
     resolve_flags = (abi.AP_FLAG_ESCAPE_GLITCH | abi.AP_FLAG_NAN_GUARD) if cpu_sem else abi.AP_FLAG_ESCAPE_GLITCH
+    if use_bla and spans_allowed(fractal_type, bbsa_tol if bla_eps is None else bla_eps):
+        unified_flags |= abi.AP_FLAG_SPANS
     if one_pass:
         unified_flags |= abi.AP_FLAG_REBASE
         resolve_flags |= abi.AP_FLAG_REBASE

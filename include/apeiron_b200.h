@@ -70,6 +70,12 @@ extern "C" {
  * m <- 0 (Zhuoran, fractalforums.org 2021).  No pixel is flagged glitched (only a
  * NaN/Inf delta is), there is no direct-iteration stage, and rebase_pass must be 0. */
 #define AP_FLAG_REBASE 64u
+/* The packed BLA table's level-0 radii are those of ap_build_bla or ap_build_bla_dc for z^2 + c at
+ * a tolerance up to 1e-4: r^2 = 4 tol^2 |Z|^2 (0 at a first step next to 0 and past the orbit's
+ * end).  With it the FP64 coarse passes on packed inputs take runs of plain steps without a test
+ * each where the orbit records say that none could fire; passes without leaps do so anyway.
+ * Values do not depend on it. */
+#define AP_FLAG_SPANS 128u
 
 typedef struct ApFrameParams {
     int32_t width, height;     /* output pixels */
