@@ -12,6 +12,8 @@
 // the arithmetic differences are ARITH.
 #pragma once
 
+#include <climits>
+
 #include "ap_common.cuh"
 
 namespace ap {
@@ -359,6 +361,9 @@ __device__ __forceinline__ double py_max(double a, double b) { return b > a ? b 
 // (math_core/cuda_kernels.py:913-923).  The loops stop on non-finite values,
 // where some reference variants would not.
 __device__ __forceinline__ void renorm16(double& x, double& y, int& e) {
+    // in range by the high words (the usual case): max in [2^-16, 2^16)
+    const int top = max(__double2hiint(x) & 0x7fffffff, __double2hiint(y) & 0x7fffffff);
+    if (top >= 0x3ef00000 && top < 0x40f00000) return;
     double mag = py_max(fabs(x), fabs(y));
     while (mag > 65536.0 && isfinite(mag)) {
         x *= 1.52587890625e-05;
@@ -382,6 +387,10 @@ __device__ __forceinline__ bool floatexp_glitch(double rx, double ry, double dzx
     if (r_max < 1e-4) return false;
     const double dz_max = py_max(fabs(dzx), fabs(dzy));
     if (dz_max <= 0.0) return false;
+    // the logarithms below are within 1 of the binary exponents: far outside the +-10 window
+    // the exponents decide (not for subnormal or non-finite values)
+    const int re = (__double2hiint(r_max) >> 20) - 1023, de = (__double2hiint(dz_max) >> 20) - 1023;
+    if (de > -1023 && de < 1024 && re < 1024 && (re - (eff_exp + de) > 13 || re - (eff_exp + de) < -13)) return false;
     const int r_exp = (int)(log(r_max) * 1.4426950408889634);
     const int dz_exp = (int)(log(dz_max) * 1.4426950408889634);
     const int diff = r_exp - (eff_exp + dz_exp);
@@ -391,6 +400,31 @@ __device__ __forceinline__ bool floatexp_glitch(double rx, double ry, double dzx
     const double zx = rxs + dzx * scale_dz, zy = rys + dzy * scale_dz;
     return zx * zx + zy * zy < 1e-6 * (rxs * rxs + rys * rys);
 }
+
+// dz = sqrt(x^2 + y^2) 2^max(-1020, shift) against a leap radius r given as r^2: the reference's
+// test r^2 > 0 && dz < sqrt(r^2), decided by exponents where they differ.  dz lies in
+// [2^t, 2^(t+2)) for t = exponent of max(|x|, |y|) + max(-1020, shift), or below what a double holds
+// where t is; sqrt(r^2) has half r^2's exponent.  At 1e-1000 nearly every test is decided so: it was
+// two square roots a level, up to 16 levels a leap (1920x1080 there: 1.89 -> 1.44 ms a frame with
+// the packed rows' level search and the renormalisation's and glitch test's exponent screens).
+struct LinearFit {
+    double x, y;
+    int t, shift;
+    __device__ __forceinline__ LinearFit(double x_, double y_, int shift_) : x(x_), y(y_), shift(max(-1020, shift_)) {
+        const int top = max(__double2hiint(x) & 0x7fffffff, __double2hiint(y) & 0x7fffffff) >> 20;
+        // zero, subnormal or not finite: never decided by the exponent
+        t = top > 0 && top < 2047 ? top - 1023 + shift : INT_MIN;
+    }
+    __device__ __forceinline__ bool operator()(double r_sq) const {
+        const int er = __double2hiint(r_sq) >> 20;
+        if (t != INT_MIN && er > 0) {
+            const int es = (er - 1023) >> 1;
+            if (t + 2 <= es) return true;
+            if (t > es && t > -1000) return false;
+        }
+        return r_sq > 0.0 && sqrt(x * x + y * y) * pow2_f64(shift) < sqrt(r_sq);
+    }
+};
 
 // FloatExp perturbation: the true delta is (dzx, dzy) 2^(z_exp - E) with the
 // mantissa pair kept in [2^-16, 2^16]; delta_c = dc_norm 2^-E (dx/dy are the
@@ -427,6 +461,8 @@ __device__ __forceinline__ SampleOut floatexp_sample_at(const ApFrameParams& p,
     const bool has_bla = levels > 1 && b.bla != nullptr && (ft == 0 || ft == 2 || ft == 4);
     const size_t L = (size_t)ref_len;
     const double inv_ln = inv_ln_for(ft, p.gen_n);
+    // packed BLA rows (ap_pack_bla), where the pass has them
+    const double* __restrict__ rows = has_bla && levels <= 16 ? b.bla_packed : nullptr;
 
     while (k < ref_len) {
         const double rx = __ldg(re + k), ry = __ldg(im + k);
@@ -447,26 +483,43 @@ __device__ __forceinline__ SampleOut floatexp_sample_at(const ApFrameParams& p,
             // |delta|^2 against r^2 in scaled form, or via square roots far below 2^-510
             const int shift_r = eff_exp;
             const bool scaled = shift_r >= -510;
-            double dz_mag2 = 0.0, dz_lin = 0.0;
+            double dz_mag2 = 0.0;
             if (scaled) {
                 const double sr = pow2_f64(shift_r);
                 dz_mag2 = (dzx * dzx + dzy * dzy) * (sr * sr);
-            } else {
-                dz_lin = sqrt(dzx * dzx + dzy * dzy) * pow2_f64(max(-1020, shift_r));
             }
-            auto fits = [&](double r_sq) {
-                return scaled ? (dz_mag2 < r_sq) : (r_sq > 0.0 && dz_lin < sqrt(r_sq));
-            };
-            if (fits(__ldg(b.bla + (size_t)k * 5 + 4))) {
+            const LinearFit linear(dzx, dzy, shift_r);
+            auto fits = [&](double r_sq) { return scaled ? (dz_mag2 < r_sq) : linear(r_sq); };
+            const double* row = rows ? rows + (size_t)k * 16 : b.bla + (size_t)k * 5 + 4;
+            if (fits(__ldg(row))) {
                 int best = 0;
-                for (int d = levels - 1; d > 0; --d) {
-                    if (k + (1 << d) < ref_len && fits(__ldg(b.bla + ((size_t)d * L + k) * 5 + 4))) {
-                        best = d;
-                        break;
+                double ar, ai, br, bi;
+                if (rows) {
+                    // the packed radii of step k: the admissible levels are a prefix (0 past
+                    // the orbit's end), so the largest is a count, taken in two rounds
+                    const int top = levels - 1;
+                    int quarter = 0;
+#pragma unroll
+                    for (int t = 1; t <= 3; ++t) quarter += (4 * t <= top && fits(__ldg(row + 4 * t))) ? 1 : 0;
+                    best = 4 * quarter;
+#pragma unroll
+                    for (int t = 1; t <= 3; ++t) {
+                        const int d = 4 * quarter + t;
+                        best += (d <= top && fits(__ldg(row + d))) ? 1 : 0;
                     }
+                    const double2* e = reinterpret_cast<const double2*>(rows + L * 16 + ((size_t)k * 16 + best) * 4);
+                    const double2 a = __ldg(e), c = __ldg(e + 1);
+                    ar = a.x, ai = a.y, br = c.x, bi = c.y;
+                } else {
+                    for (int d = levels - 1; d > 0; --d) {
+                        if (k + (1 << d) < ref_len && fits(__ldg(b.bla + ((size_t)d * L + k) * 5 + 4))) {
+                            best = d;
+                            break;
+                        }
+                    }
+                    const double* e = b.bla + ((size_t)best * L + k) * 5;
+                    ar = __ldg(e), ai = __ldg(e + 1), br = __ldg(e + 2), bi = __ldg(e + 3);
                 }
-                const double* e = b.bla + ((size_t)best * L + k) * 5;
-                const double ar = __ldg(e), ai = __ldg(e + 1), br = __ldg(e + 2), bi = __ldg(e + 3);
                 const double scale_c = (z_exp >= -1020 && z_exp <= 1020) ? pow2_f64(-z_exp) : 0.0;
                 const double cxs = dcpx * scale_c, cys = dcpy * scale_c;
                 double nx, ny;
