@@ -358,13 +358,35 @@ __device__ __forceinline__ double pow2_f64(int e) {
 __device__ __forceinline__ double py_max(double a, double b) { return b > a ? b : a; }
 
 // Keep the mantissa pair within [2^-16, 2^16] by exact 2^16 rescaling
-// (math_core/cuda_kernels.py:913-923).  The loops stop on non-finite values,
-// where some reference variants would not.
-__device__ __forceinline__ void renorm16(double& x, double& y, int& e) {
-    // in range by the high words (the usual case): max in [2^-16, 2^16)
-    const int top = max(__double2hiint(x) & 0x7fffffff, __double2hiint(y) & 0x7fffffff);
-    if (top >= 0x3ef00000 && top < 0x40f00000) return;
+// (math_core/cuda_kernels.py:913-923).  Whether the exponent changed.  The reference rescales one
+// 2^16 at a time; a leap can be worth a dozen of them, so the number is taken from the exponent
+// (by steps only where a component would become subnormal on the way, or for values that are
+// subnormal or not finite; the loops stop on non-finite ones, where some reference variants
+// would not).
+__device__ __forceinline__ bool renorm16(double& x, double& y, int& e) {
+    const int hx = __double2hiint(x) & 0x7fffffff, hy = __double2hiint(y) & 0x7fffffff;
+    const int top = max(hx, hy);
+    if (top >= 0x3ef00000 && top < 0x40f00000) return false;  // max in [2^-16, 2^16)
+    const int et = (top >> 20) - 1023;
     double mag = py_max(fabs(x), fabs(y));
+    int n = 0;  // 2^-16 rescalings (negative: 2^16)
+    if (et >= 16) {
+        n = et >> 4;  // to below 2^16, or to 2^16 itself
+        if ((et & 15) == 0 && __double_as_longlong(mag) << 12 == 0) --n;
+    } else if (et < -16) {
+        n = -((-16 - et + 15) >> 4);
+    }
+    const int ebot = (min(hx, hy) >> 20);
+    const bool small = n > 0 && ebot - 16 * n <= 0 && x != 0.0 && y != 0.0;
+    if (et > -1023 && et < 1024 && n < 60 && n > -60 && !small) {
+        if (n == 0) return false;
+        const double f = __hiloint2double((1023 - 16 * n) << 20, 0);
+        x *= f;
+        y *= f;
+        e += 16 * n;
+        return true;
+    }
+    const int before = e;
     while (mag > 65536.0 && isfinite(mag)) {
         x *= 1.52587890625e-05;
         y *= 1.52587890625e-05;
@@ -377,6 +399,7 @@ __device__ __forceinline__ void renorm16(double& x, double& y, int& e) {
         e -= 16;
         mag = py_max(fabs(x), fabs(y));
     }
+    return e != before;
 }
 
 // Pauldelbrot test on the scaled pair (check_glitch_cancellation_floatexp,
@@ -404,9 +427,8 @@ __device__ __forceinline__ bool floatexp_glitch(double rx, double ry, double dzx
 // dz = sqrt(x^2 + y^2) 2^max(-1020, shift) against a leap radius r given as r^2: the reference's
 // test r^2 > 0 && dz < sqrt(r^2), decided by exponents where they differ.  dz lies in
 // [2^t, 2^(t+2)) for t = exponent of max(|x|, |y|) + max(-1020, shift), or below what a double holds
-// where t is; sqrt(r^2) has half r^2's exponent.  At 1e-1000 nearly every test is decided so: it was
-// two square roots a level, up to 16 levels a leap (1920x1080 there: 1.89 -> 1.44 ms a frame with
-// the packed rows' level search and the renormalisation's and glitch test's exponent screens).
+// where t is; sqrt(r^2) has half r^2's exponent.  At 1e-1000 nearly every test is decided so, from
+// r^2's high word; it was two square roots a level, up to 16 levels a leap.
 struct LinearFit {
     double x, y;
     int t, shift;
@@ -415,14 +437,39 @@ struct LinearFit {
         // zero, subnormal or not finite: never decided by the exponent
         t = top > 0 && top < 2047 ? top - 1023 + shift : INT_MIN;
     }
-    __device__ __forceinline__ bool operator()(double r_sq) const {
-        const int er = __double2hiint(r_sq) >> 20;
-        if (t != INT_MIN && er > 0) {
-            const int es = (er - 1023) >> 1;
-            if (t + 2 <= es) return true;
-            if (t > es && t > -1000) return false;
-        }
+    __device__ __forceinline__ bool exact(double r_sq) const {
         return r_sq > 0.0 && sqrt(x * x + y * y) * pow2_f64(shift) < sqrt(r_sq);
+    }
+    // 1 or 0 where the exponents decide (or r = 0); else `open` is set
+    __device__ __forceinline__ int screen(double r_sq, bool& open) const {
+        const int er = __double2hiint(r_sq) >> 20, es = (er - 1023) >> 1;
+        const bool known = er > 0 && t != INT_MIN;
+        const bool yes = known && t + 2 <= es;
+        open |= !(yes || (known && t > es) || __double_as_longlong(r_sq) == 0);
+        return yes ? 1 : 0;
+    }
+    __device__ __forceinline__ bool operator()(const double* __restrict__ r_sq) const {
+        const double r = __ldg(r_sq);
+        bool open = false;
+        const int yes = screen(r, open);
+        return open ? exact(r) : yes != 0;
+    }
+    // The largest admissible level of a packed radius row (ap_pack_bla): the admissible levels are
+    // a prefix (0 past the orbit's end and the table's levels), so it is a count, taken in two
+    // rounds of three loads without a branch each.
+    __device__ __forceinline__ int level(const double* __restrict__ row) const {
+        bool open = false;
+        int quarter = 0;
+#pragma unroll
+        for (int q = 1; q <= 3; ++q) quarter += screen(__ldg(row + 4 * q), open);
+        int best = 4 * quarter;
+#pragma unroll
+        for (int q = 1; q <= 3; ++q) best += screen(__ldg(row + 4 * quarter + q), open);
+        if (open) {
+            best = 0;
+            while (best < 15 && exact(__ldg(row + best + 1))) ++best;
+        }
+        return best;
     }
 };
 
@@ -434,7 +481,9 @@ struct LinearFit {
 // they differ in the Burning Ship delta form (ARITH), the BLA leap's fused
 // multiply-adds (ARITH) and the stage-2 NaN guard (AP_FLAG_NAN_GUARD).  BBSA
 // starts are never used: the reference maps orders 4/8 to chained BLA here.
-template <int ARITH>
+// The powers of two that depend on the exponent alone, and dc in units of it, are kept between
+// renormalisations that change it.  KIND: 0 z^2 + c, 1 Burning Ship, 4 Multibrot.
+template <int ARITH, int KIND>
 __device__ __forceinline__ SampleOut floatexp_sample_at(const ApFrameParams& p,
                                                         const ApFrameBuffers& b, double sub_i,
                                                         double sub_j) {
@@ -458,18 +507,27 @@ __device__ __forceinline__ SampleOut floatexp_sample_at(const ApFrameParams& p,
         return o;
     };
     const int levels = p.bla_levels;
-    const bool has_bla = levels > 1 && b.bla != nullptr && (ft == 0 || ft == 2 || ft == 4);
+    const bool has_bla = levels > 1 && b.bla != nullptr && KIND != 1;
     const size_t L = (size_t)ref_len;
     const double inv_ln = inv_ln_for(ft, p.gen_n);
     // packed BLA rows (ap_pack_bla), where the pass has them
     const double* __restrict__ rows = has_bla && levels <= 16 ? b.bla_packed : nullptr;
 
+    int eff_exp = 0;  // the true delta is (dzx, dzy) 2^eff_exp
+    double sn = 0.0, cxs = 0.0, cys = 0.0;  // 2^eff_exp (0 below 2^-1020); dc in units of 2^z_exp
+    auto refresh = [&]() {
+        eff_exp = z_exp - E;
+        sn = eff_exp >= -1020 ? pow2_f64(eff_exp) : 0.0;
+        const double scale_c = (z_exp >= -1020 && z_exp <= 1020) ? pow2_f64(-z_exp) : 0.0;
+        cxs = dcpx * scale_c;
+        cys = dcpy * scale_c;
+    };
+    refresh();
+
     while (k < ref_len) {
         const double rx = __ldg(re + k), ry = __ldg(im + k);
-        const int eff_exp = z_exp - E;
         if (eff_exp >= -50) {
-            const double sc = pow2_f64(eff_exp);
-            const double zx = rx + dzx * sc, zy = ry + dzy * sc;
+            const double zx = rx + dzx * sn, zy = ry + dzy * sn;
             const double mag2 = zx * zx + zy * zy;
             if (mag2 > kBailout) {
                 SampleOut o = escaped_sample(k, mag2, inv_ln);
@@ -481,38 +539,31 @@ __device__ __forceinline__ SampleOut floatexp_sample_at(const ApFrameParams& p,
 
         if (has_bla && k < ref_len - 1) {
             // |delta|^2 against r^2 in scaled form, or via square roots far below 2^-510
-            const int shift_r = eff_exp;
-            const bool scaled = shift_r >= -510;
-            double dz_mag2 = 0.0;
-            if (scaled) {
-                const double sr = pow2_f64(shift_r);
-                dz_mag2 = (dzx * dzx + dzy * dzy) * (sr * sr);
-            }
-            const LinearFit linear(dzx, dzy, shift_r);
-            auto fits = [&](double r_sq) { return scaled ? (dz_mag2 < r_sq) : linear(r_sq); };
+            const bool scaled = eff_exp >= -510;
+            const double dz_mag2 = scaled ? (dzx * dzx + dzy * dzy) * (sn * sn) : 0.0;
+            const LinearFit linear(dzx, dzy, eff_exp);
+            auto fits = [&](const double* r) { return scaled ? dz_mag2 < __ldg(r) : linear(r); };
             const double* row = rows ? rows + (size_t)k * 16 : b.bla + (size_t)k * 5 + 4;
-            if (fits(__ldg(row))) {
+            if (fits(row)) {
                 int best = 0;
                 double ar, ai, br, bi;
                 if (rows) {
-                    // the packed radii of step k: the admissible levels are a prefix (0 past
-                    // the orbit's end), so the largest is a count, taken in two rounds
-                    const int top = levels - 1;
-                    int quarter = 0;
+                    if (scaled) {
+                        int quarter = 0;
 #pragma unroll
-                    for (int t = 1; t <= 3; ++t) quarter += (4 * t <= top && fits(__ldg(row + 4 * t))) ? 1 : 0;
-                    best = 4 * quarter;
+                        for (int t = 1; t <= 3; ++t) quarter += dz_mag2 < __ldg(row + 4 * t) ? 1 : 0;
+                        best = 4 * quarter;
 #pragma unroll
-                    for (int t = 1; t <= 3; ++t) {
-                        const int d = 4 * quarter + t;
-                        best += (d <= top && fits(__ldg(row + d))) ? 1 : 0;
+                        for (int t = 1; t <= 3; ++t) best += dz_mag2 < __ldg(row + 4 * quarter + t) ? 1 : 0;
+                    } else {
+                        best = linear.level(row);
                     }
                     const double2* e = reinterpret_cast<const double2*>(rows + L * 16 + ((size_t)k * 16 + best) * 4);
                     const double2 a = __ldg(e), c = __ldg(e + 1);
                     ar = a.x, ai = a.y, br = c.x, bi = c.y;
                 } else {
                     for (int d = levels - 1; d > 0; --d) {
-                        if (k + (1 << d) < ref_len && fits(__ldg(b.bla + ((size_t)d * L + k) * 5 + 4))) {
+                        if (k + (1 << d) < ref_len && fits(b.bla + ((size_t)d * L + k) * 5 + 4)) {
                             best = d;
                             break;
                         }
@@ -520,8 +571,6 @@ __device__ __forceinline__ SampleOut floatexp_sample_at(const ApFrameParams& p,
                     const double* e = b.bla + ((size_t)best * L + k) * 5;
                     ar = __ldg(e), ai = __ldg(e + 1), br = __ldg(e + 2), bi = __ldg(e + 3);
                 }
-                const double scale_c = (z_exp >= -1020 && z_exp <= 1020) ? pow2_f64(-z_exp) : 0.0;
-                const double cxs = dcpx * scale_c, cys = dcpy * scale_c;
                 double nx, ny;
                 if (kCpu) {
                     nx = (ar * dzx - ai * dzy) + (br * cxs - bi * cys);
@@ -532,8 +581,9 @@ __device__ __forceinline__ SampleOut floatexp_sample_at(const ApFrameParams& p,
                 }
                 dzx = nx;
                 dzy = ny;
-                if (isnan(dzx) || isnan(dzy) || isinf(dzx) || isinf(dzy)) return done(glitch_sample(k), k);
-                renorm16(dzx, dzy, z_exp);
+                if (((__double2hiint(dzx) & 0x7ff00000) == 0x7ff00000) | ((__double2hiint(dzy) & 0x7ff00000) == 0x7ff00000))
+                    return done(glitch_sample(k), k);
+                if (renorm16(dzx, dzy, z_exp)) refresh();
                 k += 1 << best;
                 ++leaps;
                 skipped += 1 << best;
@@ -541,32 +591,27 @@ __device__ __forceinline__ SampleOut floatexp_sample_at(const ApFrameParams& p,
             }
         }
 
-        const int shift_nl = z_exp - E;
-        const double scale_c = (z_exp >= -1020 && z_exp <= 1020) ? pow2_f64(-z_exp) : 0.0;
-        if (ft == 0 || ft == 2) {
+        if (KIND == 0) {
             double lx = 2.0 * (rx * dzx - ry * dzy);
             double ly = 2.0 * (rx * dzy + ry * dzx);
-            if (shift_nl >= -1020) {
-                const double sn = pow2_f64(shift_nl);
+            if (eff_exp >= -1020) {
                 lx += (dzx * dzx - dzy * dzy) * sn;
                 ly += (2.0 * dzx * dzy) * sn;
             }
-            dzx = lx + dcpx * scale_c;
-            dzy = ly + dcpy * scale_c;
-        } else if (ft == 1 || ft == 3) {
-            const double sn = shift_nl >= -1020 ? pow2_f64(shift_nl) : 0.0;
+            dzx = lx + cxs;
+            dzy = ly + cys;
+        } else if (KIND == 1) {
             const double sx = rx >= 0.0 ? 1.0 : -1.0, sy = ry >= 0.0 ? 1.0 : -1.0;
             if (kCpu) {  // math_core/cpu_kernels.py:795-829
-                const double se = eff_exp >= -1020 ? pow2_f64(eff_exp) : 0.0;
                 const double inv = eff_exp <= 1020 ? pow2_f64(-eff_exp) : 0.0;
                 double fx, ex, fy, ey;
-                if ((rx + dzx * se) * sx >= 0.0) { fx = sx; ex = 0.0; }
+                if ((rx + dzx * sn) * sx >= 0.0) { fx = sx; ex = 0.0; }
                 else { fx = -sx; ex = eff_exp <= 1020 ? ((-sx * 2.0) * rx) * inv : 0.0; }
-                if ((ry + dzy * se) * sy >= 0.0) { fy = sy; ey = 0.0; }
+                if ((ry + dzy * sn) * sy >= 0.0) { fy = sy; ey = 0.0; }
                 else { fy = -sy; ey = eff_exp <= 1020 ? ((-sy * 2.0) * ry) * inv : 0.0; }
-                const double lx = (2.0 * rx + dzx * sn) * dzx - (2.0 * ry + dzy * sn) * dzy + dcpx * scale_c;
+                const double lx = (2.0 * rx + dzx * sn) * dzx - (2.0 * ry + dzy * sn) * dzy + cxs;
                 const double dxn = fx * dzx + ex, dyn = fy * dzy + ey;
-                const double ly = 2.0 * (fabs(rx) * dyn + fabs(ry) * dxn + dxn * dyn * sn) - dcpy * scale_c;
+                const double ly = 2.0 * (fabs(rx) * dyn + fabs(ry) * dxn + dxn * dyn * sn) - cys;
                 dzx = lx;
                 dzy = ly;
             } else {  // math_core/cuda_kernels.py:964-985
@@ -576,15 +621,14 @@ __device__ __forceinline__ SampleOut floatexp_sample_at(const ApFrameParams& p,
                 const double ddy = (ry + dzy * sd) * sy >= 0.0 ? sy * dzy : -sy * (2.0 * ry * inv + dzy);
                 double lx = 2.0 * (rx * dzx - ry * dzy);
                 double ly = 2.0 * (fabs(rx) * ddy + fabs(ry) * ddx);
-                if (shift_nl >= -1020) {
+                if (eff_exp >= -1020) {
                     lx += (dzx * dzx - dzy * dzy) * sn;
                     ly += (2.0 * ddx * ddy) * sn;
                 }
-                dzx = lx + dcpx * scale_c;
-                dzy = ly - dcpy * scale_c;
+                dzx = lx + cxs;
+                dzy = ly - cys;
             }
         } else {
-            const double sn = shift_nl >= -1020 ? pow2_f64(shift_nl) : 0.0;
             double pr = dzx, pi = dzy, qr = rx, qi = ry;
             for (int t = 0; t < p.gen_n - 1; ++t) {
                 const cplx t1 = cmul(pr, pi, rx, ry);
@@ -597,15 +641,14 @@ __device__ __forceinline__ SampleOut floatexp_sample_at(const ApFrameParams& p,
                 qi = q.i;
             }
             const cplx kz = cmul(p.gen_kr, p.gen_ki, dzx, dzy);
-            dzx = pr + kz.r + dcpx * scale_c;
-            dzy = pi + kz.i + dcpy * scale_c;
+            dzx = pr + kz.r + cxs;
+            dzy = pi + kz.i + cys;
         }
-        renorm16(dzx, dzy, z_exp);
+        if (renorm16(dzx, dzy, z_exp)) refresh();
         ++k;
     }
 
     // Stage 2: z = Z_ref_len + delta, then direct FP64 iteration with c = ref_c + dc.
-    const int eff_exp = z_exp - E;
     const double sfb = eff_exp >= -60 ? pow2_f64(eff_exp) : 0.0;
     double zx = __ldg(re + ref_len) + dzx * sfb, zy = __ldg(im + ref_len) + dzy * sfb;
     const double scf = E <= 1020 ? pow2_f64(-E) : 0.0;

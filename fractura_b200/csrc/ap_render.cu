@@ -17,7 +17,7 @@ namespace ap {
 // one long-lived pixel of a 16 x 16 tile.
 constexpr int kTile = 8;
 
-template <int TIER, int ARITH, bool MULTI>
+template <int TIER, int ARITH, int KIND>
 __device__ __forceinline__ SampleOut sample_at(const ApFrameParams& p, const ApFrameBuffers& b,
                                                double sub_i, double sub_j) {
     if constexpr (TIER == AP_TIER_FP64) {
@@ -31,17 +31,17 @@ __device__ __forceinline__ SampleOut sample_at(const ApFrameParams& p, const ApF
         }
         return fp64_sample<ARITH>(x, y, p);
     } else if constexpr (TIER == AP_TIER_DD) {
-        return dd_sample_at<ARITH, MULTI>(p, sub_i, sub_j);
+        return dd_sample_at<ARITH, KIND == 4>(p, sub_i, sub_j);
     } else if constexpr (TIER == AP_TIER_PERTURB) {
         return perturb_sample_at<ARITH>(p, b, sub_i, sub_j);
     } else {
-        return floatexp_sample_at<ARITH>(p, b, sub_i, sub_j);
+        return floatexp_sample_at<ARITH, KIND>(p, b, sub_i, sub_j);
     }
 }
 
 // One centred sample per pixel (AP_MODE_COARSE): mandelbrot_unified_*_kernel
 // (math_core/cuda_kernels.py:1615-1917) outside its supersampling branches.
-template <int TIER, int ARITH, bool MULTI>
+template <int TIER, int ARITH, int KIND>
 __global__ void __launch_bounds__(kTile * kTile) render_pass_kernel(const ApFrameParams p,
                                                           const ApFrameBuffers b) {
     const int i = blockIdx.x * kTile + (threadIdx.x & (kTile - 1));
@@ -52,7 +52,7 @@ __global__ void __launch_bounds__(kTile * kTile) render_pass_kernel(const ApFram
     constexpr bool kPert = (TIER >= AP_TIER_PERTURB);
     const int f = p.factor;
     const double sub_offset = ((double)f - 1.0) * 0.5;
-    const SampleOut o = sample_at<TIER, ARITH, MULTI>(p, b, (double)(i * f) + sub_offset,
+    const SampleOut o = sample_at<TIER, ARITH, KIND>(p, b, (double)(i * f) + sub_offset,
                                                       (double)(j * f) + sub_offset);
     b.iter_map[idx] = o.s;
     if (b.kmap) b.kmap[idx] = o.k;
@@ -85,7 +85,7 @@ __global__ void __launch_bounds__(kTile * kTile) render_pass_kernel(const ApFram
 constexpr int kPatches = 1;
 constexpr int kSuperWarps = 2;
 
-template <int TIER, int ARITH, bool MULTI>
+template <int TIER, int ARITH, int KIND>
 __global__ void __launch_bounds__(32 * kSuperWarps) supersample_kernel(const ApFrameParams p, const ApFrameBuffers b,
                                                                        const int hist_resolve) {
     constexpr bool kPert = (TIER >= AP_TIER_PERTURB);
@@ -129,7 +129,7 @@ __global__ void __launch_bounds__(32 * kSuperWarps) supersample_kernel(const ApF
                 int i, j;
                 place(first + q / f2, i, j);
                 const int sub = q % f2;
-                const SampleOut o = sample_at<TIER, ARITH, MULTI>(p, b, (double)(i * f + sub % f),
+                const SampleOut o = sample_at<TIER, ARITH, KIND>(p, b, (double)(i * f + sub % f),
                                                                   (double)(j * f + sub / f));
                 double r = 0.0, g = 0.0, bb = 0.0;
                 if ((double)o.s >= 0.0) colour_of(p, b.lut, b.cdf, hist_colour, (double)o.s, r, g, bb);
@@ -173,24 +173,31 @@ __global__ void __launch_bounds__(32 * kSuperWarps) supersample_kernel(const ApF
     }
 }
 
-template <int TIER, int ARITH, bool MULTI>
+template <int TIER, int ARITH, int KIND>
 static int launch_pass(const ApFrameParams& p, const ApFrameBuffers& b, int hist_resolve, cudaStream_t st) {
     if (!hist_resolve && p.mode == AP_MODE_COARSE) {
         dim3 grid((p.width + kTile - 1) / kTile, (p.height + kTile - 1) / kTile);
-        render_pass_kernel<TIER, ARITH, MULTI><<<grid, kTile * kTile, 0, st>>>(p, b);
+        render_pass_kernel<TIER, ARITH, KIND><<<grid, kTile * kTile, 0, st>>>(p, b);
         return check_launch("render_pass_kernel");
     }
     constexpr int kRows = 4 * kSuperWarps;
     dim3 grid((p.width + 8 * kPatches - 1) / (8 * kPatches), (p.height + kRows - 1) / kRows);
-    supersample_kernel<TIER, ARITH, MULTI><<<grid, 32 * kSuperWarps, 0, st>>>(p, b, hist_resolve);
+    supersample_kernel<TIER, ARITH, KIND><<<grid, 32 * kSuperWarps, 0, st>>>(p, b, hist_resolve);
     return check_launch("supersample_kernel");
 }
 
+// KIND: the formula class (0 z^2 + c, 1 Burning Ship, 4 Multibrot) for the tiers whose samples are
+// built for one (double-double separates Multibrot, whose power loop wants more registers, from
+// the others); 0 for the tiers that tell formulas apart at run time.
 template <int TIER, int ARITH>
 static int launch_formula(const ApFrameParams& p, const ApFrameBuffers& b, int hist_resolve, cudaStream_t st) {
-    if (TIER == AP_TIER_DD && p.fractal_type == 4)
-        return launch_pass<TIER, ARITH, TIER == AP_TIER_DD>(p, b, hist_resolve, st);
-    return launch_pass<TIER, ARITH, false>(p, b, hist_resolve, st);
+    if constexpr (TIER == AP_TIER_DD || TIER == AP_TIER_FLOATEXP) {
+        if (p.fractal_type == 4) return launch_pass<TIER, ARITH, 4>(p, b, hist_resolve, st);
+    }
+    if constexpr (TIER == AP_TIER_FLOATEXP) {
+        if (p.fractal_type & 1) return launch_pass<TIER, ARITH, 1>(p, b, hist_resolve, st);
+    }
+    return launch_pass<TIER, ARITH, 0>(p, b, hist_resolve, st);
 }
 
 template <int TIER>
