@@ -11,25 +11,19 @@
 // (x = cx - w/2 + i w/(W-1), y = cy + h/2 - j h/(H-1), h = w H / W) and P.
 //
 //   ap_smooth_forward: s, K and checkpoints z_0, z_C, z_2C, ... (C = ckpt_every);
-//   ap_smooth_adjoint: per pixel, for the upstream gradient g = dL/ds, sweeps the
-//     orbit backwards one checkpoint segment at a time, recomputing the segment's
-//     z from its checkpoint (first every 16th z, then each 16-step sub-segment into
-//     shared memory; no orbit is stored), and accumulates dL/dtheta; one row of sums
-//     per warp of 8 x 4 pixels (deterministic, summed by the caller);
+//   ap_smooth_adjoint: per pixel, for the upstream gradient g = dL/ds, the vector-Jacobian
+//     product dL/dtheta of the whole orbit, recomputed (no orbit is stored); one row of
+//     sums per warp of 8 x 4 pixels (deterministic, summed by the caller);
 //   ap_smooth_tangent: forward mode (one tangent per parameter carried beside z),
 //     per-pixel ds/dtheta, the independent check of the adjoint.
-// Holomorphic steps make both sweeps complex multiplications: the adjoint
-// multiplies by conj(f'(z_k)), the tangent by f'(z_k).
+// Holomorphic steps make both sweeps complex multiplications: the adjoint multiplies by the
+// conjugates of the orbit's derivatives, the tangent by f'(z_k).
 #include "ap_common.cuh"
+#include "ap_fp64.cuh"
 
 namespace ap {
 
 constexpr int kMaxSegment = 1024;
-// The adjoint replays a checkpoint segment twice: once keeping z every kSub steps (local
-// memory, kMaxSubs values), then, sub-segment by sub-segment from the last, to hold that
-// sub-segment's z in shared memory for the reverse sweep.  No orbit reaches global memory.
-constexpr int kSub = 16;
-constexpr int kMaxSubs = kMaxSegment / kSub;
 
 struct C2d {
     double r, i;
@@ -37,16 +31,28 @@ struct C2d {
 __device__ __forceinline__ C2d cmul2(C2d a, C2d b) { return {a.r * b.r - a.i * b.i, a.r * b.i + a.i * b.r}; }
 __device__ __forceinline__ C2d cadd2(C2d a, C2d b) { return {a.r + b.r, a.i + b.i}; }
 
-// z' = f(z) and f'(z) for the three formulas.
+// a b and a b + s with fused multiply-adds (derivatives only: an orbit keeps the unfused steps that
+// the escape step was found with).
+__device__ __forceinline__ C2d cmul_f(C2d a, C2d b) {
+    return {fma(a.r, b.r, -(a.i * b.i)), fma(a.r, b.i, a.i * b.r)};
+}
+__device__ __forceinline__ C2d cfma(C2d a, C2d b, C2d s) {
+    return {fma(a.r, b.r, fma(-a.i, b.i, s.r)), fma(a.r, b.i, fma(a.i, b.r, s.i))};
+}
+__device__ __forceinline__ C2d conj2(C2d a) { return {a.r, -a.i}; }
+
+// z' = f(z) and f'(z) for the three formulas.  FT: 0 Mandelbrot, 2 Julia, 4 Multibrot, 3 Multibrot
+// with n = 3.
+template <int FT>
 __device__ __forceinline__ void step_f(const ApGradView& v, C2d z, C2d c, C2d& zn, C2d& dfdz) {
-    if (v.fractal_type == 4 && v.gen_n == 3) {
+    if (FT == 3) {
         // the generic loop's values (z^2 = z z, z^3 = z^2 z, the same sums) without its
         // first product by 1: two fewer dependent multiplies per step
         const C2d z2 = cmul2(z, z);
         const C2d P = {v.pr, v.pi};
         zn = cadd2(cadd2(cmul2(z2, z), cmul2(P, z)), c);
         dfdz = cadd2({3.0 * z2.r, 3.0 * z2.i}, P);
-    } else if (v.fractal_type == 4) {
+    } else if (FT == 4) {
         C2d zp = {1.0, 0.0};  // z^(n-1)
         for (int t = 0; t < v.gen_n - 1; ++t) zp = cmul2(zp, z);
         const C2d P = {v.pr, v.pi};
@@ -87,6 +93,12 @@ __device__ __forceinline__ double inv_ln_of(const ApGradView& v) {
 // Blocks of 8 x 8 pixels (two warps of 8 x 4): a block lives as long as its slowest
 // pixel, so small blocks let the SMs refill as blocks finish, and the grid of a 512 x 512
 // view (4096 blocks) is resident at once (32 blocks of 64 threads per SM: 4736).
+// After kLead tested steps the orbit runs in blocks of kBlock steps tested at their end, with
+// cycle detection (fp64_orbit, ap_fp64.cuh), where no checkpoint falls inside; a cycle's remaining
+// checkpoints are found within one turn of it each.  Lanes whose block escaped wait for the others
+// to leave their blocks and are finished together.  512x512 at depth 2000, Julia 80 -> 49 us,
+// Multibrot n = 3 340 -> 215 us (the last warps' chains).
+template <int FT>
 __global__ void __launch_bounds__(64) smooth_forward_kernel(const ApGradView v, double* __restrict__ s64,
                                                             int32_t* __restrict__ kmap,
                                                             double2* __restrict__ ckpt, int n_ck) {
@@ -101,23 +113,61 @@ __global__ void __launch_bounds__(64) smooth_forward_kernel(const ApGradView v, 
     double s = -1.0;
     int K = -1;
     if (!skip) {
+        const bool growing = fp64_growing(FT == 0 || FT == 2 ? kKindQuad : kKindMulti, c.r, c.i, v.gen_n, v.pr, v.pi);
         int until_ck = 0, slot = 0;  // steps to the next checkpoint, and its slot
-        for (int k = 0; k < v.max_iter; ++k) {
-            if (until_ck == 0) {
-                if (ckpt && slot < n_ck) ckpt[idx * n_ck + slot] = make_double2(z.r, z.i);
-                ++slot;
-                until_ck = v.ckpt_every;
+        C2d kept = z;                // the z that block ends are compared with
+        int kept_k = 0, left = 1, window = 1;
+        int k = 0, tested = growing ? kLead : v.max_iter;  // steps to test one by one
+        bool done = false;
+        while (!done && k < v.max_iter) {
+            for (; tested > 0 && k < v.max_iter; --tested) {
+                if (until_ck == 0) {
+                    if (ckpt && slot < n_ck) ckpt[idx * n_ck + slot] = make_double2(z.r, z.i);
+                    ++slot;
+                    until_ck = v.ckpt_every;
+                }
+                const double m = z.r * z.r + z.i * z.i;
+                if (m > kBailout) {
+                    const double lm = log(m);
+                    s = lm > 1.0 ? ((double)k + 1.0) - (log(0.5 * lm) - kLnBailoutLog) * inv_ln_of(v)
+                                 : (double)k;
+                    K = k;
+                    done = true;
+                    break;
+                }
+                step_f<FT>(v, z, c, z, d);
+                --until_ck;
+                ++k;
             }
-            --until_ck;
-            const double m = z.r * z.r + z.i * z.i;
-            if (m > kBailout) {
-                const double lm = log(m);
-                s = lm > 1.0 ? ((double)k + 1.0) - (log(0.5 * lm) - kLnBailoutLog) * inv_ln_of(v)
-                             : (double)k;
-                K = k;
-                break;
+            while (!done && until_ck >= kBlock && k + kBlock <= v.max_iter) {
+                const C2d before = z;
+#pragma unroll
+                for (int t = 0; t < kBlock; ++t) step_f<FT>(v, z, c, z, d);
+                if (!(z.r * z.r + z.i * z.i <= kBailout)) {
+                    z = before;
+                    break;
+                }
+                k += kBlock;
+                until_ck -= kBlock;
+                if (z.r == kept.r && z.i == kept.i) {  // repeats: never escapes
+                    const int turn = k - kept_k;
+                    for (; ckpt && slot < n_ck && k + until_ck < v.max_iter; ++slot) {
+                        for (int t = until_ck % turn; t > 0; --t) step_f<FT>(v, z, c, z, d);
+                        k += until_ck;
+                        until_ck = v.ckpt_every;
+                        ckpt[idx * n_ck + slot] = make_double2(z.r, z.i);
+                    }
+                    done = true;
+                } else if (--left == 0) {
+                    kept = z;
+                    kept_k = k;
+                    window *= 2;
+                    left = window;
+                }
             }
-            step_f(v, z, c, z, d);
+            // what a block could not take: the steps of the one that escaped, or up to past the
+            // next checkpoint, or to max_iter
+            tested = min(kBlock, until_ck) + 1;
         }
     }
     s64[idx] = s;
@@ -132,22 +182,27 @@ __device__ __forceinline__ C2d ds_dzK(const ApGradView& v, C2d zK) {
     return {f * zK.r, f * zK.i};
 }
 
-// Each warp takes 8 x 4 pixels and writes its own row of sums (shuffles, no block
-// barrier); a block of kAdjWarps warps holds its shared sub-segment buffer until its
-// slowest pixel is done, so small blocks keep the SMs filling up behind long-lived pixels.
-#ifndef AP_ADJ_WARPS
-#define AP_ADJ_WARPS 4
-#endif
-constexpr int kAdjWarps = AP_ADJ_WARPS;
+// Each warp takes 8 x 4 pixels and writes its own row of sums (shuffles, no block barrier).
+//
+// A pixel's orbit is one complex function z_K of its pixel and P, so the adjoint of all its steps,
+// applied to the one complex dL/dz_K, takes two complex numbers: dz_K/dpixel and dz_K/dP.  They are
+// accumulated beside the recomputed orbit (D' = f' D + df/dpixel, B' = f' B + df/dP; a Julia
+// set's pixel is z_0: D_0 = 1), and then dL/dpixel = G conj(D), dL/dP = G conj(B).  One walk over
+// the orbit from z_0 replaces the sweep from the checkpoints, which replayed each segment twice
+// (every 16th z, then 16 z at a time into shared memory) to run it backwards: 18 FP64 operations a
+// Julia step for 32, 34 a Multibrot n = 3 step for 96, the derivatives in chains of their own
+// beside z's, no local or shared memory, and the gradient does not depend on the checkpoints at
+// all: 512x512 at depth 2000, Julia 178 -> 81 us, Multibrot n = 3 317 -> 91 us.  A pixel that never escapes, or has no gradient, costs nothing.
+constexpr int kAdjWarps = 4;
 
+template <int FT>
 __global__ void __launch_bounds__(32 * kAdjWarps) smooth_adjoint_kernel(const ApGradView v,
                                                                         const double* __restrict__ grad_s,
                                                                         const int32_t* __restrict__ kmap,
-                                                                        const double2* __restrict__ ckpt,
-                                                                        int n_ck, double* __restrict__ pix_grads,
+                                                                        double* __restrict__ pix_grads,
                                                                         double* __restrict__ block_sums,
                                                                         int n_tiles) {
-    __shared__ double2 buf[kSub][32 * kAdjWarps];  // one sub-segment of z per thread (8 KiB per warp)
+    constexpr bool kJulia = FT == 2, kMulti = FT == 3 || FT == 4;
     const int tile = blockIdx.x * kAdjWarps + (threadIdx.x >> 5);
     if (tile >= n_tiles) return;  // whole warps only: the shuffles below stay full
     const int lane = threadIdx.x & 31;
@@ -165,55 +220,18 @@ __global__ void __launch_bounds__(32 * kAdjWarps) smooth_adjoint_kernel(const Ap
             double dpx_dw, dpy_dw;
             bool skip;
             pixel_setup(v, i, j, z0, c, dpx_dw, dpy_dw, skip);
-            double2 sub[kMaxSubs];  // this segment's sub-checkpoints (local memory, 1 KiB)
-            const int C = v.ckpt_every;
-            C2d G = {0.0, 0.0};  // dL/dz_{k+1} during the sweep
-            C2d gc = {0.0, 0.0}, gp = {0.0, 0.0};
-            bool first = true;
-            for (int sg = K / C; sg >= 0; --sg) {
-                const int k0 = sg * C;
-                const int k1 = min(K, k0 + C);  // this segment's steps z_k -> z_{k+1}, k in [k0, k1)
-                const double2 st = ckpt[idx * n_ck + sg];
-                C2d z = {st.x, st.y}, d;
-                for (int k = k0; k < k1; ++k) {  // pass 1: z every kSub steps
-                    if (((k - k0) & (kSub - 1)) == 0) sub[(k - k0) / kSub] = make_double2(z.r, z.i);
-                    step_f(v, z, c, z, d);
-                }
-                if (first) {  // the last segment ends at k1 = K: z is z_K
-                    const C2d dz = ds_dzK(v, z);
-                    G = {gs * dz.r, gs * dz.i};
-                    first = false;
-                }
-                for (int s0 = k0 + ((k1 - k0 - 1) / kSub) * kSub; s0 >= k0 && k1 > k0; s0 -= kSub) {
-                  const int s1 = min(k1, s0 + kSub);
-                  {  // pass 2: this sub-segment's inputs z_s0 .. z_(s1-1) into shared memory
-                    const double2 w0 = sub[(s0 - k0) / kSub];
-                    C2d w = {w0.x, w0.y}, dw;
-                    for (int k = s0; k < s1; ++k) {
-                        buf[k - s0][threadIdx.x] = make_double2(w.r, w.i);
-                        step_f(v, w, c, w, dw);
-                    }
-                  }
-                  for (int k = s1 - 1; k >= s0; --k) {
-                    const double2 bk = buf[k - s0][threadIdx.x];
-                    const C2d zk = {bk.x, bk.y};
-                    // parameter terms of z_{k+1} = f(z_k)
-                    if (v.fractal_type == 2) {
-                        gp = cadd2(gp, G);  // dz'/dP = 1
-                    } else {
-                        gc = cadd2(gc, G);  // dz'/dc = 1
-                        if (v.fractal_type == 4) {  // dz'/d(Re P) = z_k, dz'/d(Im P) = i z_k
-                            gp.r += G.r * zk.r + G.i * zk.i;
-                            gp.i += -G.r * zk.i + G.i * zk.r;
-                        }
-                    }
-                    C2d zn, dfdz;
-                    step_f(v, zk, c, zn, dfdz);
-                    G = cmul2(G, {dfdz.r, -dfdz.i});  // G_k = G_{k+1} conj(f'(z_k))
-                  }
-                }
+            C2d z = z0, B = {0.0, 0.0}, D = {kJulia ? 1.0 : 0.0, 0.0};
+#pragma unroll 4
+            for (int k = 0; k < K; ++k) {
+                C2d zn, f;
+                step_f<FT>(v, z, c, zn, f);
+                D = kJulia ? cmul_f(f, D) : cfma(f, D, {1.0, 0.0});
+                if (kJulia) B = cfma(f, B, {1.0, 0.0});
+                if (kMulti) B = cfma(f, B, z);
+                z = zn;
             }
-            if (v.fractal_type == 2) gc = G;  // the pixel is z_0
+            const C2d dz = ds_dzK(v, z), G = {gs * dz.r, gs * dz.i};
+            const C2d gc = cmul_f(G, conj2(D)), gp = kJulia || kMulti ? cmul_f(G, conj2(B)) : C2d{0.0, 0.0};
             g[0] = gc.r;
             g[1] = gc.i;
             g[2] = v.w * (gc.r * dpx_dw + gc.i * dpy_dw);
@@ -231,6 +249,7 @@ __global__ void __launch_bounds__(32 * kAdjWarps) smooth_adjoint_kernel(const Ap
         for (int q = 0; q < 5; ++q) block_sums[(size_t)tile * 5 + q] = g[q];
 }
 
+template <int FT>
 __global__ void __launch_bounds__(256) smooth_tangent_kernel(const ApGradView v, double* __restrict__ ds) {
     const int i = blockIdx.x * 16 + (threadIdx.x & 15);
     const int j = blockIdx.y * 16 + (threadIdx.x >> 4);
@@ -258,7 +277,7 @@ __global__ void __launch_bounds__(256) smooth_tangent_kernel(const ApGradView v,
                 break;
             }
             C2d zn, dfdz;
-            step_f(v, z, c, zn, dfdz);
+            step_f<FT>(v, z, c, zn, dfdz);
             for (int q = 0; q < 5; ++q) t[q] = cmul2(dfdz, t[q]);
             if (v.fractal_type == 2) {
                 t[3].r += 1.0;  // dz'/d(Re P) = 1
@@ -274,6 +293,23 @@ __global__ void __launch_bounds__(256) smooth_tangent_kernel(const ApGradView v,
         }
     }
     for (int q = 0; q < 5; ++q) ds[idx * 5 + q] = out[q];
+}
+
+// Calls f with the formula class of step_f as a compile-time constant.
+template <int N>
+struct Formula {
+    constexpr int operator()() const { return N; }
+};
+template <typename F>
+static void for_formula(const ApGradView& v, F&& f) {
+    if (v.fractal_type == 4) {
+        if (v.gen_n == 3) f(Formula<3>());
+        else f(Formula<4>());
+    } else if (v.fractal_type == 2) {
+        f(Formula<2>());
+    } else {
+        f(Formula<0>());
+    }
 }
 
 static int check_view(const ApGradView* v, const char* what) {
@@ -297,8 +333,10 @@ extern "C" int ap_smooth_forward(const ApGradView* v, double* s64, int32_t* kmap
         return AP_E_INVALID;
     }
     dim3 grid((v->width + 7) / 8, (v->height + 7) / 8);
-    ap::smooth_forward_kernel<<<grid, 64, 0, static_cast<cudaStream_t>(stream)>>>(
-        *v, s64, kmap, reinterpret_cast<double2*>(ckpt), n_ck);
+    ap::for_formula(*v, [&](auto ft) {
+        ap::smooth_forward_kernel<ft()><<<grid, 64, 0, static_cast<cudaStream_t>(stream)>>>(
+            *v, s64, kmap, reinterpret_cast<double2*>(ckpt), n_ck);
+    });
     return ap::check_launch("smooth_forward_kernel");
 }
 
@@ -318,9 +356,11 @@ extern "C" int ap_smooth_adjoint(const ApGradView* v, const double* grad_s, cons
         return AP_E_INVALID;
     }
     const int blocks = ap_smooth_adjoint_blocks(v->width, v->height);
-    ap::smooth_adjoint_kernel<<<(blocks + ap::kAdjWarps - 1) / ap::kAdjWarps, 32 * ap::kAdjWarps, 0,
-                                static_cast<cudaStream_t>(stream)>>>(
-        *v, grad_s, kmap, reinterpret_cast<const double2*>(ckpt), n_ck, pix_grads, block_sums, blocks);
+    ap::for_formula(*v, [&](auto ft) {
+        ap::smooth_adjoint_kernel<ft()><<<(blocks + ap::kAdjWarps - 1) / ap::kAdjWarps, 32 * ap::kAdjWarps, 0,
+                                          static_cast<cudaStream_t>(stream)>>>(
+            *v, grad_s, kmap, pix_grads, block_sums, blocks);
+    });
     return ap::check_launch("smooth_adjoint_kernel");
 }
 
@@ -332,6 +372,8 @@ extern "C" int ap_smooth_tangent(const ApGradView* v, double* ds, void* stream) 
         return AP_E_INVALID;
     }
     dim3 grid((v->width + 15) / 16, (v->height + 15) / 16);
-    ap::smooth_tangent_kernel<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(*v, ds);
+    ap::for_formula(*v, [&](auto ft) {
+        ap::smooth_tangent_kernel<ft()><<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(*v, ds);
+    });
     return ap::check_launch("smooth_tangent_kernel");
 }

@@ -434,8 +434,8 @@ AP_API int ap_render_batch(const ApTileDesc* tiles, const int64_t* first_patch, 
  *   ckpt_every-th step: ckpt[H, W, n_ck] complex float64, n_ck >= ceil(max_iter/ckpt_every)+1.
  * ap_smooth_adjoint: for grad_s[H, W] = dL/ds, dL/dtheta summed per tile of 8 x 4 pixels
  *   into block_sums[ap_smooth_adjoint_blocks(W, H), 5] (the caller sums the rows); the orbit
- *   is recomputed segment by segment from ckpt, never stored; pix_grads[H, W, 5]
- *   (optional) receives each pixel's term.
+ *   is recomputed, never stored (ckpt, from ap_smooth_forward, is checked as before, but the
+ *   sweep needs nothing from it); pix_grads[H, W, 5] (optional) receives each pixel's term.
  * ap_smooth_tangent: forward mode, ds[H, W, 5] = ds/dtheta per pixel. */
 AP_API int ap_smooth_forward(const ApGradView* v, double* s64, int32_t* kmap, double* ckpt,
                              int32_t n_ck, void* stream);
