@@ -59,6 +59,94 @@ __global__ void __launch_bounds__(256) histogram_kernel(const float* __restrict_
     }
 }
 
+// Larger maps are counted in shared memory first: a block of 1024 threads counts up to 65408 pixels
+// into 16-bit counters, two a word (128 KiB at 65536 bins), four pixels a thread at a time, then adds
+// its non-empty bins to the global histogram.  Most of a frame's pixels fall into a few thousand bins,
+// so that is an eighth of the global atomics or fewer.  Bound by latency: one block an SM, its loads,
+// its shared atomics and the walk over its counters, one after the other.
+constexpr int kHistThreads = 1024;
+constexpr int kHistMaxBins = 65536;
+constexpr size_t kHistPixels = 65408;  // below 2^16, a multiple of 128
+
+__global__ void __launch_bounds__(kHistThreads) histogram_shared_kernel(const float* __restrict__ it, size_t n,
+                                                                        size_t chunk, double inv_max, int num_bins,
+                                                                        int* __restrict__ hist) {
+    extern __shared__ unsigned counts[];
+    const int words = (num_bins + 1) / 2;
+    for (int w = threadIdx.x; w < words; w += kHistThreads) counts[w] = 0u;
+    __syncthreads();
+    const size_t first = blockIdx.x * chunk, end = first + chunk < n ? first + chunk : n;
+    const bool aligned = (reinterpret_cast<uintptr_t>(it) & 15u) == 0;
+    for (size_t base = first + 4 * (threadIdx.x & ~31u); base < end; base += 4 * kHistThreads) {
+        const size_t q = base + 4 * (threadIdx.x & 31);
+        float s[4] = {-1.0f, -1.0f, -1.0f, -1.0f};
+        if (aligned && q + 4 <= end) {
+            const float4 v = *reinterpret_cast<const float4*>(it + q);
+            s[0] = v.x, s[1] = v.y, s[2] = v.z, s[3] = v.w;
+        } else {
+#pragma unroll
+            for (int t = 0; t < 4; ++t)
+                if (q + t < end) s[t] = it[q + t];
+        }
+        int bin[4];
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+            bin[t] = -1;
+            if (s[t] >= 0.0f) {
+                const double pos = ((double)s[t] * inv_max) * (double)(num_bins - 1);
+                bin[t] = (int)pos;
+                if (bin[t] >= num_bins) bin[t] = num_bins - 1;
+                else if (bin[t] < 0) bin[t] = 0;
+            }
+        }
+        // a flat stretch of the map adds once a warp
+        const int lead = __shfl_sync(0xffffffffu, bin[0], 0);
+        if (__all_sync(0xffffffffu, bin[0] == lead && bin[1] == lead && bin[2] == lead && bin[3] == lead)) {
+            if (lead >= 0 && (threadIdx.x & 31) == 0) atomicAdd(counts + (lead >> 1), 128u << (16 * (lead & 1)));
+        } else {
+#pragma unroll
+            for (int t = 0; t < 4; ++t)
+                if (bin[t] >= 0) atomicAdd(counts + (bin[t] >> 1), 1u << (16 * (bin[t] & 1)));
+        }
+    }
+    __syncthreads();
+    for (int w = threadIdx.x; w < words; w += kHistThreads) {
+        const unsigned c = counts[w];
+        if (c & 0xffffu) atomicAdd(hist + 2 * w, (int)(c & 0xffffu));
+        if (c >> 16) atomicAdd(hist + 2 * w + 1, (int)(c >> 16));
+    }
+}
+
+// From this many pixels on, the kernels of fewer, longer threads win.  Histogram: 3840x2160 64 us with
+// histogram_kernel, 25 with histogram_shared_kernel (a flat map 174 and 17); 1920x1080 24.6 and 15.5;
+// 640x360 11.2 with the first and more with the second, whose 128 KiB of counters are cleared and
+// walked.  Colour: 3840x2160 69 us with a pixel a thread, 50 with four; 640x360 5.4 and 7.5.
+constexpr size_t kLargeMap = (size_t)1 << 19;
+
+// Adds the map's counts to hist.
+static int launch_histogram(const float* it, size_t n, double inv_max, int num_bins, int* hist, cudaStream_t st) {
+    if (n >= kLargeMap && num_bins <= kHistMaxBins) {
+        size_t blocks = (n + kHistPixels - 1) / kHistPixels;
+        const size_t spread = (n + 4095) / 4096 < 148 ? (n + 4095) / 4096 : 148;
+        if (blocks < spread) blocks = spread;
+        const size_t chunk = ((n + blocks - 1) / blocks + 127) / 128 * 128;  // kHistPixels at most
+        const size_t bytes = (size_t)((num_bins + 1) / 2) * 4;
+        if (blocks < (size_t)1 << 30) {
+            const cudaError_t e = cudaFuncSetAttribute(histogram_shared_kernel,
+                                                       cudaFuncAttributeMaxDynamicSharedMemorySize, kHistMaxBins * 2);
+            if (e != cudaSuccess) {
+                set_error("histogram_shared_kernel: shared memory: %s", cudaGetErrorString(e));
+                return AP_E_CUDA;
+            }
+            histogram_shared_kernel<<<(int)blocks, kHistThreads, bytes, st>>>(it, n, chunk, inv_max, num_bins, hist);
+            return check_launch("histogram_shared_kernel");
+        }
+    }
+    int blocks = (int)((n + 255) / 256 < 148 * 16 ? (n + 255) / 256 : 148 * 16);
+    histogram_kernel<<<blocks, 256, 0, st>>>(it, n, inv_max, num_bins, hist);
+    return check_launch("histogram_kernel");
+}
+
 // One block of 1024 threads: inclusive prefix sum of the histogram in exact
 // integer arithmetic, then cdf[b] = float32(prefix[b] / total) as the
 // float64 scan of math_core/cuda_kernels.py:1929-1996 produces it.  Serves bin
@@ -280,8 +368,12 @@ static int launch_cdf(const int32_t* hist, int num_bins, float* cdf, cudaStream_
 // ----------------------------------------------------------------- colour
 // apply_histogram_equalization_kernel (math_core/cuda_kernels.py:2016) and
 // recolor_iter_map_cuda_kernel (math_core/cuda_kernels.py:3201).
+// Any alignment, and the masked form of rebase passes: a pixel a thread.
 __global__ void __launch_bounds__(256) colour_kernel(const ApFrameParams p, const ApFrameBuffers b,
                                                      int hist) {
+    __shared__ Palette palette;
+    if (threadIdx.x == 0) palette = palette_of(p, hist != 0);
+    __syncthreads();
     const int i = blockIdx.x * 16 + (threadIdx.x & 15);
     const int j = blockIdx.y * 16 + (threadIdx.x >> 4);
     if (i >= p.width || j >= p.height) return;
@@ -289,8 +381,87 @@ __global__ void __launch_bounds__(256) colour_kernel(const ApFrameParams p, cons
     if (p.rebase_pass > 0 && b.glitch_in != nullptr && b.glitch_in[idx] == 0) return;
     const double s = (double)b.iter_map[idx];
     double r = 0.0, g = 0.0, bb = 0.0;
-    if (s >= 0.0) colour_of(p, b.lut, b.cdf, hist != 0, s, r, g, bb);
+    if (s >= 0.0) colour_of(p, palette, b.lut, b.cdf, hist != 0, s, r, g, bb);
     store_rgb(b.rgb, p.is_hdr, idx, r, g, bb);
+}
+
+// Whole frames, rows ignored: four consecutive pixels a thread, one float4 load and three words
+// stored (six for 16-bit components) instead of three bytes a pixel, one scheme a kernel (SCHEME 11:
+// the histogram transfer).  Bound by the transfer function's FP64 operations, then by the
+// conversions: a 3840x2160 histogram frame 69 us -> 50.
+template <int SCHEME, bool HDR>
+__global__ void __launch_bounds__(256) colour4_kernel(const ApFrameParams p, const ApFrameBuffers b, size_t n4) {
+    __shared__ Palette palette;
+    if (threadIdx.x == 0) palette = palette_of(p, SCHEME == 11);
+    __syncthreads();
+    const Palette c = palette;
+    const bool f32 = p.arith == AP_ARITH_REF_CPU;
+    for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < n4; q += (size_t)gridDim.x * blockDim.x) {
+        const float4 v = reinterpret_cast<const float4*>(b.iter_map)[q];
+        const float s4[4] = {v.x, v.y, v.z, v.w};
+        unsigned part[12];
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+            const double s = (double)s4[t];
+            double r = 0.0, g = 0.0, bb = 0.0;
+            if (s >= 0.0) {
+                const double norm = SCHEME == 11 ? cdf_norm(c, s, b.cdf, p.num_bins, p.color_contrast)
+                                                 : palette_norm(c, s, SCHEME, f32);
+                lut_lerp(b.lut, norm, r, g, bb);
+            }
+            part[3 * t] = colour_int(r);
+            part[3 * t + 1] = colour_int(g);
+            part[3 * t + 2] = colour_int(bb);
+        }
+        unsigned* o = static_cast<unsigned*>(b.rgb) + q * (HDR ? 6 : 3);
+        if (HDR) {
+#pragma unroll
+            for (int w = 0; w < 6; ++w) o[w] = (part[2 * w] & 0xffffu) | (part[2 * w + 1] << 16);
+        } else {
+#pragma unroll
+            for (int w = 0; w < 3; ++w)
+                o[w] = (part[4 * w] & 0xffu) | ((part[4 * w + 1] & 0xffu) << 8) | ((part[4 * w + 2] & 0xffu) << 16) |
+                       (part[4 * w + 3] << 24);
+        }
+    }
+}
+
+template <int SCHEME>
+static void launch_colour4(const ApFrameParams& p, const ApFrameBuffers& b, size_t n4, cudaStream_t st) {
+    const size_t blocks = (n4 + 255) / 256;
+    const int grid = (int)(blocks < 148 * 32 ? blocks : 148 * 32);
+    if (p.is_hdr) colour4_kernel<SCHEME, true><<<grid, 256, 0, st>>>(p, b, n4);
+    else colour4_kernel<SCHEME, false><<<grid, 256, 0, st>>>(p, b, n4);
+}
+
+// A large frame whose pixels come in fours, with aligned maps and no mask, takes colour4_kernel.
+static int launch_colour(const ApFrameParams& p, const ApFrameBuffers& b, int hist, cudaStream_t st) {
+    const size_t n = (size_t)p.width * p.height;
+    const bool masked = p.rebase_pass > 0 && b.glitch_in != nullptr;
+    if (n >= kLargeMap && !masked && (n & 3) == 0 && (reinterpret_cast<uintptr_t>(b.iter_map) & 15u) == 0 &&
+        (reinterpret_cast<uintptr_t>(b.rgb) & 3u) == 0) {
+        const size_t n4 = n / 4;
+        switch (hist ? 11 : p.scheme_id) {
+        case 1: launch_colour4<1>(p, b, n4, st); break;
+        case 2: launch_colour4<2>(p, b, n4, st); break;
+        case 3: launch_colour4<3>(p, b, n4, st); break;
+        case 5: launch_colour4<5>(p, b, n4, st); break;
+        case 6: launch_colour4<6>(p, b, n4, st); break;
+        case 7: launch_colour4<7>(p, b, n4, st); break;
+        case 8: launch_colour4<8>(p, b, n4, st); break;
+        case 9: launch_colour4<9>(p, b, n4, st); break;
+        case 10: launch_colour4<10>(p, b, n4, st); break;
+        case 11:  // without a CDF the scheme colours as 0
+            if (hist) launch_colour4<11>(p, b, n4, st);
+            else launch_colour4<0>(p, b, n4, st);
+            break;
+        default: launch_colour4<0>(p, b, n4, st);  // 0, 4 and ids above 11: palette_of tells them apart
+        }
+        return check_launch("colour4_kernel");
+    }
+    dim3 grid((p.width + 15) / 16, (p.height + 15) / 16);
+    colour_kernel<<<grid, 256, 0, st>>>(p, b, hist);
+    return check_launch("colour_kernel");
 }
 
 // ---------------------------------------------------------- listed pixels
@@ -310,7 +481,8 @@ __global__ void __launch_bounds__(256) set_pixels_kernel(const ApFrameParams p, 
     const double s = values[q];
     b.iter_map[idx] = (float)s;
     double cr = 0.0, cg = 0.0, cb = 0.0;
-    if (s >= 0.0 && s < (double)p.max_iter) colour_of(p, b.lut, b.cdf, hist != 0, s, cr, cg, cb);
+    if (s >= 0.0 && s < (double)p.max_iter)
+        colour_of(p, palette_of(p, hist != 0), b.lut, b.cdf, hist != 0, s, cr, cg, cb);
     store_rgb(b.rgb, p.is_hdr, idx, cr, cg, cb);
     if (b.glitch_out) b.glitch_out[idx] = 0;
 }
@@ -367,10 +539,7 @@ extern "C" int ap_histogram_cdf(const float* iter_map, int32_t width, int32_t he
     }
     const size_t n = (size_t)width * height;
     const double inv_max = 1.0 / fmax(1.0, (double)max_iter);
-    int blocks = (int)((n + 255) / 256);
-    if (blocks > 148 * 16) blocks = 148 * 16;
-    ap::histogram_kernel<<<blocks, 256, 0, st>>>(iter_map, n, inv_max, num_bins, hist);
-    int rc = ap::check_launch("histogram_kernel");
+    int rc = ap::launch_histogram(iter_map, n, inv_max, num_bins, hist, st);
     if (rc != AP_OK) return rc;
     return ap::launch_cdf(hist, num_bins, cdf, st);
 }
@@ -390,10 +559,7 @@ extern "C" int ap_histogram(const float* iter_map, int32_t width, int32_t height
     const size_t n = (size_t)width * height;
     if (n == 0) return AP_OK;
     const double inv_max = 1.0 / fmax(1.0, (double)max_iter);
-    int blocks = (int)((n + 255) / 256);
-    if (blocks > 148 * 16) blocks = 148 * 16;
-    ap::histogram_kernel<<<blocks, 256, 0, st>>>(iter_map, n, inv_max, num_bins, hist);
-    return ap::check_launch("histogram_kernel");
+    return ap::launch_histogram(iter_map, n, inv_max, num_bins, hist, st);
 }
 
 extern "C" int ap_cdf_from_histogram(const int32_t* hist, int32_t num_bins, float* cdf, void* stream) {
@@ -414,9 +580,7 @@ extern "C" int ap_colour(const ApFrameParams* p, const ApFrameBuffers* b, void* 
         ap::set_error("ap_colour: num_bins must be >= 2");
         return AP_E_INVALID;
     }
-    dim3 grid((p->width + 15) / 16, (p->height + 15) / 16);
-    ap::colour_kernel<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(*p, *b, hist);
-    return ap::check_launch("colour_kernel");
+    return ap::launch_colour(*p, *b, hist, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int ap_glitch_bins(const uint8_t* glitch_map, int32_t width, int32_t height,

@@ -101,12 +101,16 @@ constexpr int kSpan = 8;
 // Transfer functions of math_core/cuda_kernels.py:157-259, evaluated in
 // float64 on the float32 smooth value.
 
-__device__ __forceinline__ double py_mod(double x, double m) {
-    double r = fmod(x, m);
+// Python's x % M for M = 1, 2.  fmod is exact, and so is x - M trunc(x / M) here: x / M only moves the
+// exponent, the multiple of M is exact, and the difference is representable (it is the fmod).
+template <int M>
+__device__ __forceinline__ double py_mod(double x) {
+    const double m = (double)M;
+    double r = M == 2 ? x - 2.0 * trunc(0.5 * x) : x - trunc(x);
     if (r != 0.0) {
-        if ((r < 0.0) != (m < 0.0)) r += m;
+        if (r < 0.0) r += m;
     } else {
-        r = copysign(0.0, m);
+        r = 0.0;
     }
     return r;
 }
@@ -121,79 +125,125 @@ __device__ __forceinline__ double sqrt_s(double s, bool f32) {
     return f32 ? (double)__fsqrt_rn((float)s) : sqrt(s);
 }
 
-static __device__ __noinline__ double palette_norm(double s, int scheme, double off, double density,
-                                                   double contrast, bool f32) {
-    const double dens = density <= 0.0 ? 1.0 : density;
-    const double cont = contrast <= 0.0 ? 1.0 : contrast;
-    const double kTwoPi = 6.28318530718;
-    switch (scheme) {
-    case 1:
-        return tri_wave(py_mod(log(s * cont + 1.0) * (0.45 * dens) + off * 2.0, 2.0));
+// What a transfer function takes from the frame alone: computed once per block or thread (a tanh,
+// an exp or a division each) instead of once per sample.
+struct Palette {
+    double dens, cont, off, off2, m, k, scale;
+};
+
+constexpr double kTwoPi = 6.28318530718;
+
+// hist: the histogram transfer (scheme 11), where m is 1 / max(1, max_iter).
+__device__ __forceinline__ Palette palette_of(const ApFrameParams& p, bool hist) {
+    Palette c;
+    c.dens = p.color_density <= 0.0 ? 1.0 : p.color_density;
+    c.cont = p.color_contrast <= 0.0 ? 1.0 : p.color_contrast;
+    c.off = p.palette_offset;
+    c.off2 = c.off * 2.0;
+    c.m = c.k = c.scale = 0.0;
+    if (hist) {
+        c.m = 1.0 / fmax(1.0, (double)p.max_iter);
+        return c;
+    }
+    switch (p.scheme_id) {
+    case 1: c.m = 0.45 * c.dens; break;
     case 2: {
-        const double tri = tri_wave(py_mod(sqrt_s(s, f32) * (0.125 * dens) + off * 2.0, 2.0));
-        const double k = 4.0 * cont;
-        const double td = tanh(0.5 * k);
-        const double scale = fabs(td) > 1e-7 ? 0.5 / td : 0.5186574;
-        return 0.5 + tanh((tri - 0.5) * k) * scale;
+        c.m = 0.125 * c.dens;
+        c.k = 4.0 * c.cont;
+        const double td = tanh(0.5 * c.k);
+        c.scale = fabs(td) > 1e-7 ? 0.5 / td : 0.5186574;
+        break;
     }
     case 3: {
-        const double tri = tri_wave(py_mod(sqrt_s(s, f32) * (0.125 * dens) + off * 2.0, 2.0));
-        const double k = 3.0 * cont;
-        const double ed = exp(k) - 1.0;
-        const double scale = fabs(ed) > 1e-7 ? 1.0 / ed : 0.0523957;
-        return (exp(k * tri) - 1.0) * scale;
+        c.m = 0.125 * c.dens;
+        c.k = 3.0 * c.cont;
+        const double ed = exp(c.k) - 1.0;
+        c.scale = fabs(ed) > 1e-7 ? 1.0 / ed : 0.0523957;
+        break;
     }
-    case 4: {
-        const double tri = tri_wave(py_mod(sqrt_s(s, f32) * (0.5 * dens) + off * 2.0, 2.0));
-        return cont != 1.0 ? pow(tri, cont) : tri;
+    case 4: c.m = 0.5 * c.dens; break;
+    case 5:
+        c.m = 0.05 * c.dens;
+        c.k = 1.61803398875 * c.cont;
+        break;
+    case 6: c.m = 0.08 * c.dens; break;
+    case 7: {
+        c.m = 0.05 * c.dens;
+        const double b = 0.5 * c.cont;
+        c.k = b;
+        const double ns = 1.0 + b + b * b + b * b * b;
+        c.scale = ns > 1e-7 ? 0.5 / ns : 0.26666666666666666;
+        break;
+    }
+    case 8: c.m = 0.1 * c.dens; break;
+    case 9:
+        c.m = 0.04 * c.dens;
+        c.k = 0.00008 * c.dens * c.cont;
+        break;
+    case 10: c.m = -0.06 * c.cont; break;
+    default: c.m = 0.125 * c.dens;
+    }
+    return c;
+}
+
+__device__ __forceinline__ double palette_norm(const Palette& c, double s, int scheme, bool f32) {
+    switch (scheme) {
+    case 1: return tri_wave(py_mod<2>(log(s * c.cont + 1.0) * c.m + c.off2));
+    case 2: {
+        const double tri = tri_wave(py_mod<2>(sqrt_s(s, f32) * c.m + c.off2));
+        return 0.5 + tanh((tri - 0.5) * c.k) * c.scale;
+    }
+    case 3: {
+        const double tri = tri_wave(py_mod<2>(sqrt_s(s, f32) * c.m + c.off2));
+        return (exp(c.k * tri) - 1.0) * c.scale;
     }
     case 5: {
-        const double ang = s * (0.05 * dens) + off * kTwoPi;
-        const double ratio = 1.61803398875 * cont;
-        return 0.5 + 0.25 * (sin(ang) + sin(ang * ratio));
+        const double ang = s * c.m + c.off * kTwoPi;
+        return 0.5 + 0.25 * (sin(ang) + sin(ang * c.k));
     }
     case 6: {
-        const double ang = s * (0.08 * dens) + off * kTwoPi;
+        const double ang = s * c.m + c.off * kTwoPi;
         const double val = 0.5 * (1.0 - cos(ang));
-        return cont != 1.0 ? pow(val, cont) : val;
+        return c.cont != 1.0 ? pow(val, c.cont) : val;
     }
     case 7: {
-        const double ph = s * (0.05 * dens) + off * kTwoPi;
-        const double b = 0.5 * cont;
+        const double ph = s * c.m + c.off * kTwoPi;
+        const double b = c.k;
         const double wave = sin(ph) + b * sin(ph * 2.0 + 1.2) + (b * b) * sin(ph * 4.0 + 2.4) +
                             (b * b * b) * sin(ph * 8.0 + 3.6);
-        const double ns = 1.0 + b + b * b + b * b * b;
-        const double scale = ns > 1e-7 ? 0.5 / ns : 0.26666666666666666;
-        return 0.5 + scale * wave;
+        return 0.5 + c.scale * wave;
     }
     case 8: {
-        double tri = tri_wave(py_mod(sqrt_s(s, f32) * (0.1 * dens) + off * 2.0, 2.0));
-        if (cont != 1.0) tri = pow(tri, cont);
+        double tri = tri_wave(py_mod<2>(sqrt_s(s, f32) * c.m + c.off2));
+        if (c.cont != 1.0) tri = pow(tri, c.cont);
         const double t2 = tri * tri;
         return t2 * tri * (tri * (tri * 6.0 - 15.0) + 10.0);
     }
     case 9: {
-        const double ang = s * (0.04 * dens) + (s * s) * (0.00008 * dens * cont) + off * kTwoPi;
+        const double ang = s * c.m + (s * s) * c.k + c.off * kTwoPi;
         return 0.5 + 0.5 * sin(ang);
     }
     case 10: {
-        const double raw = py_mod(1.0 - exp(-0.06 * cont * sqrt(s * dens)) + off, 1.0);
+        const double raw = py_mod<1>(1.0 - exp(c.m * sqrt(s * c.dens)) + c.off);
         return raw >= 0.0 ? raw : raw + 1.0;
     }
-    default: {  // scheme 0 and every id above 10
-        const double tri = tri_wave(py_mod(sqrt_s(s, f32) * (0.125 * dens) + off * 2.0, 2.0));
-        return cont != 1.0 ? pow(tri, cont) : tri;
+    default: {  // scheme 0, 4 and every id above 10
+        const double tri = tri_wave(py_mod<2>(sqrt_s(s, f32) * c.m + c.off2));
+        return c.cont != 1.0 ? pow(tri, c.cont) : tri;
     }
     }
 }
 
+// The same in one function for kernels that colour beside other work.
+static __device__ __noinline__ double palette_norm_call(const Palette& c, double s, int scheme, bool f32) {
+    return palette_norm(c, s, scheme, f32);
+}
+
 // Histogram-equalised transfer (math_core/cuda_kernels.py:237-259).
-__device__ __forceinline__ double cdf_norm(double s, int max_iter, const float* __restrict__ cdf,
-                                           int num_bins, double off, double density,
-                                           double contrast) {
+__device__ __forceinline__ double cdf_norm(const Palette& pc, double s, const float* __restrict__ cdf,
+                                           int num_bins, double contrast) {
     if (s < 0.0) return -1.0;
-    const double inv_max = 1.0 / fmax(1.0, (double)max_iter);
-    const double pos = (s * inv_max) * (double)(num_bins - 1);
+    const double pos = (s * pc.m) * (double)(num_bins - 1);
     const int k = (int)pos;
     double c;
     if (k >= num_bins - 1) {
@@ -206,8 +256,7 @@ __device__ __forceinline__ double cdf_norm(double s, int max_iter, const float* 
         c = (double)c0 + frac * (double)__fsub_rn(c1, c0);
     }
     if (contrast != 1.0 && contrast > 0.0) c = pow(c, contrast);
-    const double dens = density <= 0.0 ? 1.0 : density;
-    return tri_wave(py_mod(c * (2.0 * dens) + off * 2.0, 2.0));
+    return tri_wave(py_mod<2>(c * (2.0 * pc.dens) + pc.off2));
 }
 
 // 2048-entry LUT lerp (math_core/cuda_kernels.py:157-168).
@@ -224,29 +273,34 @@ __device__ __forceinline__ void lut_lerp(const float* __restrict__ lut, double n
     b = (double)__ldg(lut + i0 * 3 + 2) * inv + (double)__ldg(lut + i1 * 3 + 2) * frac;
 }
 
+// A colour component as its integer: int conversion where it is in range (LUT values are 0..65535),
+// the 64-bit one of the reference's casts otherwise.
+__device__ __forceinline__ unsigned colour_int(double v) {
+    const double t = v + 0.5;
+    return fabs(t) < 1073741824.0 ? (unsigned)(int)t : (unsigned)(long long)t;
+}
+
 __device__ __forceinline__ void store_rgb(void* rgb, int is_hdr, size_t idx, double r, double g,
                                           double b) {
     if (is_hdr) {
         uint16_t* o = static_cast<uint16_t*>(rgb) + idx * 3;
-        o[0] = (uint16_t)(long long)(r + 0.5);
-        o[1] = (uint16_t)(long long)(g + 0.5);
-        o[2] = (uint16_t)(long long)(b + 0.5);
+        o[0] = (uint16_t)colour_int(r);
+        o[1] = (uint16_t)colour_int(g);
+        o[2] = (uint16_t)colour_int(b);
     } else {
         uint8_t* o = static_cast<uint8_t*>(rgb) + idx * 3;
-        o[0] = (uint8_t)(long long)(r + 0.5);
-        o[1] = (uint8_t)(long long)(g + 0.5);
-        o[2] = (uint8_t)(long long)(b + 0.5);
+        o[0] = (uint8_t)colour_int(r);
+        o[1] = (uint8_t)colour_int(g);
+        o[2] = (uint8_t)colour_int(b);
     }
 }
 
-// Colour of one smooth value under the frame's transfer function.
-__device__ __forceinline__ void colour_of(const ApFrameParams& p, const float* __restrict__ lut,
+// Colour of one smooth value under the frame's transfer function (c = palette_of(p, hist)).
+__device__ __forceinline__ void colour_of(const ApFrameParams& p, const Palette& c, const float* __restrict__ lut,
                                           const float* __restrict__ cdf, bool hist, double s,
                                           double& r, double& g, double& b) {
-    const double norm = hist ? cdf_norm(s, p.max_iter, cdf, p.num_bins, p.palette_offset,
-                                        p.color_density, p.color_contrast)
-                             : palette_norm(s, p.scheme_id, p.palette_offset, p.color_density,
-                                            p.color_contrast, p.arith == AP_ARITH_REF_CPU);
+    const double norm = hist ? cdf_norm(c, s, cdf, p.num_bins, p.color_contrast)
+                             : palette_norm_call(c, s, p.scheme_id, p.arith == AP_ARITH_REF_CPU);
     lut_lerp(lut, norm, r, g, b);
 }
 

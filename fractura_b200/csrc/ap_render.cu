@@ -44,6 +44,12 @@ __device__ __forceinline__ SampleOut sample_at(const ApFrameParams& p, const ApF
 template <int TIER, int ARITH, int KIND>
 __global__ void __launch_bounds__(kTile * kTile) render_pass_kernel(const ApFrameParams p,
                                                           const ApFrameBuffers b) {
+    __shared__ Palette palette;
+    const bool rgb = !(p.flags & AP_FLAG_NO_RGB), hist_colour = (p.flags & AP_FLAG_HIST_COLOUR) != 0;
+    if (rgb) {
+        if (threadIdx.x == 0) palette = palette_of(p, hist_colour);
+        __syncthreads();
+    }
     const int i = blockIdx.x * kTile + (threadIdx.x & (kTile - 1));
     const int j = blockIdx.y * kTile + (threadIdx.x / kTile);
     if (i >= p.width || j >= p.height) return;
@@ -61,10 +67,9 @@ __global__ void __launch_bounds__(kTile * kTile) render_pass_kernel(const ApFram
         reinterpret_cast<int4*>(b.counters)[idx] = make_int4(o.iters, o.leaps, o.iters2, 0);
     }
     if (kPert && b.glitch_out) b.glitch_out[idx] = o.glitch > 0 ? 1 : 0;
-    if (!(p.flags & AP_FLAG_NO_RGB)) {
+    if (rgb) {
         double r = 0.0, g = 0.0, bb = 0.0;
-        if ((double)o.s >= 0.0)
-            colour_of(p, b.lut, b.cdf, (p.flags & AP_FLAG_HIST_COLOUR) != 0, (double)o.s, r, g, bb);
+        if ((double)o.s >= 0.0) colour_of(p, palette, b.lut, b.cdf, hist_colour, (double)o.s, r, g, bb);
         store_rgb(b.rgb, p.is_hdr, idx, r, g, bb);
     }
 }
@@ -92,8 +97,12 @@ __global__ void __launch_bounds__(32 * kSuperWarps) supersample_kernel(const ApF
     __shared__ double red[kSuperWarps][32], green[kSuperWarps][32], blue[kSuperWarps][32];
     __shared__ int work[kSuperWarps][32][4];  // iterations, leaps, stage-2 steps, glitch
     __shared__ uint8_t list[kSuperWarps][32 * kPatches];
+    __shared__ Palette palette;
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const bool hist_colour = hist_resolve || (p.flags & AP_FLAG_HIST_COLOUR);
+    if (threadIdx.x == 0) palette = palette_of(p, hist_colour);
+    __syncthreads();
     const int i0 = blockIdx.x * (8 * kPatches), j0 = (blockIdx.y * kSuperWarps + warp) * 4;
     if (j0 >= p.height) return;
     int n = 0;
@@ -110,7 +119,6 @@ __global__ void __launch_bounds__(32 * kSuperWarps) supersample_kernel(const ApF
         n += __popc(sel);
     }
     __syncwarp();
-    const bool hist_colour = hist_resolve || (p.flags & AP_FLAG_HIST_COLOUR);
     const bool write_iter = hist_resolve ? (p.rebase_pass > 0) : ((p.flags & AP_FLAG_ITER_LAST_SUB) != 0);
     const int f = p.factor, f2 = f * f;
     auto place = [&](int q, int& i, int& j) {
@@ -132,7 +140,7 @@ __global__ void __launch_bounds__(32 * kSuperWarps) supersample_kernel(const ApF
                 const SampleOut o = sample_at<TIER, ARITH, KIND>(p, b, (double)(i * f + sub % f),
                                                                   (double)(j * f + sub / f));
                 double r = 0.0, g = 0.0, bb = 0.0;
-                if ((double)o.s >= 0.0) colour_of(p, b.lut, b.cdf, hist_colour, (double)o.s, r, g, bb);
+                if ((double)o.s >= 0.0) colour_of(p, palette, b.lut, b.cdf, hist_colour, (double)o.s, r, g, bb);
                 red[warp][lane] = r;
                 green[warp][lane] = g;
                 blue[warp][lane] = bb;

@@ -204,7 +204,7 @@ __global__ void __launch_bounds__(kStrictThreads) strict_eval_kernel(
     const size_t idx = (size_t)r * p.width + c;
     b.iter_map[idx] = s;
     double cr = 0.0, cg = 0.0, cb = 0.0;
-    if (s >= 0.0f) colour_of(p, b.lut, b.cdf, hist != 0, (double)s, cr, cg, cb);
+    if (s >= 0.0f) colour_of(p, palette_of(p, hist != 0), b.lut, b.cdf, hist != 0, (double)s, cr, cg, cb);
     store_rgb(b.rgb, p.is_hdr, idx, cr, cg, cb);
     if (b.glitch_out) b.glitch_out[idx] = 0;
 }
