@@ -120,3 +120,12 @@ def test_engine_compute_bbsa_coeffs_cuda_guards():
     assert engine.compute_bbsa_coeffs_cuda(re, im, m["ref_len"], 1e-160, 0, bbsa_order=32) == zero
     assert engine.compute_bbsa_coeffs_cuda(re, im, 1, 1e-160, 0) == zero                     # ref_len < 2
     assert engine.compute_bbsa_coeffs_cuda(re, im, m["ref_len"], 0.0, 0) == zero             # max_r <= 0
+
+
+def test_zero_coefficients_keep_their_signs():
+    """Order-4 steps of a Julia series whose quadratic products all underflow: Re a4 is a sum of zeros,
+    and its sign is that of -fma(-a1r, a3r, a1i a3i), not of fma(a1r, a3r, -(a1i a3i))."""
+    re, im, out = np.full(3, -0.3), np.full(3, 0.2), np.full(17, 5.0)
+    _lib.check(_lib.load().ap_bbsa_coeffs(re.ctypes.data_as(C.c_void_p), im.ctypes.data_as(C.c_void_p), 3, 1e-200, 2,
+                                          1e-6, 4, 0, 0.0, 0.0, 0, out.ctypes.data_as(C.c_void_p)), "ap_bbsa_coeffs")
+    assert out[7] == 0.0 and np.signbit(out[7])
