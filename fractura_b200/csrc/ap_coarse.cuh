@@ -217,7 +217,7 @@ __device__ __forceinline__ void leap_delta(const double4 e, double& dzx, double&
     dzy = ny;
 }
 
-// One step of the delta at the orbit value (rx, ry), in the profile's operations.
+// One step of the delta at the orbit value (rx, ry), in the profile's roundings.
 template <int ARITH, int FT>
 __device__ __forceinline__ void delta_step(const ApFrameParams& p, double rx, double ry, double& dzx, double& dzy,
                                            double dcx, double dcy) {
@@ -230,11 +230,11 @@ __device__ __forceinline__ void delta_step(const ApFrameParams& p, double rx, do
             nx = fma(ax, dzx, fma(-ay, dzy, dcx));
             ny = fma(ax, dzy, fma(ay, dzx, dcy));
         } else if (kCpu) {
-            nx = (2.0 * rx + dzx) * dzx - (2.0 * ry + dzy) * dzy + dcx;
-            ny = 2.0 * ((rx + dzx) * dzy + ry * dzx) + dcy;
+            nx = twice_plus(rx, dzx) * dzx - twice_plus(ry, dzy) * dzy + dcx;
+            ny = twice_plus((rx + dzx) * dzy + ry * dzx, dcy);
         } else {
-            nx = fma(2.0 * rx + dzx, dzx, fma(-(2.0 * ry + dzy), dzy, dcx));
-            ny = fma(2.0, fma(rx + dzx, dzy, ry * dzx), dcy);
+            nx = fma(twice_plus(rx, dzx), dzx, fma(-twice_plus(ry, dzy), dzy, dcx));
+            ny = twice_plus(fma(rx + dzx, dzy, ry * dzx), dcy);
         }
         dzx = nx;
         dzy = ny;
@@ -247,10 +247,10 @@ __device__ __forceinline__ void delta_step(const ApFrameParams& p, double rx, do
             dzy = fma(2.0, fma(fabs(rx), ddy, fma(fabs(ry), ddx, ddx * ddy)), -dcy);
             dzx = nx;
         } else {
-            const double ax = 2.0 * rx + dzx, ay = 2.0 * ry + dzy;
+            const double ax = twice_plus(rx, dzx), ay = twice_plus(ry, dzy);
             const double nx = ax * dzx - ay * dzy + dcx;
             const double ddx = fold_delta(rx, zx, dzx, ax), ddy = fold_delta(ry, zy, dzy, ay);
-            dzy = 2.0 * (fabs(rx) * ddy + fabs(ry) * ddx + ddx * ddy) - dcy;
+            dzy = twice_plus(fabs(rx) * ddy + fabs(ry) * ddx + ddx * ddy, -dcy);
             dzx = nx;
         }
     } else if (kFast) {

@@ -138,20 +138,21 @@ __device__ __forceinline__ SampleOut rebase_sample_at(const ApFrameParams& p, co
                 nx = fma(ax, dzx, fma(-ay, dzy, dcx));
                 ny = fma(ax, dzy, fma(ay, dzx, dcy));
             } else if (kCpu) {
-                nx = (2.0 * rx + dzx) * dzx - (2.0 * ry + dzy) * dzy + dcx;
-                ny = 2.0 * ((rx + dzx) * dzy + ry * dzx) + dcy;
+                nx = twice_plus(rx, dzx) * dzx - twice_plus(ry, dzy) * dzy + dcx;
+                ny = twice_plus((rx + dzx) * dzy + ry * dzx, dcy);
             } else {
-                nx = fma(2.0 * rx + dzx, dzx, fma(-(2.0 * ry + dzy), dzy, dcx));
+                nx = fma(twice_plus(rx, dzx), dzx, fma(-twice_plus(ry, dzy), dzy, dcx));
                 ny = fma(2.0, fma(rx + dzx, dzy, ry * dzx), dcy);
             }
             dzx = nx;
             dzy = ny;
         } else if (ft == 1) {
-            const double nx = (2.0 * rx + dzx) * dzx - (2.0 * ry + dzy) * dzy + dcx;
+            const double ax = twice_plus(rx, dzx), ay = twice_plus(ry, dzy);
+            const double nx = ax * dzx - ay * dzy + dcx;
             const double sx = rx >= 0.0 ? 1.0 : -1.0, sy = ry >= 0.0 ? 1.0 : -1.0;
-            const double ddx = (rx + dzx) * sx >= 0.0 ? sx * dzx : -sx * (2.0 * rx + dzx);
-            const double ddy = (ry + dzy) * sy >= 0.0 ? sy * dzy : -sy * (2.0 * ry + dzy);
-            dzy = 2.0 * (fabs(rx) * ddy + fabs(ry) * ddx + ddx * ddy) - dcy;
+            const double ddx = (rx + dzx) * sx >= 0.0 ? sx * dzx : -sx * ax;
+            const double ddy = (ry + dzy) * sy >= 0.0 ? sy * dzy : -sy * ay;
+            dzy = twice_plus(fabs(rx) * ddy + fabs(ry) * ddx + ddx * ddy, -dcy);
             dzx = nx;
         } else {
             double pr = dzx, pi = dzy, qr = rx, qi = ry;
@@ -271,20 +272,21 @@ __device__ __forceinline__ SampleOut perturb_sample_at(const ApFrameParams& p,
         if (ft == 0 || ft == 2) {
             double nx, ny;
             if (kCpu) {
-                nx = (2.0 * rx + dzx) * dzx - (2.0 * ry + dzy) * dzy + dcpx;
-                ny = 2.0 * ((rx + dzx) * dzy + ry * dzx) + dcpy;
+                nx = twice_plus(rx, dzx) * dzx - twice_plus(ry, dzy) * dzy + dcpx;
+                ny = twice_plus((rx + dzx) * dzy + ry * dzx, dcpy);
             } else {
-                nx = fma(2.0 * rx + dzx, dzx, fma(-(2.0 * ry + dzy), dzy, dcpx));
+                nx = fma(twice_plus(rx, dzx), dzx, fma(-twice_plus(ry, dzy), dzy, dcpx));
                 ny = fma(2.0, fma(rx + dzx, dzy, ry * dzx), dcpy);
             }
             dzx = nx;
             dzy = ny;
         } else if (ft == 1 || ft == 3) {
-            const double nx = (2.0 * rx + dzx) * dzx - (2.0 * ry + dzy) * dzy + dcpx;
+            const double ax = twice_plus(rx, dzx), ay = twice_plus(ry, dzy);
+            const double nx = ax * dzx - ay * dzy + dcpx;
             const double sx = rx >= 0.0 ? 1.0 : -1.0, sy = ry >= 0.0 ? 1.0 : -1.0;
-            const double ddx = (rx + dzx) * sx >= 0.0 ? sx * dzx : -sx * (2.0 * rx + dzx);
-            const double ddy = (ry + dzy) * sy >= 0.0 ? sy * dzy : -sy * (2.0 * ry + dzy);
-            dzy = 2.0 * (fabs(rx) * ddy + fabs(ry) * ddx + ddx * ddy) - dcpy;
+            const double ddx = (rx + dzx) * sx >= 0.0 ? sx * dzx : -sx * ax;
+            const double ddy = (ry + dzy) * sy >= 0.0 ? sy * dzy : -sy * ay;
+            dzy = twice_plus(fabs(rx) * ddy + fabs(ry) * ddx + ddx * ddy, -dcpy);
             dzx = nx;
         } else {
             double pr = dzx, pi = dzy, qr = rx, qi = ry;
@@ -592,11 +594,14 @@ __device__ __forceinline__ SampleOut floatexp_sample_at(const ApFrameParams& p,
         }
 
         if (KIND == 0) {
-            double lx = 2.0 * (rx * dzx - ry * dzy);
-            double ly = 2.0 * (rx * dzy + ry * dzx);
+            const double hx = rx * dzx - ry * dzy, hy = rx * dzy + ry * dzx;
+            double lx, ly;
             if (eff_exp >= -1020) {
-                lx += (dzx * dzx - dzy * dzy) * sn;
-                ly += (2.0 * dzx * dzy) * sn;
+                lx = twice_plus(hx, (dzx * dzx - dzy * dzy) * sn);
+                ly = twice_plus(hy, (2.0 * dzx * dzy) * sn);
+            } else {
+                lx = 2.0 * hx;
+                ly = 2.0 * hy;
             }
             dzx = lx + cxs;
             dzy = ly + cys;
@@ -609,9 +614,9 @@ __device__ __forceinline__ SampleOut floatexp_sample_at(const ApFrameParams& p,
                 else { fx = -sx; ex = eff_exp <= 1020 ? ((-sx * 2.0) * rx) * inv : 0.0; }
                 if ((ry + dzy * sn) * sy >= 0.0) { fy = sy; ey = 0.0; }
                 else { fy = -sy; ey = eff_exp <= 1020 ? ((-sy * 2.0) * ry) * inv : 0.0; }
-                const double lx = (2.0 * rx + dzx * sn) * dzx - (2.0 * ry + dzy * sn) * dzy + cxs;
+                const double lx = twice_plus(rx, dzx * sn) * dzx - twice_plus(ry, dzy * sn) * dzy + cxs;
                 const double dxn = fx * dzx + ex, dyn = fy * dzy + ey;
-                const double ly = 2.0 * (fabs(rx) * dyn + fabs(ry) * dxn + dxn * dyn * sn) - cys;
+                const double ly = twice_plus(fabs(rx) * dyn + fabs(ry) * dxn + dxn * dyn * sn, -cys);
                 dzx = lx;
                 dzy = ly;
             } else {  // math_core/cuda_kernels.py:964-985
