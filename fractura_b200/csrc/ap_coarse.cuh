@@ -466,6 +466,7 @@ __device__ __forceinline__ void pixel_advance(const ApFrameParams& p, const ApFr
         bool paused = false;
         constexpr int kKind = FT == kFtQuad ? kKindQuad : FT == kFtShip ? kKindShip : kKindMulti;
         const bool growing = fp64_growing(kKind, cx, cy, p.gen_n, p.gen_kr, p.gen_ki);
+        const bool doubles = fp64_doubles(zy, cy);
         int tested = 0;  // steps to test one by one before the next block
         while (k < max_iter) {
             if (BUDGET && --budget < 0) {
@@ -475,7 +476,7 @@ __device__ __forceinline__ void pixel_advance(const ApFrameParams& p, const ApFr
             // blocks tested at their end only, as in direct iteration (fp64_orbit, ap_fp64.cuh)
             if (growing && tested == 0 && k + kBlock <= max_iter) {
                 const double bx = zx, by = zy;
-                for_degree(kKind, p.gen_n, [&](auto n) {
+                for_degree(kKind, p.gen_n, doubles, [&](auto n) {
 #pragma unroll
                     for (int t = 0; t < kBlock; ++t)
                         fp64_step<AP_ARITH_REF_CUDA, kKind, n()>(zx, zy, zx * zx, zy * zy, cx, cy, p.gen_n, p.gen_kr,

@@ -14,15 +14,20 @@ namespace ap {
 
 constexpr int kKindQuad = 0, kKindShip = 1, kKindMulti = 4;
 
-// Calls f with the Multibrot degree as a compile-time constant for 2..5, else (and for the
-// quadratic kinds) with 0.
+// Calls f with the Multibrot degree as a compile-time constant for 2..5, else with 0; for the
+// quadratic kinds with 1 where fp64_step may fuse the doubling (`doubles`), else with 0.
 template <int N>
 struct Degree {
     __host__ __device__ constexpr int operator()() const { return N; }
 };
 template <typename F>
-__device__ __forceinline__ void for_degree(int kind, int n, F&& f) {
-    switch (kind == kKindMulti ? n : 0) {
+__device__ __forceinline__ void for_degree(int kind, int n, bool doubles, F&& f) {
+    if (kind != kKindMulti) {
+        if (doubles) f(Degree<1>());
+        else f(Degree<0>());
+        return;
+    }
+    switch (n) {
     case 2: f(Degree<2>()); break;
     case 3: f(Degree<3>()); break;
     case 4: f(Degree<4>()); break;
@@ -31,8 +36,18 @@ __device__ __forceinline__ void for_degree(int kind, int n, F&& f) {
     }
 }
 
-// One step of z in the profile's operations; zx2, zy2 the squares (quadratic kinds).  N: the
-// Multibrot degree where it is known at compile time (2..5, the powers unrolled), else 0.
+// Whether fma(2, zx zy, cy) is (2 zx) zy + cy in every step from zy on, so that a quadratic step of the
+// CUDA profile is six FP64 operations instead of seven.  The two products differ only below the
+// smallest normal number, 2^-1022, where the sum with |cy| >= 2^-960 is cy for both; and they are zeros
+// of one sign throughout where cy = zy = 0.  1283x721 Julia with 2x SSAA 733 -> 681 us; second stages of
+// perturbation (1279x719 at 1e-26 with a series, a frame) 1810 -> 1752 us.
+__device__ __forceinline__ bool fp64_doubles(double zy, double cy) {
+    return fabs(cy) >= 0x1p-960 || (cy == 0.0 && zy == 0.0);
+}
+
+// One step of z in the profile's roundings; zx2, zy2 the squares (quadratic kinds).  N: the
+// Multibrot degree where it is known at compile time (2..5, the powers unrolled), else 0; for the
+// quadratic kinds 1 where fp64_doubles holds, else 0.
 template <int ARITH, int KIND, int N>
 __device__ __forceinline__ void fp64_step(double& zx, double& zy, double zx2, double zy2, double cx, double cy,
                                           int n, double kr, double ki) {
@@ -43,7 +58,7 @@ __device__ __forceinline__ void fp64_step(double& zx, double& zy, double zx2, do
             zx = (cx - zy2) + zx2;
             zy = nzy;
         } else {
-            zy = 2.0 * zx * zy + cy;
+            zy = N == 1 ? twice_plus(zx * zy, cy) : 2.0 * zx * zy + cy;
             zx = zx2 - zy2 + cx;
         }
     } else if (KIND == kKindShip) {
@@ -53,7 +68,7 @@ __device__ __forceinline__ void fp64_step(double& zx, double& zy, double zx2, do
             zx = (cx + zx2) - zy2;
             zy = nzy;
         } else {
-            zy = 2.0 * ax * ay - cy;
+            zy = N == 1 ? twice_plus(ax * ay, -cy) : 2.0 * ax * ay - cy;
             zx = zx2 - zy2 + cx;
         }
     } else {
@@ -143,13 +158,18 @@ __device__ __forceinline__ int fp64_orbit(double zx, double zy, double cx, doubl
         }
         if (stop == max_iter) break;
         stop = max_iter;
+        const bool doubles = ARITH != AP_ARITH_REF_CPU && fp64_doubles(zy, cy);
         double sx = zx, sy = zy;  // the z that block ends are compared with
         int left = 1, window = 1;
         while (k + kBlock <= max_iter) {
             const double bx = zx, by = zy;
+            auto block = [&](auto form) {
 #pragma unroll
-            for (int t = 0; t < kBlock; ++t)
-                fp64_step<ARITH, KIND, N>(zx, zy, zx * zx, zy * zy, cx, cy, n, kr, ki);
+                for (int t = 0; t < kBlock; ++t)
+                    fp64_step<ARITH, KIND, form()>(zx, zy, zx * zx, zy * zy, cx, cy, n, kr, ki);
+            };
+            if (KIND != kKindMulti && doubles) block(Degree<1>());
+            else block(Degree<N>());
             if (!(fp64_mag2<ARITH, KIND>(zx, zy) <= kBailout)) {
                 zx = bx;
                 zy = by;
@@ -196,7 +216,7 @@ __device__ __forceinline__ SampleOut fp64_sample(double x, double y, const ApFra
     double mag2 = 0.0;
     int steps = 0, k;
     if (ft == 4) {
-        for_degree(kKindMulti, n, [&](auto degree) {
+        for_degree(kKindMulti, n, false, [&](auto degree) {
             k = fp64_orbit<ARITH, kKindMulti, degree()>(zx, zy, cx, cy, p.max_iter, growing, n, kr, ki, mag2, steps);
         });
     } else if (ft & 1) {
