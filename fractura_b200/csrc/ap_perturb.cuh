@@ -485,6 +485,16 @@ struct LinearFit {
 // starts are never used: the reference maps orders 4/8 to chained BLA here.
 // The powers of two that depend on the exponent alone, and dc in units of it, are kept between
 // renormalisations that change it.  KIND: 0 z^2 + c, 1 Burning Ship, 4 Multibrot.
+//
+// Steps of z^2 + c with eff_exp >= -50 run on the delta itself instead of its mantissas (`plain`
+// below): every operation of the scaled step is the plain one times a power of two, so the values
+// are the same as long as nothing under- or overflows.  That holds while both components are in
+// [2^-100, 2^100), which each step is checked for before it counts: their products and squares are
+// normal; a product with a component of Z that is itself below 2^-800 may be subnormal, but then
+// it, exact or not, is far below half a unit of what it is added to, or the step's result is below
+// 2^-100 and the scaled step takes it.  dc, below 2^-200 there, is below half a unit of a component.
+// The exponent is kept up with, so that its thresholds fall where they fell.  A 1920x1080 view at
+// 1e-1000 (22 leaps and 16 such steps a pixel) 1150 -> 1110 us a frame.
 template <int ARITH, int KIND>
 __device__ __forceinline__ SampleOut floatexp_sample_at(const ApFrameParams& p,
                                                         const ApFrameBuffers& b, double sub_i,
@@ -526,7 +536,55 @@ __device__ __forceinline__ SampleOut floatexp_sample_at(const ApFrameParams& p,
     };
     refresh();
 
+    constexpr int kPlainLow = (1023 - 100) << 20, kPlainHigh = (1023 + 100) << 20;
+    const bool plain = KIND == 0 && E >= 300 && fabs(dcpx) < 0x1p100 && fabs(dcpy) < 0x1p100 && (!has_bla || rows);
     while (k < ref_len) {
+        if (KIND == 0 && plain && eff_exp >= -50) {
+            double x = dzx * sn, y = dzy * sn;
+            const int hx = __double2hiint(x) & 0x7fffffff, hy = __double2hiint(y) & 0x7fffffff;
+            bool stay = min(hx, hy) >= kPlainLow && max(hx, hy) < kPlainHigh;
+            const int k_in = k;
+            while (stay) {
+                const double rx = __ldg(re + k), ry = __ldg(im + k);
+                const double x2 = x * x, y2 = y * y;
+                if (has_bla && k < ref_len - 1 && x2 + y2 < __ldg(rows + (size_t)k * 16)) break;  // a leap
+                const double zx = rx + x, zy = ry + y;
+                const double mag2 = zx * zx + zy * zy;
+                if (mag2 > kBailout) {
+                    SampleOut o = escaped_sample(k, mag2, inv_ln);
+                    o.glitch = glitch;
+                    return done(o, k);
+                }
+                // the test's own comparison first: its logarithms only where that is near
+                if (strict && k > 15 && mag2 < 2e-6 * (rx * rx + ry * ry)) {
+                    const double inv = pow2_f64(-eff_exp);
+                    if (floatexp_glitch(rx, ry, x * inv, y * inv, eff_exp)) glitch = 1;
+                }
+                const double nx = twice_plus(rx * x - ry * y, x2 - y2);
+                const double ny = twice_plus(rx * y + ry * x, 2.0 * x * y);
+                const int nhx = __double2hiint(nx) & 0x7fffffff, nhy = __double2hiint(ny) & 0x7fffffff;
+                const int top = max(nhx, nhy);
+                if (min(nhx, nhy) < kPlainLow || top >= kPlainHigh) break;
+                x = nx;
+                y = ny;
+                ++k;
+                const int mantissa = top - eff_exp * (1 << 20);
+                if (mantissa < 0x3ef00000 || mantissa >= 0x40f00000) {
+                    const double inv = pow2_f64(-eff_exp);
+                    double mx = x * inv, my = y * inv;
+                    renorm16(mx, my, z_exp);
+                    eff_exp = z_exp - E;
+                }
+                stay = k < ref_len && eff_exp >= -50;
+            }
+            if (k != k_in) {
+                refresh();
+                const double inv = pow2_f64(-eff_exp);
+                dzx = x * inv;
+                dzy = y * inv;
+                if (k >= ref_len) break;
+            }
+        }
         const double rx = __ldg(re + k), ry = __ldg(im + k);
         if (eff_exp >= -50) {
             const double zx = rx + dzx * sn, zy = ry + dzy * sn;
