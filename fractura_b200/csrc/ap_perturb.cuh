@@ -370,24 +370,19 @@ __device__ __forceinline__ bool renorm16(double& x, double& y, int& e) {
     const int top = max(hx, hy);
     if (top >= 0x3ef00000 && top < 0x40f00000) return false;  // max in [2^-16, 2^16)
     const int et = (top >> 20) - 1023;
-    double mag = py_max(fabs(x), fabs(y));
-    int n = 0;  // 2^-16 rescalings (negative: 2^16)
-    if (et >= 16) {
-        n = et >> 4;  // to below 2^16, or to 2^16 itself
-        if ((et & 15) == 0 && __double_as_longlong(mag) << 12 == 0) --n;
-    } else if (et < -16) {
-        n = -((-16 - et + 15) >> 4);
-    }
-    const int ebot = (min(hx, hy) >> 20);
-    const bool small = n > 0 && ebot - 16 * n <= 0 && x != 0.0 && y != 0.0;
-    if (et > -1023 && et < 1024 && n < 60 && n > -60 && !small) {
-        if (n == 0) return false;
+    // 2^-16 rescalings: to below 2^16, or (negative) up to 2^-16.  2^16 itself stays, so what may be a
+    // power of 2^16 goes by steps.
+    const int n = et >= 16 ? et >> 4 : -((-1 - et) >> 4);
+    const bool power = (et & 15) == 0 && (top & 0xfffff) == 0;
+    const bool small = n > 0 && (min(hx, hy) >> 20) - 16 * n <= 0 && x != 0.0 && y != 0.0;
+    if (et > -1023 && et < 1024 && n < 60 && n > -60 && !power && !small) {
         const double f = __hiloint2double((1023 - 16 * n) << 20, 0);
         x *= f;
         y *= f;
         e += 16 * n;
         return true;
     }
+    double mag = py_max(fabs(x), fabs(y));
     const int before = e;
     while (mag > 65536.0 && isfinite(mag)) {
         x *= 1.52587890625e-05;
@@ -433,42 +428,40 @@ __device__ __forceinline__ bool floatexp_glitch(double rx, double ry, double dzx
 // r^2's high word; it was two square roots a level, up to 16 levels a leap.
 struct LinearFit {
     double x, y;
-    int t, shift;
+    int shift;
+    int yes;       // r^2 from this high word on: admissible
+    long long no;  // r^2 below these bits: not admissible (with 0 and what is negative)
     __device__ __forceinline__ LinearFit(double x_, double y_, int shift_) : x(x_), y(y_), shift(max(-1020, shift_)) {
         const int top = max(__double2hiint(x) & 0x7fffffff, __double2hiint(y) & 0x7fffffff) >> 20;
-        // zero, subnormal or not finite: never decided by the exponent
-        t = top > 0 && top < 2047 ? top - 1023 + shift : INT_MIN;
+        const int e = 2 * (top - 1023 + shift) + 1023;  // the biased exponent of 2^2t
+        // an r^2 of biased exponent >= e + 4 has sqrt(r^2) >= 2^(t+2), one below e has sqrt(r^2) < 2^t;
+        // x, y zero, subnormal or not finite: neither
+        const bool normal = top > 0 && top < 2047;
+        yes = normal ? min(max(e + 4, 1), 2047) << 20 : INT_MAX;
+        no = normal && e > 0 ? (long long)min(e, 2047) << 52 : 1LL;
     }
     __device__ __forceinline__ bool exact(double r_sq) const {
         return r_sq > 0.0 && sqrt(x * x + y * y) * pow2_f64(shift) < sqrt(r_sq);
     }
-    // 1 or 0 where the exponents decide (or r = 0); else `open` is set
-    __device__ __forceinline__ int screen(double r_sq, bool& open) const {
-        const int er = __double2hiint(r_sq) >> 20, es = (er - 1023) >> 1;
-        const bool known = er > 0 && t != INT_MIN;
-        const bool yes = known && t + 2 <= es;
-        open |= !(yes || (known && t > es) || __double_as_longlong(r_sq) == 0);
-        return yes ? 1 : 0;
-    }
     __device__ __forceinline__ bool operator()(const double* __restrict__ r_sq) const {
         const double r = __ldg(r_sq);
-        bool open = false;
-        const int yes = screen(r, open);
-        return open ? exact(r) : yes != 0;
+        if (__double2hiint(r) >= yes) return true;
+        return __double_as_longlong(r) >= no && exact(r);
     }
-    // The largest admissible level of a packed radius row (ap_pack_bla): the admissible levels are
-    // a prefix (0 past the orbit's end and the table's levels), so it is a count, taken in two
-    // rounds of three loads without a branch each.
+    // The largest admissible level of a packed radius row (ap_pack_bla), or -1: radii never increase
+    // with the level (0 past the orbit's end and the table's levels), so it is a count, taken in two
+    // rounds of loads of high words, and the next level decides whether the exponents were enough.
     __device__ __forceinline__ int level(const double* __restrict__ row) const {
-        bool open = false;
+        const int* hi = reinterpret_cast<const int*>(row) + 1;
         int quarter = 0;
 #pragma unroll
-        for (int q = 1; q <= 3; ++q) quarter += screen(__ldg(row + 4 * q), open);
-        int best = 4 * quarter;
+        for (int q = 1; q <= 3; ++q) quarter += __ldg(hi + 8 * q) >= yes ? 1 : 0;
+        int best = 4 * quarter - 1;
+        hi += 8 * quarter;
 #pragma unroll
-        for (int q = 1; q <= 3; ++q) best += screen(__ldg(row + 4 * quarter + q), open);
-        if (open) {
-            best = 0;
+        for (int q = 0; q <= 3; ++q) best += __ldg(hi + 2 * q) >= yes ? 1 : 0;
+        if (best < 15 && __double_as_longlong(__ldg(row + best + 1)) >= no) {
+            best = -1;
             while (best < 15 && exact(__ldg(row + best + 1))) ++best;
         }
         return best;
@@ -600,34 +593,38 @@ __device__ __forceinline__ SampleOut floatexp_sample_at(const ApFrameParams& p,
         if (has_bla && k < ref_len - 1) {
             // |delta|^2 against r^2 in scaled form, or via square roots far below 2^-510
             const bool scaled = eff_exp >= -510;
-            const double dz_mag2 = scaled ? (dzx * dzx + dzy * dzy) * (sn * sn) : 0.0;
-            const LinearFit linear(dzx, dzy, eff_exp);
-            auto fits = [&](const double* r) { return scaled ? dz_mag2 < __ldg(r) : linear(r); };
-            const double* row = rows ? rows + (size_t)k * 16 : b.bla + (size_t)k * 5 + 4;
-            if (fits(row)) {
-                int best = 0;
-                double ar, ai, br, bi;
-                if (rows) {
-                    if (scaled) {
+            int best = -1;
+            if (rows) {
+                const double* row = rows + (size_t)k * 16;
+                if (scaled) {
+                    const double dz_mag2 = (dzx * dzx + dzy * dzy) * (sn * sn);
+                    if (dz_mag2 < __ldg(row)) {
                         int quarter = 0;
 #pragma unroll
                         for (int t = 1; t <= 3; ++t) quarter += dz_mag2 < __ldg(row + 4 * t) ? 1 : 0;
                         best = 4 * quarter;
 #pragma unroll
                         for (int t = 1; t <= 3; ++t) best += dz_mag2 < __ldg(row + 4 * quarter + t) ? 1 : 0;
-                    } else {
-                        best = linear.level(row);
                     }
+                } else {
+                    best = LinearFit(dzx, dzy, eff_exp).level(row);
+                }
+            } else {
+                const double dz_mag2 = scaled ? (dzx * dzx + dzy * dzy) * (sn * sn) : 0.0;
+                const LinearFit linear(dzx, dzy, eff_exp);
+                auto fits = [&](const double* r) { return scaled ? dz_mag2 < __ldg(r) : linear(r); };
+                if (fits(b.bla + (size_t)k * 5 + 4)) {
+                    best = levels - 1;
+                    while (best > 0 && !(k + (1 << best) < ref_len && fits(b.bla + ((size_t)best * L + k) * 5 + 4))) --best;
+                }
+            }
+            if (best >= 0) {
+                double ar, ai, br, bi;
+                if (rows) {
                     const double2* e = reinterpret_cast<const double2*>(rows + L * 16 + ((size_t)k * 16 + best) * 4);
                     const double2 a = __ldg(e), c = __ldg(e + 1);
                     ar = a.x, ai = a.y, br = c.x, bi = c.y;
                 } else {
-                    for (int d = levels - 1; d > 0; --d) {
-                        if (k + (1 << d) < ref_len && fits(b.bla + ((size_t)d * L + k) * 5 + 4)) {
-                            best = d;
-                            break;
-                        }
-                    }
                     const double* e = b.bla + ((size_t)best * L + k) * 5;
                     ar = __ldg(e), ai = __ldg(e + 1), br = __ldg(e + 2), bi = __ldg(e + 3);
                 }
