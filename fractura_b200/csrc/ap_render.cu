@@ -80,105 +80,105 @@ __global__ void __launch_bounds__(kTile * kTile) render_pass_kernel(const ApFram
 // hist_resolve = 1: ssaa_resolve_hist_*_kernel (math_core/cuda_kernels.py:2038-2234).
 // Few pixels are selected (edges, glitches), and the lanes of a warp that ran a pixel each would
 // be mostly idle and take their f x f samples one after the other.  A warp lists the selected
-// pixels of its kPatches 8 x 4 patches and deals out single samples to its lanes; the lane that owns
-// a pixel then adds the pixel's colours up in sample order (sy, then sx), so the sums round as
-// the sequential loop's.  Warps do not wait for one another.  One patch a warp: with two or four
-// the warps over deep edges last longer than the lanes they fill save (1283x721 Julia frame 730 us
-// with one, 800 with two, 915 with four).  Measured against a pixel per lane: 1280x720
-// double-double Burning Ship with 2x SSAA 56.6 -> 53.1 ms; the Julia frame, whose edges are
-// dense, as before.
-constexpr int kPatches = 1;
-constexpr int kSuperWarps = 2;
-
+// pixels of an 8 x 4 patch, takes `share` of them (the share-th of the patch that its block index
+// names; most blocks find none and end) and deals out single samples to its lanes; the lane that
+// owns a pixel then adds the pixel's colours up in sample order (sy, then sx), so the sums round as
+// the sequential loop's.  Measured against a pixel per lane: 1280x720 double-double Burning Ship
+// with 2x SSAA 56.6 -> 53.1 ms with one warp a patch.  Its time was then the tail of the patches whose
+// pixels are all selected and bounded (four rounds of 20000 steps one after the other, the SMs 20 %
+// busy); with the rounds on warps of their own 53.7 -> 44.1 ms, and a 1283x721 Julia frame
+// 681 -> 645 us.
 template <int TIER, int ARITH, int KIND>
-__global__ void __launch_bounds__(32 * kSuperWarps) supersample_kernel(const ApFrameParams p, const ApFrameBuffers b,
-                                                                       const int hist_resolve) {
+__global__ void __launch_bounds__(32) supersample_kernel(const ApFrameParams p, const ApFrameBuffers b,
+                                                         const int hist_resolve, const int share, const int shares) {
     constexpr bool kPert = (TIER >= AP_TIER_PERTURB);
-    __shared__ double red[kSuperWarps][32], green[kSuperWarps][32], blue[kSuperWarps][32];
-    __shared__ int work[kSuperWarps][32][4];  // iterations, leaps, stage-2 steps, glitch
-    __shared__ uint8_t list[kSuperWarps][32 * kPatches];
+    __shared__ double red[32], green[32], blue[32];
+    __shared__ int work[32][4];  // iterations, leaps, stage-2 steps, glitch
+    __shared__ uint8_t list[32];
     __shared__ Palette palette;
     const unsigned full = 0xffffffffu;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const bool hist_colour = hist_resolve || (p.flags & AP_FLAG_HIST_COLOUR);
-    if (threadIdx.x == 0) palette = palette_of(p, hist_colour);
-    __syncthreads();
-    const int i0 = blockIdx.x * (8 * kPatches), j0 = (blockIdx.y * kSuperWarps + warp) * 4;
-    if (j0 >= p.height) return;
-    int n = 0;
-    for (int t = 0; t < kPatches; ++t) {
-        const int i = i0 + 8 * t + (lane & 7), j = j0 + (lane >> 3);
-        bool take = i < p.width && j < p.height;
-        if (take) {
-            const size_t idx = (size_t)j * p.width + i;
-            if (p.rebase_pass > 0 && b.glitch_in[idx] == 0) take = false;
-            else if (hist_resolve ? p.rebase_pass == 0 : p.mode == AP_MODE_EDGE) take = b.edge_mask[idx] != 0;
-        }
-        const unsigned sel = __ballot_sync(full, take);
-        if (take) list[warp][n + __popc(sel & ((1u << lane) - 1u))] = (uint8_t)(32 * t + lane);
-        n += __popc(sel);
+    const int lane = threadIdx.x;
+    const int i0 = (blockIdx.x / shares) * 8, j0 = (blockIdx.z * gridDim.y + blockIdx.y) * 4;
+    const int first = (blockIdx.x % shares) * share;
+    int i = i0 + (lane & 7), j = j0 + (lane >> 3);
+    bool take = i < p.width && j < p.height;
+    if (take) {
+        const size_t idx = (size_t)j * p.width + i;
+        if (p.rebase_pass > 0 && b.glitch_in[idx] == 0) take = false;
+        else if (hist_resolve ? p.rebase_pass == 0 : p.mode == AP_MODE_EDGE) take = b.edge_mask[idx] != 0;
     }
+    const unsigned sel = __ballot_sync(full, take);
+    const int count = min(share, __popc(sel) - first);  // pixels, owned by lanes 0, 1, ...
+    if (count <= 0) return;
+    const int place = __popc(sel & ((1u << lane) - 1u)) - first;
+    if (take && place >= 0 && place < count) list[place] = (uint8_t)lane;
+    const bool hist_colour = hist_resolve || (p.flags & AP_FLAG_HIST_COLOUR);
+    if (lane == 0) palette = palette_of(p, hist_colour);
     __syncwarp();
     const bool write_iter = hist_resolve ? (p.rebase_pass > 0) : ((p.flags & AP_FLAG_ITER_LAST_SUB) != 0);
     const int f = p.factor, f2 = f * f;
-    auto place = [&](int q, int& i, int& j) {
-        const int c = list[warp][q];
-        i = i0 + 8 * (c >> 5) + (c & 7);
-        j = j0 + ((c & 31) >> 3);
-    };
-    for (int first = 0; first < n; first += 32) {  // up to 32 pixels, owned by lanes 0, 1, ...
-        const int count = min(32, n - first);
-        double ra = 0.0, ga = 0.0, ba = 0.0;
-        int glitches = 0, iters = 0, leaps = 0, iters2 = 0;
-        const int lo = lane * f2, hi = lo + f2;  // the owned pixel's samples
-        for (int base = 0; base < count * f2; base += 32) {
-            const int q = base + lane;
-            if (q < count * f2) {
-                int i, j;
-                place(first + q / f2, i, j);
-                const int sub = q % f2;
-                const SampleOut o = sample_at<TIER, ARITH, KIND>(p, b, (double)(i * f + sub % f),
-                                                                  (double)(j * f + sub / f));
-                double r = 0.0, g = 0.0, bb = 0.0;
-                if ((double)o.s >= 0.0) colour_of(p, palette, b.lut, b.cdf, hist_colour, (double)o.s, r, g, bb);
-                red[warp][lane] = r;
-                green[warp][lane] = g;
-                blue[warp][lane] = bb;
-                work[warp][lane][0] = o.iters;
-                work[warp][lane][1] = o.leaps;
-                work[warp][lane][2] = o.iters2;
-                work[warp][lane][3] = o.glitch;
-                if (write_iter && sub == f2 - 1) {
-                    const size_t idx = (size_t)j * p.width + i;
-                    b.iter_map[idx] = o.s;
-                    if (b.kmap) b.kmap[idx] = o.k;
-                    if (b.s64) b.s64[idx] = o.s64;
-                }
+    double ra = 0.0, ga = 0.0, ba = 0.0;
+    int glitches = 0, iters = 0, leaps = 0, iters2 = 0;
+    const int lo = lane * f2, hi = lo + f2;  // the owned pixel's samples
+    for (int base = 0; base < count * f2; base += 32) {
+        const int q = base + lane;
+        if (q < count * f2) {
+            const int at = list[q / f2];
+            i = i0 + (at & 7);
+            j = j0 + (at >> 3);
+            const int sub = q % f2;
+            const SampleOut o = sample_at<TIER, ARITH, KIND>(p, b, (double)(i * f + sub % f), (double)(j * f + sub / f));
+            double r = 0.0, g = 0.0, bb = 0.0;
+            if ((double)o.s >= 0.0) colour_of(p, palette, b.lut, b.cdf, hist_colour, (double)o.s, r, g, bb);
+            red[lane] = r;
+            green[lane] = g;
+            blue[lane] = bb;
+            work[lane][0] = o.iters;
+            work[lane][1] = o.leaps;
+            work[lane][2] = o.iters2;
+            work[lane][3] = o.glitch;
+            if (write_iter && sub == f2 - 1) {
+                const size_t idx = (size_t)j * p.width + i;
+                b.iter_map[idx] = o.s;
+                if (b.kmap) b.kmap[idx] = o.k;
+                if (b.s64) b.s64[idx] = o.s64;
             }
-            __syncwarp();
-            if (lane < count) {
-                for (int t = max(lo, base); t < min(hi, base + 32); ++t) {
-                    ra += red[warp][t - base];
-                    ga += green[warp][t - base];
-                    ba += blue[warp][t - base];
-                    iters += work[warp][t - base][0];
-                    leaps += work[warp][t - base][1];
-                    iters2 += work[warp][t - base][2];
-                    glitches += work[warp][t - base][3] > 0 ? 1 : 0;
-                }
-            }
-            __syncwarp();
         }
+        __syncwarp();
         if (lane < count) {
-            int i, j;
-            place(first + lane, i, j);
-            const size_t idx = (size_t)j * p.width + i;
-            const double inv = 1.0 / (double)f2;
-            store_rgb(b.rgb, p.is_hdr, idx, ra * inv, ga * inv, ba * inv);
-            if (kPert && b.glitch_out) b.glitch_out[idx] = glitches > 0 ? 1 : 0;
-            if (b.counters) reinterpret_cast<int4*>(b.counters)[idx] = make_int4(iters, leaps, iters2, 0);
+            for (int t = max(lo, base); t < min(hi, base + 32); ++t) {
+                ra += red[t - base];
+                ga += green[t - base];
+                ba += blue[t - base];
+                iters += work[t - base][0];
+                leaps += work[t - base][1];
+                iters2 += work[t - base][2];
+                glitches += work[t - base][3] > 0 ? 1 : 0;
+            }
         }
+        __syncwarp();
     }
+    if (lane < count) {
+        i = i0 + (list[lane] & 7);
+        j = j0 + (list[lane] >> 3);
+        const size_t idx = (size_t)j * p.width + i;
+        const double inv = 1.0 / (double)f2;
+        store_rgb(b.rgb, p.is_hdr, idx, ra * inv, ga * inv, ba * inv);
+        if (kPert && b.glitch_out) b.glitch_out[idx] = glitches > 0 ? 1 : 0;
+        if (b.counters) reinterpret_cast<int4*>(b.counters)[idx] = make_int4(iters, leaps, iters2, 0);
+    }
+}
+
+// The pixels a warp takes of its patch: the fewest (from four on, so that a patch is eight blocks at
+// most) whose f x f samples leave no more than a sixteenth of the lanes idle in the last round; the
+// whole patch for one sample a pixel, and where the marks that choose pixels are the map that the
+// pass writes its glitches to, which its other warps may still have to read.
+static int patch_share(const ApFrameParams& p, const ApFrameBuffers& b) {
+    if (p.factor == 1 || (b.glitch_out && (b.glitch_out == b.glitch_in || b.glitch_out == b.edge_mask))) return 32;
+    const long long f2 = (long long)p.factor * p.factor;
+    int share = 4;
+    while (share < 32 && 16 * share * f2 < 15 * ((share * f2 + 31) / 32 * 32)) ++share;
+    return share;
 }
 
 template <int TIER, int ARITH, int KIND>
@@ -188,9 +188,10 @@ static int launch_pass(const ApFrameParams& p, const ApFrameBuffers& b, int hist
         render_pass_kernel<TIER, ARITH, KIND><<<grid, kTile * kTile, 0, st>>>(p, b);
         return check_launch("render_pass_kernel");
     }
-    constexpr int kRows = 4 * kSuperWarps;
-    dim3 grid((p.width + 8 * kPatches - 1) / (8 * kPatches), (p.height + kRows - 1) / kRows);
-    supersample_kernel<TIER, ARITH, KIND><<<grid, 32 * kSuperWarps, 0, st>>>(p, b, hist_resolve);
+    const int share = patch_share(p, b), shares = (32 + share - 1) / share;
+    const int rows = (p.height + 3) / 4, fold = min(rows, 32768);  // a grid's y ends at 65535
+    dim3 grid((p.width + 7) / 8 * shares, fold, (rows + fold - 1) / fold);
+    supersample_kernel<TIER, ARITH, KIND><<<grid, 32, 0, st>>>(p, b, hist_resolve, share, shares);
     return check_launch("supersample_kernel");
 }
 

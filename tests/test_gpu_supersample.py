@@ -42,3 +42,36 @@ def test_perturbation_frames(factor, glitch, width):
     fr, _ = oracle_pert_frame(m)
     assert np.array_equal(it.view(np.uint32), fr.iter_map.view(np.uint32))
     assert np.array_equal(rgb, fr.rgb)
+
+
+@pytest.mark.parametrize("factor", [2, 3])
+def test_glitch_map_in_place(factor):
+    """A rebase pass that writes its glitches into the map that chose its pixels equals one with two maps."""
+    import ctypes as C
+
+    import torch
+    from fractura_b200 import _lib
+    from fractura_b200.palette import synthetic_lut
+    from helpers import load_golden
+    from test_oracle_fexp import floatexp_params
+    G, META = load_golden("fexp_samples.npz")
+    m = next(x for x in META if x["name"] == "fexp_mandel")
+    _, p = floatexp_params(m, "plain", abi.AP_ARITH_REF_CUDA)
+    W, H = 61, 22
+    p.width, p.height, p.factor, p.mode, p.rebase_pass = W, H, factor, abi.AP_MODE_FULL, 1
+    dev = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()
+    re, im, lut = dev(G["fexp_mandel__re"]), dev(G["fexp_mandel__im"]), dev(synthetic_lut())
+    marks = (np.random.default_rng(factor).random((H, W)) < 0.8).astype(np.uint8)
+    got = []
+    for same in (False, True):
+        gin, it = dev(marks), torch.zeros((H, W), dtype=torch.float32, device="cuda")
+        gout = gin if same else dev(marks)
+        rgb = torch.zeros((H, W, 3), dtype=torch.uint8, device="cuda")
+        b = abi.ApFrameBuffers()
+        ptr = lambda x: C.c_void_p(x.data_ptr())
+        b.ref_re, b.ref_im, b.lut, b.iter_map, b.rgb = ptr(re), ptr(im), ptr(lut), ptr(it), ptr(rgb)
+        b.glitch_in, b.glitch_out = ptr(gin), ptr(gout)
+        _lib.check(_lib.load().ap_render_pass(C.byref(p), C.byref(b), None), "ap_render_pass")
+        got.append((rgb.cpu().numpy(), gout.cpu().numpy()))
+    assert np.array_equal(got[0][0], got[1][0]) and np.array_equal(got[0][1], got[1][1])
+    assert got[0][0].any()
