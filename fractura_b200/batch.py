@@ -5,8 +5,8 @@ workers/image_workers.py:428-601, calls render_frame_ssaa per tile).  Here a
 batch of tiles of any size, formula and max_iter is prepared on the host
 (reference orbit, device BLA table, packed inputs, one descriptor per tile) and
 rendered by a single persistent kernel whose blocks take consecutive pixels from
-a shared counter, run them a quantum of loop steps at a time and compact the
-unfinished ones between quanta.  Each tile's values equal the per-frame coarse
+a shared counter, run them in rounds of equal time and compact the unfinished ones
+between rounds.  Each tile's values equal the per-frame coarse
 pass (ap_render_pass) for the same parameters.  arith="fast" gives one-pass tiles
 the fused step (the batch's single-reference tiles run "ref_cuda"); a tile with
 delta_form="fp32" runs the FP32-mantissa FloatExp form (AP_TIER_FLOATEXP32), as the
@@ -61,8 +61,8 @@ class Tile:
 class BatchConfig:
     """Launch shape of the persistent kernel: patch_w x patch_h = 256 pixels per work
     item, blocks_per_sm resident blocks of 512 threads, min_blocks = the register
-    budget (4: 64 registers, 6: 42), quantum = loop steps per pixel between two
-    compactions of a block's pixels."""
+    budget (4: 64 registers, 6: 42), quantum = length of a round, the time between two
+    compactions of a block's pixels (in units that grow with the pixels per thread)."""
     patch_w: int = 16
     patch_h: int = 16
     blocks_per_sm: int = 2

@@ -10,8 +10,8 @@
 // first).  The grid holds blocks_per_sm blocks per SM for the whole batch; the
 // queue is one global pixel counter.
 //
-// A block works in rounds.  In a round each thread runs one pixel for `quantum`
-// loop steps, resumable (the per-frame kernel's pixel_begin / pixel_advance /
+// A block works in rounds of equal time.  In a round each thread runs one pixel,
+// resumable (the per-frame kernel's pixel_begin / pixel_advance /
 // rebase_advance / pixel_finish, and fe32_begin / fe32_advance / fe32_finish for FP32
 // tiles, so values are identical).  A pixel that finishes is
 // written out; one that does not leaves its state in the block's shared slots.  At
@@ -125,14 +125,14 @@ __device__ __forceinline__ void slot_store_run(BatchSlots& S, int q, const Pixel
 // rebasing): separate functions, so each keeps the register allocation it has in the
 // per-frame kernel.
 template <int ARITH, int FT, bool BLA, bool REBASE>
-__device__ __noinline__ bool slot_run(const ApTileDesc* __restrict__ t, BatchSlots& S, int q, int quantum) {
+__device__ __noinline__ bool slot_run(const ApTileDesc* __restrict__ t, BatchSlots& S, int q, Round round) {
     const ApFrameBuffers b = tile_buffers(t);
     PixelRun s;
     slot_load_run(S, q, s, REBASE);
     if (REBASE)
-        rebase_advance<ARITH, FT, BLA, true>(t->p, b, s, quantum, S.cycles, q);
+        rebase_advance<ARITH, FT, BLA, true>(t->p, b, s, round, S.cycles, q);
     else
-        pixel_advance<ARITH, FT, BLA, true>(t->p, b, s, quantum, S.cycles, q);
+        pixel_advance<ARITH, FT, BLA, true>(t->p, b, s, round, S.cycles, q);
     if (s.stage == 3) {
         s.idx = S.idx[q];
         s.k0 = S.k0[q];
@@ -202,11 +202,11 @@ __device__ __forceinline__ void fe32_slot_store_run(BatchSlots& S, int q, const 
 
 // One round of an FP32 pixel (as slot_run).
 template <int FT, bool BLA, bool REBASE>
-__device__ __noinline__ bool fe32_slot_run(const ApTileDesc* __restrict__ t, BatchSlots& S, int q, int quantum) {
+__device__ __noinline__ bool fe32_slot_run(const ApTileDesc* __restrict__ t, BatchSlots& S, int q, Round round) {
     const ApFrameBuffers b = tile_buffers(t);
     Fe32Run s;
     fe32_slot_load(S, q, s, REBASE);
-    fe32_advance<FT, BLA, REBASE, true>(t->p, b, s, quantum);
+    fe32_advance<FT, BLA, REBASE, true>(t->p, b, s, round);
     if (s.stage == 3) {
         s.idx = S.idx[q];
         fe32_finish(t->p, b, s);
@@ -217,56 +217,56 @@ __device__ __noinline__ bool fe32_slot_run(const ApTileDesc* __restrict__ t, Bat
 }
 
 // FP32 formula dispatch (Burning Ship types take no leaps, as in the per-frame pass).
-__device__ __forceinline__ bool fe32_batch_run(const ApTileDesc* t, BatchSlots& S, int q, int quantum) {
+__device__ __forceinline__ bool fe32_batch_run(const ApTileDesc* t, BatchSlots& S, int q, Round round) {
     const bool bla = t->p.bla_levels > 1 && t->bla_packed != nullptr;
     const bool rebase = (t->p.flags & AP_FLAG_REBASE) != 0;
     switch (t->p.fractal_type) {
     case 1:
     case 3:
-        return rebase ? fe32_slot_run<kFtShip, false, true>(t, S, q, quantum)
-                      : fe32_slot_run<kFtShip, false, false>(t, S, q, quantum);
+        return rebase ? fe32_slot_run<kFtShip, false, true>(t, S, q, round)
+                      : fe32_slot_run<kFtShip, false, false>(t, S, q, round);
     case 4:
         if (rebase)
-            return bla ? fe32_slot_run<kFtMulti, true, true>(t, S, q, quantum)
-                       : fe32_slot_run<kFtMulti, false, true>(t, S, q, quantum);
-        return bla ? fe32_slot_run<kFtMulti, true, false>(t, S, q, quantum)
-                   : fe32_slot_run<kFtMulti, false, false>(t, S, q, quantum);
+            return bla ? fe32_slot_run<kFtMulti, true, true>(t, S, q, round)
+                       : fe32_slot_run<kFtMulti, false, true>(t, S, q, round);
+        return bla ? fe32_slot_run<kFtMulti, true, false>(t, S, q, round)
+                   : fe32_slot_run<kFtMulti, false, false>(t, S, q, round);
     default:
         if (rebase)
-            return bla ? fe32_slot_run<kFtQuad, true, true>(t, S, q, quantum)
-                       : fe32_slot_run<kFtQuad, false, true>(t, S, q, quantum);
-        return bla ? fe32_slot_run<kFtQuad, true, false>(t, S, q, quantum)
-                   : fe32_slot_run<kFtQuad, false, false>(t, S, q, quantum);
+            return bla ? fe32_slot_run<kFtQuad, true, true>(t, S, q, round)
+                       : fe32_slot_run<kFtQuad, false, true>(t, S, q, round);
+        return bla ? fe32_slot_run<kFtQuad, true, false>(t, S, q, round)
+                   : fe32_slot_run<kFtQuad, false, false>(t, S, q, round);
     }
 }
 
 // Formula dispatch.  AP_ARITH_FAST serves one-pass tiles only; a FAST batch's
 // single-reference tiles (Julia types) run the CUDA-source profile.
 template <int ARITH>
-__device__ __forceinline__ bool batch_run(const ApTileDesc* t, BatchSlots& S, int q, int quantum) {
+__device__ __forceinline__ bool batch_run(const ApTileDesc* t, BatchSlots& S, int q, Round round) {
     constexpr int kPlain = (ARITH == AP_ARITH_FAST) ? AP_ARITH_REF_CUDA : ARITH;
-    if (t->p.tier == AP_TIER_FLOATEXP32) return fe32_batch_run(t, S, q, quantum);
+    if (t->p.tier == AP_TIER_FLOATEXP32) return fe32_batch_run(t, S, q, round);
     const bool bla = t->p.bla_levels > 1 && t->bla_packed != nullptr;
     if (t->p.flags & AP_FLAG_REBASE) {
         switch (t->p.fractal_type) {
-        case 1: return slot_run<ARITH, kFtShip, false, true>(t, S, q, quantum);
+        case 1: return slot_run<ARITH, kFtShip, false, true>(t, S, q, round);
         case 4:
-            return bla ? slot_run<ARITH, kFtMulti, true, true>(t, S, q, quantum)
-                       : slot_run<ARITH, kFtMulti, false, true>(t, S, q, quantum);
+            return bla ? slot_run<ARITH, kFtMulti, true, true>(t, S, q, round)
+                       : slot_run<ARITH, kFtMulti, false, true>(t, S, q, round);
         default:
-            return bla ? slot_run<ARITH, kFtQuad, true, true>(t, S, q, quantum)
-                       : slot_run<ARITH, kFtQuad, false, true>(t, S, q, quantum);
+            return bla ? slot_run<ARITH, kFtQuad, true, true>(t, S, q, round)
+                       : slot_run<ARITH, kFtQuad, false, true>(t, S, q, round);
         }
     }
     switch (t->p.fractal_type) {
     case 1:
-    case 3: return slot_run<kPlain, kFtShip, false, false>(t, S, q, quantum);
+    case 3: return slot_run<kPlain, kFtShip, false, false>(t, S, q, round);
     case 4:
-        return bla ? slot_run<kPlain, kFtMulti, true, false>(t, S, q, quantum)
-                   : slot_run<kPlain, kFtMulti, false, false>(t, S, q, quantum);
+        return bla ? slot_run<kPlain, kFtMulti, true, false>(t, S, q, round)
+                   : slot_run<kPlain, kFtMulti, false, false>(t, S, q, round);
     default:
-        return bla ? slot_run<kPlain, kFtQuad, true, false>(t, S, q, quantum)
-                   : slot_run<kPlain, kFtQuad, false, false>(t, S, q, quantum);
+        return bla ? slot_run<kPlain, kFtQuad, true, false>(t, S, q, round)
+                   : slot_run<kPlain, kFtQuad, false, false>(t, S, q, round);
     }
 }
 
@@ -331,14 +331,14 @@ __device__ __forceinline__ int batch_class(const ApTileDesc* t) {
 }
 constexpr int kBatchClasses = 6;
 
-// Loop steps of a round for tile t: `quantum` of the dearest step (Multibrot n = 5, 58 FP64
-// operations), more of a cheaper one, so that the warps of a block, which wait for one
-// another at the end of a round, take about as long whatever they run (21 mixed tiles 42.6 ->
-// 35.5 ms; blocks of 64, 128 and 256 threads 46, 41 and 36 ms).
-__device__ __forceinline__ int batch_quantum(const ApTileDesc* t, int quantum) {
-    const int ft = t->p.fractal_type;
-    const int cost = ft == 4 ? max(12, min(58, 12 * t->p.gen_n - 2)) : (ft & 1) ? 16 : 12;
-    return quantum * 58 / cost;
+// Clock cycles of a round per unit of its length (`quantum`).  A short round gives the lanes of
+// finished pixels new ones soon, a long one spends less on waiting and compacting: 512 where the
+// batch has no more than two pixels a slot, 4096 where it has sixteen (21 mixed tiles, 20 a slot:
+// 512 32.6 ms, 1024 31.5, 2048 30.2, 4096 29.2, 8192 29.6, 16384 34.6; single tiles of one or two
+// pixels a slot lose 9 to 23 % from 512 to 4096).
+__device__ __forceinline__ unsigned round_cycles(long long pixels) {
+    const long long c = 256 * (pixels / ((long long)gridDim.x * kBatchThreads));
+    return (unsigned)max(512ll, min(4096ll, c));
 }
 
 template <int ARITH, int MINB>
@@ -354,12 +354,15 @@ __global__ void __launch_bounds__(kBatchThreads, MINB * 256 / kBatchThreads) bat
     const unsigned full = 0xffffffffu;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const long long total = first[n] * 256;
+    // half the clock's range at most, so that its wrap-around is told apart
+    const unsigned span = (unsigned)min((long long)quantum * round_cycles(total), 1ll << 30);
     if (tid == 0) {
         live_s = 0;
         drained_s = 0;
     }
     __syncthreads();
     for (;;) {
+        const unsigned end = (unsigned)clock() + span;  // of this round
         // the slots past the live pixels take the next pixels of the queue
         const int live = live_s;
         const bool take = !drained_s && live < kBatchThreads;
@@ -384,7 +387,7 @@ __global__ void __launch_bounds__(kBatchThreads, MINB * 256 / kBatchThreads) bat
             if (u < total && batch_pixel_at(tiles, first, n, patch_w, patch_h, u, &tile, &i, &j))
                 running = slot_begin<ARITH>(tiles + tile, tile, S, tid, i, j);
         }
-        if (running) running = batch_run<ARITH>(tiles + tile, S, tid, batch_quantum(tiles + tile, quantum));
+        if (running) running = batch_run<ARITH>(tiles + tile, S, tid, Round{min(quantum, kRoundCheck), end});
         // compact the unfinished pixels into the first slots, by variant and in order within
         // one: a warp whose lanes run different variants runs them one after the other
         const int cls = running ? batch_class(tiles + tile) : -1;

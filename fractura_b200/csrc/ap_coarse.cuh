@@ -123,10 +123,26 @@ __device__ __forceinline__ int tail_gap(const CycleStore<N>& C, int q, OrbitTail
     return d == 0 ? 0 : (d < 0 ? -d : tail.p - d);
 }
 
+// A round of the batch kernel: it lasts until the SM's clock passes `end`, looked at every kRoundCheck
+// loop iterations (`left`, the same for all lanes of a loop), and for the first iterations in any
+// case.  Rounds counted in steps, weighted by formula, lasted as long as their block's dearest warp:
+// 44 % of the warps' time went into waiting for it (21 mixed tiles 33.3 -> 29.2 ms with the clock;
+// looking every 8, 16 or 32 iterations times alike).
+constexpr int kRoundCheck = 16;
+struct Round {
+    int left;
+    unsigned end;
+    __device__ __forceinline__ bool over() {
+        if (--left >= 0) return false;
+        left = kRoundCheck - 1;
+        return (int)((unsigned)clock() - end) >= 0;
+    }
+};
+
 // One pixel of a coarse pass, resumable: pixel_begin sets it up, pixel_advance runs
-// its stage-1 (perturbation) and stage-2 (direct) loops -- all of them, or at most
-// `budget` loop iterations (steps or leaps) per call when BUDGET is set, so that a
-// persistent kernel can hand a lane whose pixel finished a new one -- and
+// its stage-1 (perturbation) and stage-2 (direct) loops -- all of them, or until `round` is
+// over when BUDGET is set, so that a persistent kernel can hand a lane whose pixel finished
+// a new one -- and
 // pixel_finish writes its outputs.  coarse_pixel runs the three in a row; the
 // per-frame kernel below and the batch kernel (ap_batch.cu) share this code, so both
 // give identical values.
@@ -326,7 +342,7 @@ __device__ __forceinline__ void value_barrier(int& v) { asm volatile("" : "+r"(v
 
 template <int ARITH, int FT, bool BLA, bool BUDGET, int N>
 __device__ __forceinline__ void pixel_advance(const ApFrameParams& p, const ApFrameBuffers& b, PixelRun& s,
-                                              int budget, CycleStore<N>& C, int q) {
+                                              Round round, CycleStore<N>& C, int q) {
     constexpr bool kCpu = (ARITH == AP_ARITH_REF_CPU);
     constexpr bool kMerge = (FT == kFtMulti);
     const bool julia = (p.fractal_type == 2 || p.fractal_type == 3);
@@ -369,7 +385,7 @@ __device__ __forceinline__ void pixel_advance(const ApFrameParams& p, const ApFr
                 }
                 bound = gap < ref_len - k ? k + gap : ref_len;
             }
-            if (BUDGET && --budget < 0) {
+            if (BUDGET && round.over()) {
                 paused = true;
                 break;
             }
@@ -380,7 +396,6 @@ __device__ __forceinline__ void pixel_advance(const ApFrameParams& p, const ApFr
             if (FT == kFtQuad && k + kSpan <= bound && span_fits<BLA>(dz_hi, Z, dc_exp60)) {
                 span_steps<ARITH, FT>(p, orb + k, dzx, dzy, dcpx, dcpy);
                 k += kSpan;
-                if (BUDGET) budget -= kSpan - 1;
                 continue;
             }
             // One branch on the common path: inside the safe radius (no test can fire)
@@ -469,7 +484,7 @@ __device__ __forceinline__ void pixel_advance(const ApFrameParams& p, const ApFr
         const bool doubles = fp64_doubles(zy, cy);
         int tested = 0;  // steps to test one by one before the next block
         while (k < max_iter) {
-            if (BUDGET && --budget < 0) {
+            if (BUDGET && round.over()) {
                 paused = true;
                 break;
             }
@@ -484,7 +499,6 @@ __device__ __forceinline__ void pixel_advance(const ApFrameParams& p, const ApFr
                 });
                 if (zx * zx + zy * zy <= kBailout) {
                     k += kBlock;
-                    if (BUDGET) budget -= kBlock - 1;
                     if (cycle_visit(C, q, zx, zy, k, -1) > 0) {  // it repeats: never escapes
                         s.k2 += max_iter - k;
                         skipped += max_iter - k;
@@ -556,7 +570,7 @@ __device__ __forceinline__ void pixel_advance(const ApFrameParams& p, const ApFr
 // power costs 14 instead of 22), leaps as the CUDA profile.
 template <int ARITH, int FT, bool BLA, bool BUDGET, int N>
 __device__ __forceinline__ void rebase_advance(const ApFrameParams& p, const ApFrameBuffers& b, PixelRun& s,
-                                               int budget, CycleStore<N>& C, int q) {
+                                               Round round, CycleStore<N>& C, int q) {
     constexpr bool kCpu = (ARITH == AP_ARITH_REF_CPU);
     constexpr bool kFast = (ARITH == AP_ARITH_FAST);
     constexpr bool kMerge = (FT == kFtMulti);
@@ -607,7 +621,7 @@ __device__ __forceinline__ void rebase_advance(const ApFrameParams& p, const ApF
             bound = gap < lim - m ? m + gap : lim;
             if (m >= lim) break;
         }
-        if (BUDGET && --budget < 0) {
+        if (BUDGET && round.over()) {
             paused = true;
             break;
         }
@@ -618,7 +632,6 @@ __device__ __forceinline__ void rebase_advance(const ApFrameParams& p, const ApF
         if (FT == kFtQuad && m + kSpan <= bound && span_fits<BLA>(dz_hi, Z, dc_exp60)) {
             span_steps<ARITH, FT>(p, orb + m, dzx, dzy, dcpx, dcpy);
             m += kSpan;
-            if (BUDGET) budget -= kSpan - 1;
             continue;
         }
         // ap_pack_orbit leaves the orbit's last record (m == ref_len) with safe radius 0,
@@ -723,9 +736,9 @@ __device__ __forceinline__ void coarse_pixel(const ApFrameParams& p, const ApFra
     if (!pixel_begin<ARITH, FT>(p, b, i, j, s)) return;
     C.visits[q] = 0;
     if (REBASE)
-        rebase_advance<ARITH, FT, BLA, false>(p, b, s, 0, C, q);
+        rebase_advance<ARITH, FT, BLA, false>(p, b, s, Round{}, C, q);
     else
-        pixel_advance<ARITH, FT, BLA, false>(p, b, s, 0, C, q);
+        pixel_advance<ARITH, FT, BLA, false>(p, b, s, Round{}, C, q);
     pixel_finish(p, b, s);
 }
 

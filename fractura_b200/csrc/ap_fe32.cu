@@ -57,7 +57,7 @@ __global__ void __launch_bounds__(64, 16) fe32_coarse_kernel(const ApFrameParams
     if (i >= p.width || j >= p.height) return;
     Fe32Run s;
     if (!fe32_begin(p, b, i, j, s)) return;
-    fe32_advance<FT, BLA, REBASE, false>(p, b, s, 0);
+    fe32_advance<FT, BLA, REBASE, false>(p, b, s, Round{});
     fe32_finish(p, b, s);
 }
 

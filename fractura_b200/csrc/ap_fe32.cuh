@@ -210,10 +210,10 @@ __device__ __forceinline__ void fe32_direct_step(const ApFrameParams& p, double&
 }
 
 // One pixel of an FP32 coarse pass, resumable like the FP64 passes' PixelRun:
-// fe32_begin sets it up, fe32_advance runs its loops -- all of them, or at most
-// `budget` loop iterations (steps or leaps) per call when BUDGET is set -- and
-// fe32_finish writes its outputs.  The per-frame kernel (ap_fe32.cu) runs the three
-// in a row; the batch kernel (ap_batch.cu) runs fe32_advance a quantum at a time.
+// fe32_begin sets it up, fe32_advance runs its loops -- all of them, or until `round` is
+// over when BUDGET is set -- and fe32_finish writes its outputs.  The per-frame kernel
+// (ap_fe32.cu) runs the three in a row; the batch kernel (ap_batch.cu) runs fe32_advance
+// a round at a time.
 // Between calls the delta is kept as (wx, wy, e) exactly as the loop holds it (no
 // renormalisation at a call boundary), so both give identical values.
 struct Fe32Run {
@@ -265,7 +265,7 @@ __device__ __forceinline__ bool fe32_begin(const ApFrameParams& p, const ApFrame
 
 template <int FT, bool BLA, bool REBASE, bool BUDGET>
 __device__ __forceinline__ void fe32_advance(const ApFrameParams& p, const ApFrameBuffers& b, Fe32Run& s,
-                                             int budget) {
+                                             Round round) {
     constexpr int bias = kRadiusBias;
     const int ref_len = p.ref_len, max_iter = p.max_iter;
     const double4* __restrict__ orb = reinterpret_cast<const double4*>(b.orbit_packed);
@@ -310,7 +310,7 @@ __device__ __forceinline__ void fe32_advance(const ApFrameParams& p, const ApFra
     const double inv_ln = inv_ln_for(p.fractal_type, p.gen_n);
 
     while (s.stage == 1 && (REBASE ? (k < lim) : (k < ref_len))) {
-        if (BUDGET && --budget < 0) {
+        if (BUDGET && round.over()) {
             paused = true;
             break;
         }
@@ -478,7 +478,7 @@ __device__ __forceinline__ void fe32_advance(const ApFrameParams& p, const ApFra
     }
     const bool nan_guard = (p.flags & AP_FLAG_NAN_GUARD) != 0;
     while (k < max_iter) {
-        if (BUDGET && --budget < 0) {
+        if (BUDGET && round.over()) {
             paused = true;
             break;
         }

@@ -412,8 +412,9 @@ AP_API int ap_decimal_arith(int32_t op, const int64_t* a_meta, const uint64_t* a
  * tiles should come in decreasing order of expected cost.
  * ap_render_batch: renders all tiles with one persistent kernel of blocks_per_sm blocks per
  * SM that take pixels from a shared counter (device word *queue_head, reset here).  A block
- * works in rounds: each thread runs one pixel for `quantum` loop steps; the unfinished
- * pixels are compacted into the block's first slots (shared memory) and the slots left
+ * works in rounds of a length that `quantum` scales (at least that many loop steps, up to 16, and
+ * quantum x 512 to 4096 clock cycles, more with more pixels a thread): each thread runs one pixel;
+ * the unfinished pixels are compacted into the block's first slots (shared memory) and the slots left
  * over take the next consecutive pixels of the queue with one atomicAdd.
  * tiles and first_patch are device copies of the planned arrays.  min_blocks (4 or 6) picks
  * the register budget the kernel is compiled for; arith is the tiles' common profile
