@@ -117,10 +117,9 @@ __global__ void __launch_bounds__(kHistThreads) histogram_shared_kernel(const fl
     }
 }
 
-// From this many pixels on, the kernels of fewer, longer threads win.  Histogram: 3840x2160 64 us with
-// histogram_kernel, 25 with histogram_shared_kernel (a flat map 174 and 17); 1920x1080 24.6 and 15.5;
-// 640x360 11.2 with the first and more with the second, whose 128 KiB of counters are cleared and
-// walked.  Colour: 3840x2160 69 us with a pixel a thread, 50 with four; 640x360 5.4 and 7.5.
+// From this many pixels on, the shared-memory histogram wins: 3840x2160 64 us with histogram_kernel,
+// 25 with histogram_shared_kernel (a flat map 174 and 17); 1920x1080 24.6 and 15.5; 640x360 11.2 with
+// the first and more with the second, whose 128 KiB of counters are cleared and walked.
 constexpr size_t kLargeMap = (size_t)1 << 19;
 
 // Adds the map's counts to hist.
@@ -371,9 +370,16 @@ static int launch_cdf(const int32_t* hist, int num_bins, float* cdf, cudaStream_
 // Any alignment, and the masked form of rebase passes: a pixel a thread.
 __global__ void __launch_bounds__(256) colour_kernel(const ApFrameParams p, const ApFrameBuffers b,
                                                      int hist) {
-    __shared__ Palette palette;
-    if (threadIdx.x == 0) palette = palette_of(p, hist != 0);
-    __syncthreads();
+    // schemes 2 and 3 take a tanh or an exp and a division from the frame alone, the others products
+    __shared__ Palette shared;
+    Palette palette;
+    if (!hist && (p.scheme_id == 2 || p.scheme_id == 3)) {
+        if (threadIdx.x == 0) shared = palette_of(p, false);
+        __syncthreads();
+        palette = shared;
+    } else {
+        palette = palette_of(p, hist != 0);
+    }
     const int i = blockIdx.x * 16 + (threadIdx.x & 15);
     const int j = blockIdx.y * 16 + (threadIdx.x >> 4);
     if (i >= p.width || j >= p.height) return;
@@ -381,7 +387,11 @@ __global__ void __launch_bounds__(256) colour_kernel(const ApFrameParams p, cons
     if (p.rebase_pass > 0 && b.glitch_in != nullptr && b.glitch_in[idx] == 0) return;
     const double s = (double)b.iter_map[idx];
     double r = 0.0, g = 0.0, bb = 0.0;
-    if (s >= 0.0) colour_of(p, palette, b.lut, b.cdf, hist != 0, s, r, g, bb);
+    if (s >= 0.0) {
+        const double norm = hist ? cdf_norm(palette, s, b.cdf, p.num_bins, p.color_contrast)
+                                 : palette_norm(palette, s, p.scheme_id, p.arith == AP_ARITH_REF_CPU);
+        lut_lerp(b.lut, norm, r, g, bb);
+    }
     store_rgb(b.rgb, p.is_hdr, idx, r, g, bb);
 }
 
@@ -434,11 +444,15 @@ static void launch_colour4(const ApFrameParams& p, const ApFrameBuffers& b, size
     else colour4_kernel<SCHEME, false><<<grid, 256, 0, st>>>(p, b, n4);
 }
 
+// From this many pixels on, four pixels a thread win: 3840x2160 with the histogram scheme 69 us with a
+// pixel a thread, 50 with four; 1920x1080 23.4 and 15.3; 1024x600 10.6 and 12.2.
+constexpr size_t kLargeFrame = (size_t)1 << 20;
+
 // A large frame whose pixels come in fours, with aligned maps and no mask, takes colour4_kernel.
 static int launch_colour(const ApFrameParams& p, const ApFrameBuffers& b, int hist, cudaStream_t st) {
     const size_t n = (size_t)p.width * p.height;
     const bool masked = p.rebase_pass > 0 && b.glitch_in != nullptr;
-    if (n >= kLargeMap && !masked && (n & 3) == 0 && (reinterpret_cast<uintptr_t>(b.iter_map) & 15u) == 0 &&
+    if (n >= kLargeFrame && !masked && (n & 3) == 0 && (reinterpret_cast<uintptr_t>(b.iter_map) & 15u) == 0 &&
         (reinterpret_cast<uintptr_t>(b.rgb) & 3u) == 0) {
         const size_t n4 = n / 4;
         switch (hist ? 11 : p.scheme_id) {

@@ -1,4 +1,4 @@
-"""The kernels that large maps take (from 2^19 pixels on): the histogram counted in shared memory,
+"""The kernels that large maps take (from 2^19 and 2^20 pixels on): the histogram counted in shared memory,
 against the oracle's counts, and the colouring of four pixels a thread, bit for bit against the same
 map coloured in strips below that size."""
 import ctypes as C
@@ -97,7 +97,7 @@ def test_colour_of_a_large_map_is_the_strips(scheme, hdr):
     rng = np.random.default_rng(scheme)
     lut = torch.from_numpy((rng.random((2048, 3)) * (65535 if hdr else 255)).astype(np.float32)).cuda()
     cdf = torch.from_numpy(np.sort(rng.random(65536)).astype(np.float32)).cuda() if scheme == 11 else None
-    for (H, W), offset in (((512, 1024), 0), ((727, 724), 0), ((727, 724), 1)):
+    for (H, W), offset in (((1024, 1024), 0), ((1031, 1028), 0), ((1031, 1028), 1)):
         it = a_map(H, W, 700)
         for arith in (abi.AP_ARITH_REF_CPU, abi.AP_ARITH_FAST):
             whole = coloured(it, H, scheme, hdr, arith, lut, cdf, offset)
