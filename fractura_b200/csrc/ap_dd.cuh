@@ -92,33 +92,61 @@ __device__ __forceinline__ dd add_normalised(dd a, dd b) {
 
 __device__ __forceinline__ bool dd_normalised(dd a) { return a.hi + a.lo == a.hi; }
 
-// Integer tests of a high word, off the FP64 pipe.  plain_high: 2^-200 <= |v| < 181
-// (181^2 + 181^2 < 65536); zero is not plain.  plain_low: |v| >= 2^-700, or 0.
-__device__ __forceinline__ bool plain_high(double v) {
-    constexpr unsigned lo = (1023u - 200u) << 20, hi = 0x4066a000u;  // the high words of 2^-200 and 181.0
-    return ((unsigned)__double2hiint(v) & 0x7fffffffu) - lo < hi - lo;
-}
-__device__ __forceinline__ bool plain_low(double v) {
-    const unsigned h = (unsigned)__double2hiint(v) & 0x7fffffffu;
-    return h >= (1023u - 700u) << 20 || (h | (unsigned)__double2loint(v)) == 0u;
-}
-
-// One step z <- z^2 + c (SHIP: (|Re z| + i |Im z|)^2 - i-mirrored c) of the reference's
-// operations in its order, for any operands.
-struct dd2 {
-    dd x, y;
+// Integer tests of the high words of the values that a run of steps has started from, off the FP64
+// pipe and off the steps' dependent chain: every high part 0 or 2^-200 <= |v| < 181 (181^2 + 181^2 <
+// 65536), every low part 0 or at least 2^-700.  What is below 2^-1042 counts as 0: its products can
+// differ from the general step's in the last bit of a subnormal number, 2^-1074.
+struct PlainRange {
+    unsigned top = 0u, high = ~0u, low = ~0u;
+    __device__ __forceinline__ void add(dd x, dd y) {
+        const unsigned hx = (unsigned)__double2hiint(x.hi) & 0x7fffffffu, hy = (unsigned)__double2hiint(y.hi) & 0x7fffffffu;
+        const unsigned lx = (unsigned)__double2hiint(x.lo) & 0x7fffffffu, ly = (unsigned)__double2hiint(y.lo) & 0x7fffffffu;
+        top = max(top, max(hx, hy));
+        high = min(high, min(hx - 1u, hy - 1u));  // 0 counts as the largest
+        low = min(low, min(lx - 1u, ly - 1u));
+    }
+    __device__ __forceinline__ bool plain() const {
+        constexpr unsigned k181 = 0x4066a000u, kHigh = (1023u - 200u) << 20, kLow = (1023u - 700u) << 20;
+        return (top < k181) & (high >= kHigh - 1u) & (low >= kLow - 1u);
+    }
 };
+
+// One step z <- z^2 + c (SHIP: (|Re z| + i |Im z|)^2 - i-mirrored c) of the reference's operations
+// in its order, for any operands; zx2, zy2 the squares.
 template <int ARITH, bool SHIP>
-__device__ __noinline__ dd2 dd_step_general(dd2 z, dd2 c) {
-    const dd sub = dd_sub(dd_sqr<ARITH>(z.x), dd_sqr<ARITH>(z.y));
-    const dd zxy = SHIP ? dd_mul<ARITH>(dd_abs(z.x), dd_abs(z.y)) : dd_mul<ARITH>(z.x, z.y);
+__device__ __forceinline__ void dd_step_general(dd& zx, dd& zy, dd zx2, dd zy2, dd cx, dd cy) {
+    const dd sub = dd_sub(zx2, zy2);
+    const dd zxy = SHIP ? dd_mul<ARITH>(dd_abs(zx), dd_abs(zy)) : dd_mul<ARITH>(zx, zy);
     const dd two{zxy.hi * 2.0, zxy.lo * 2.0};
-    return {dd_add(sub, c.x), SHIP ? dd_sub(two, c.y) : dd_add(two, c.y)};
+    zx = dd_add(sub, cx);
+    zy = SHIP ? dd_sub(two, cy) : dd_add(two, cy);
 }
 
-// The orbit of z under z^2 + c (SHIP: Burning Ship), bit for bit as dd_step_general gives it
-// in either profile, in 58 FP64 operations a step instead of 117 (REF_CPU, whose Dekker
-// product takes 17) or 80 (REF_CUDA):
+// The same for normalised operands in PlainRange (see dd_quad_orbit).
+template <bool SHIP>
+__device__ __forceinline__ void dd_step_plain(dd& zx, dd& zy, dd cx, dd cy) {
+    const double x2 = zx.hi + zx.hi, y2 = zy.hi + zy.hi;
+    double p = zx.hi * zx.hi;
+    const dd zx2 = quick_sum(p, fma(zx.hi, zx.hi, -p) + x2 * zx.lo);
+    p = zy.hi * zy.hi;
+    const dd zy2 = quick_sum(p, fma(zy.hi, zy.hi, -p) + y2 * zy.lo);
+    p = x2 * zy.hi;
+    dd zxy = quick_sum(p, fma(x2, zy.hi, -p) + x2 * zy.lo + zx.lo * y2);  // 2 z_x z_y
+    zx = add_normalised(add_normalised(zx2, dd{-zy2.hi, -zy2.lo}), cx);
+    if (SHIP) {
+        // 2 |z_x| |z_y|: the low part's sign turns with the high part's
+        const int flip = __double2hiint(zxy.hi) & 0x80000000;
+        zxy.hi = fabs(zxy.hi);
+        zxy.lo = __hiloint2double(__double2hiint(zxy.lo) ^ flip, __double2loint(zxy.lo));
+        zy = add_normalised(zxy, dd{-cy.hi, -cy.lo});
+    } else {
+        zy = add_normalised(zxy, cy);
+    }
+}
+
+// The orbit of z under z^2 + c (SHIP: Burning Ship), bit for bit (but for the signs of zeros, which
+// no magnitude depends on) as dd_step_general gives it in either profile, in 58 FP64 operations a
+// step instead of 117 (REF_CPU, whose Dekker product takes 17) or 80 (REF_CUDA):
 //   * Dekker's product error is exact, as fma(a, b, -ab) is, wherever no partial product
 //     underflows, so both profiles take the two-operation product;
 //   * every second sum of a normalised operation has its operands in order of magnitude
@@ -126,44 +154,46 @@ __device__ __noinline__ dd2 dd_step_general(dd2 z, dd2 c) {
 //   * 2 z_x and 2 z_y are formed once for the squares' cross terms and for 2 z_x z_y
 //     (scaling by 2 commutes with every rounding that does not underflow);
 //   * while both high parts are below 181 the orbit cannot have passed the bailout, so |z|^2
-//     is formed only by the general step, which every other z takes: one near the bailout,
-//     and one with a high part below 2^-200 (zero included: the first step) or a low part
-//     below 2^-700, where a product could underflow.
-// Bound by the FP64 pipe (84 % of its issue slots; 59.5 FP64 instructions a step and warp).
-// Measured: 1280x720 Burning Ship at 2e-17, max_iter 20000, 2x SSAA, REF_CPU 102.0 -> 56.6 ms;
-// 960x540 Mandelbrot at 1e-18, REF_CUDA 20.4 -> 16.6 ms.
+//     is formed only beside the general step, which a z takes that is near the bailout or has a
+//     high part below 2^-200 or a low part below 2^-700 (not 0), where a product could underflow.
+// The steps run in blocks whose tests are gathered into three words; where they fail, the block is
+// taken again from its start by general steps, which the lanes of a warp do together.  With a test
+// and a branch a step on all four parts of z, the chain of a lone warp waited for each: a frame that
+// leaves most of the GPU idle is bound by it (128x96 Mandelbrot at 1e-18, depth 8500, REF_CUDA: 1559 us
+// with a test a step, 1230 with blocks and a flag, 1117 with the three words; 1217 before the short
+// step), a large one by the FP64 pipe (960x540 20.1 -> 15.5 ms, 16.2 with a test a step; 960x540
+// Burning Ship at 2e-17, depth 6000, REF_CPU 13.1 -> 7.2 ms, 7.5 with a test a step).  Blocks of 4, 8 and
+// 16 steps: 128x96 1117, 1117 and 1093 us; 599x400 Burning Ship at depth 6000 4246, 3954 and 3981;
+// 128x96 Mandelbrot set at depth 500 161, 163 and 166.
+constexpr int kDdBlock = 8;
 // Returns the escape step, or -1.
 template <int ARITH, bool SHIP>
 __device__ __forceinline__ int dd_quad_orbit(dd zx, dd zy, const dd cx, const dd cy, int max_iter,
                                              bool normalised, double& mag2_out) {
-    for (int k = 0; k < max_iter; ++k) {
-        if (!(normalised && plain_high(zx.hi) && plain_high(zy.hi) && plain_low(zx.lo) && plain_low(zy.lo))) {
-            const double mag2 = dd_sqr<ARITH>(zx).hi + dd_sqr<ARITH>(zy).hi;
+    for (int k = 0; k < max_iter;) {
+        while (normalised && max_iter - k >= kDdBlock) {
+            const dd bx = zx, by = zy;
+            PlainRange range;
+#pragma unroll
+            for (int t = 0; t < kDdBlock; ++t) {
+                range.add(zx, zy);
+                dd_step_plain<SHIP>(zx, zy, cx, cy);
+            }
+            if (!range.plain()) {
+                zx = bx;
+                zy = by;
+                break;
+            }
+            k += kDdBlock;
+        }
+        for (const int stop = normalised ? k + min(kDdBlock, max_iter - k) : max_iter; k < stop; ++k) {
+            const dd zx2 = dd_sqr<ARITH>(zx), zy2 = dd_sqr<ARITH>(zy);
+            const double mag2 = zx2.hi + zy2.hi;
             if (mag2 > kBailout) {
                 mag2_out = mag2;
                 return k;
             }
-            const dd2 n = dd_step_general<ARITH, SHIP>(dd2{zx, zy}, dd2{cx, cy});
-            zx = n.x;
-            zy = n.y;
-            continue;
-        }
-        const double x2 = zx.hi + zx.hi, y2 = zy.hi + zy.hi;
-        double p = zx.hi * zx.hi;
-        const dd zx2 = quick_sum(p, fma(zx.hi, zx.hi, -p) + x2 * zx.lo);
-        p = zy.hi * zy.hi;
-        const dd zy2 = quick_sum(p, fma(zy.hi, zy.hi, -p) + y2 * zy.lo);
-        p = x2 * zy.hi;
-        dd zxy = quick_sum(p, fma(x2, zy.hi, -p) + x2 * zy.lo + zx.lo * y2);  // 2 z_x z_y
-        zx = add_normalised(add_normalised(zx2, dd{-zy2.hi, -zy2.lo}), cx);
-        if (SHIP) {
-            // 2 |z_x| |z_y|: the low part's sign turns with the high part's
-            const int flip = __double2hiint(zxy.hi) & 0x80000000;
-            zxy.hi = fabs(zxy.hi);
-            zxy.lo = __hiloint2double(__double2hiint(zxy.lo) ^ flip, __double2loint(zxy.lo));
-            zy = add_normalised(zxy, dd{-cy.hi, -cy.lo});
-        } else {
-            zy = add_normalised(zxy, cy);
+            dd_step_general<ARITH, SHIP>(zx, zy, zx2, zy2, cx, cy);
         }
     }
     return -1;

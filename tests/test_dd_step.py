@@ -80,3 +80,53 @@ def test_device_equals_oracle_where_the_step_changes_path(case, ft, arith):
                "ap_render_pass")
     assert np.array_equal(km.cpu().numpy(), fr.kmap)
     assert np.array_equal(it.cpu().numpy().view(np.uint32), fr.iter_map.view(np.uint32))
+
+
+def plain_range(parts):
+    """PlainRange of ap_dd.cuh on columns (x.hi, y.hi, x.lo, y.lo): high words, unsigned."""
+    h = [(p.view(np.uint64) >> np.uint64(32)).astype(np.uint32) & np.uint32(0x7fffffff) for p in parts]
+    high = np.minimum(h[0] - np.uint32(1), h[1] - np.uint32(1))
+    low = np.minimum(h[2] - np.uint32(1), h[3] - np.uint32(1))
+    return ((np.maximum(h[0], h[1]) < 0x4066a000) & (high >= ((1023 - 200) << 20) - 1) & (low >= ((1023 - 700) << 20) - 1))
+
+
+def test_range_words_are_the_ranges_they_stand_for():
+    """Both edges of each range, zeros of both signs, infinities and NaN of both signs, in every part.  (Numbers below
+    2^-1042, whose high word is 0, count as 0.)"""
+    inf, nan = np.inf, np.nan
+    edges = [0.0, 2.0 ** -1042, 2.0 ** -1000, 2.0 ** -700, np.nextafter(2.0 ** -700, 0), 2.0 ** -200,
+             np.nextafter(2.0 ** -200, 0), 1.0, 2.0, np.nextafter(181.0, 0), 181.0, 256.0, 1e300, inf, nan]
+    v = np.array(edges + [-e for e in edges])
+    grid = [g.ravel().copy() for g in np.meshgrid(v, v, v, v)]
+    with np.errstate(invalid="ignore"):
+        a = np.abs(np.array(grid))
+        want = np.ones(a.shape[1], bool)
+        for q in (0, 1):
+            want &= (a[q] < 181.0) & ((a[q] == 0.0) | (a[q] >= 2.0 ** -200))
+        for q in (2, 3):
+            want &= (a[q] == 0.0) | (a[q] >= 2.0 ** -700) | np.isnan(a[q])  # a NaN low part has a NaN high one
+    assert np.array_equal(plain_range(grid), want)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("arith", [abi.AP_ARITH_REF_CPU, abi.AP_ARITH_REF_CUDA])
+@pytest.mark.parametrize("ft", [0, 1, 2])
+@pytest.mark.parametrize("max_iter", [0, 1, 7, 8, 9, 16, 17, 40, 203])
+def test_depths_that_end_anywhere_in_a_block(max_iter, ft, arith):
+    """The whole sets (escapes at every place of a block, a zero row, bounded pixels)."""
+    import oracle
+    import torch
+    W, H = 41, 33
+    p = abi.new_params(width=W, height=H, factor=1, max_iter=max_iter, fractal_type=ft, tier=abi.AP_TIER_DD, arith=arith,
+                       mode=abi.AP_MODE_COARSE, flags=abi.AP_FLAG_NO_RGB, x_min_hi=-2.1, x_min_lo=1e-18, y_max_hi=1.5,
+                       dx_hi=3.2 / 40, dy_hi=3.0 / 32, julia_cx_hi=-0.8, julia_cx_lo=1e-20, julia_cy_hi=0.156)
+    fr = oracle.Frame(W, H)
+    oracle.render_pass(p, fr)
+    it = torch.empty((H, W), dtype=torch.float32, device="cuda")
+    km = torch.empty((H, W), dtype=torch.int32, device="cuda")
+    b = abi.ApFrameBuffers()
+    b.iter_map, b.kmap = C.c_void_p(it.data_ptr()), C.c_void_p(km.data_ptr())
+    _lib.check(_lib.load().ap_render_pass(C.byref(p), C.byref(b), C.c_void_p(torch.cuda.current_stream().cuda_stream)),
+               "ap_render_pass")
+    assert np.array_equal(km.cpu().numpy(), fr.kmap)
+    assert np.array_equal(it.cpu().numpy().view(np.uint32), fr.iter_map.view(np.uint32))
