@@ -214,6 +214,13 @@ __device__ __forceinline__ int leap_level(const double* __restrict__ row, double
     return lo;
 }
 
+// Whether |dz|^2 (its high word) is not below a record's safe radius: unsigned words, so that a NaN of
+// either sign (CUDA's own has the sign bit set) lies above every radius and a NaN delta is always
+// tested -- the end of the reference is a radius of 0, which nothing passes untested.
+__device__ __forceinline__ bool outside(int dz_mag2_hi, double safe) {
+    return (unsigned)dz_mag2_hi >= (unsigned)__double2hiint(safe);
+}
+
 __device__ __forceinline__ bool not_finite(double v) {
     return (__double2hiint(v) & 0x7ff00000) == 0x7ff00000;
 }
@@ -402,7 +409,7 @@ __device__ __forceinline__ void pixel_advance(const ApFrameParams& p, const ApFr
             // and outside the level-0 BLA radius (no leap), the step runs straight
             // through.  The packed radii are 0 wherever k + 2^d >= ref_len, so no level
             // is admissible at the last step without a separate bound check.
-            const bool unsafe = dz_hi >= __double2hiint(Z.z);
+            const bool unsafe = outside(dz_hi, Z.z);
             const bool leap = BLA && (dz_mag2 < Z.w);
             act = kActStep;
             if (unsafe || leap) {
@@ -636,7 +643,7 @@ __device__ __forceinline__ void rebase_advance(const ApFrameParams& p, const ApF
         }
         // ap_pack_orbit leaves the orbit's last record (m == ref_len) with safe radius 0,
         // so the end of the reference takes this branch without a test of its own
-        const bool unsafe = dz_hi >= __double2hiint(Z.z);
+        const bool unsafe = outside(dz_hi, Z.z);
         const bool leap = BLA && (dz_mag2 < Z.w);
         act = kActStep;
         if (unsafe || leap) {
@@ -645,9 +652,9 @@ __device__ __forceinline__ void rebase_advance(const ApFrameParams& p, const ApF
                 const double zx = rx + dzx, zy = ry + dzy;
                 const double mag2 = kFast ? fma(zx, zx, zy * zy) : zx * zx + zy * zy;
                 // high words decide most: neither test fires where |z|^2's lies above |dz|^2's
-                // and below the bailout's (NaN lies above it)
-                const int mag_hi = __double2hiint(mag2);
-                if (mag_hi > dz_hi && mag_hi < 0x40f00000 && m != ref_len) {
+                // and below the bailout's (unsigned: NaN lies above it)
+                const unsigned mag_hi = (unsigned)__double2hiint(mag2);
+                if (mag_hi > (unsigned)dz_hi && mag_hi < 0x40f00000u && m != ref_len) {
                 } else if (!(mag2 <= kBailout)) {
                     esc_mag2 = mag2;
                     act = kActEscaped;
