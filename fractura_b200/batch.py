@@ -200,7 +200,8 @@ def _tile_inputs(t, ref, arith, bla_form, torch, stream, L, scratch):
         raise NotImplementedError("one-pass rebasing serves Mandelbrot, Burning Ship and Multibrot tiles")
     if rebase:
         flags |= abi.AP_FLAG_REBASE
-    if use_bla and spans_allowed(t.fractal_type, ACCURATE_BLA_EPS if bla_form == "accurate" else float(t.bla_tol)):
+    if use_bla and spans_allowed(t.fractal_type, ACCURATE_BLA_EPS if bla_form == "accurate" else float(t.bla_tol),
+                                 loosest=1e-4):
         flags |= abi.AP_FLAG_SPANS
     p = abi.new_params(width=t.W, height=t.H, factor=1, max_iter=int(t.max_iter),
                        fractal_type=int(t.fractal_type),

@@ -124,15 +124,15 @@ __device__ __forceinline__ void slot_store_run(BatchSlots& S, int q, const Pixel
 // state is then back in slot q.  One variant per (profile, formula class, BLA,
 // rebasing): separate functions, so each keeps the register allocation it has in the
 // per-frame kernel.
-template <int ARITH, int FT, bool BLA, bool REBASE>
+template <int ARITH, int FT, bool BLA, bool REBASE, bool SPANS>
 __device__ __noinline__ bool slot_run(const ApTileDesc* __restrict__ t, BatchSlots& S, int q, Round round) {
     const ApFrameBuffers b = tile_buffers(t);
     PixelRun s;
     slot_load_run(S, q, s, REBASE);
     if (REBASE)
-        rebase_advance<ARITH, FT, BLA, true>(t->p, b, s, round, S.cycles, q);
+        rebase_advance<ARITH, FT, BLA, true, true, SPANS>(t->p, b, s, round, S.cycles, q);
     else
-        pixel_advance<ARITH, FT, BLA, true>(t->p, b, s, round, S.cycles, q);
+        pixel_advance<ARITH, FT, BLA, true, SPANS>(t->p, b, s, round, true, S.cycles, q);
     if (s.stage == 3) {
         s.idx = S.idx[q];
         s.k0 = S.k0[q];
@@ -247,26 +247,29 @@ __device__ __forceinline__ bool batch_run(const ApTileDesc* t, BatchSlots& S, in
     constexpr int kPlain = (ARITH == AP_ARITH_FAST) ? AP_ARITH_REF_CUDA : ARITH;
     if (t->p.tier == AP_TIER_FLOATEXP32) return fe32_batch_run(t, S, q, round);
     const bool bla = t->p.bla_levels > 1 && t->bla_packed != nullptr;
+    const bool spans = (t->p.flags & AP_FLAG_SPANS) != 0;
     if (t->p.flags & AP_FLAG_REBASE) {
         switch (t->p.fractal_type) {
-        case 1: return slot_run<ARITH, kFtShip, false, true>(t, S, q, round);
+        case 1: return slot_run<ARITH, kFtShip, false, true, false>(t, S, q, round);
         case 4:
-            return bla ? slot_run<ARITH, kFtMulti, true, true>(t, S, q, round)
-                       : slot_run<ARITH, kFtMulti, false, true>(t, S, q, round);
+            return bla ? slot_run<ARITH, kFtMulti, true, true, false>(t, S, q, round)
+                       : slot_run<ARITH, kFtMulti, false, true, false>(t, S, q, round);
         default:
-            return bla ? slot_run<ARITH, kFtQuad, true, true>(t, S, q, round)
-                       : slot_run<ARITH, kFtQuad, false, true>(t, S, q, round);
+            if (!bla) return slot_run<ARITH, kFtQuad, false, true, true>(t, S, q, round);
+            return spans ? slot_run<ARITH, kFtQuad, true, true, true>(t, S, q, round)
+                         : slot_run<ARITH, kFtQuad, true, true, false>(t, S, q, round);
         }
     }
     switch (t->p.fractal_type) {
     case 1:
-    case 3: return slot_run<kPlain, kFtShip, false, false>(t, S, q, round);
+    case 3: return slot_run<kPlain, kFtShip, false, false, false>(t, S, q, round);
     case 4:
-        return bla ? slot_run<kPlain, kFtMulti, true, false>(t, S, q, round)
-                   : slot_run<kPlain, kFtMulti, false, false>(t, S, q, round);
+        return bla ? slot_run<kPlain, kFtMulti, true, false, false>(t, S, q, round)
+                   : slot_run<kPlain, kFtMulti, false, false, false>(t, S, q, round);
     default:
-        return bla ? slot_run<kPlain, kFtQuad, true, false>(t, S, q, round)
-                   : slot_run<kPlain, kFtQuad, false, false>(t, S, q, round);
+        if (!bla) return slot_run<kPlain, kFtQuad, false, false, true>(t, S, q, round);
+        return spans ? slot_run<kPlain, kFtQuad, true, false, true>(t, S, q, round)
+                     : slot_run<kPlain, kFtQuad, true, false, false>(t, S, q, round);
     }
 }
 

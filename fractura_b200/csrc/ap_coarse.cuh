@@ -5,17 +5,21 @@
 // by ap_render_pass when the buffers carry the packed orbit (ap_pack_orbit)
 // and, with BLA, the packed table (ap_pack_bla).  What changes is only how the
 // loop gets its inputs:
-//   * one 32-byte read per step: Z_k, a safe radius and the level-0 BLA
-//     radius.  While |dz| is below the safe radius neither the escape test nor
+//   * one 32-byte record per step: Z_k, a safe radius (its low word: the span window) and the
+//     level-0 BLA radius.  While |dz| is below the safe radius neither the escape test nor
 //     the Pauldelbrot test can fire, so |Z + dz|^2 and the threshold are not
 //     formed (the rounded |dz|^2 decides, and the BLA test reuses it);
+//   * runs of plain steps of z^2 + c without a test each (span_steps), stage 2 in blocks tested at
+//     their end, and whole cycles of bounded pixels added at once (cycle_visit);
 //   * the 16 BLA radii of step k in one 128-byte row.  Radii never increase
 //     with the level (each level's radius is the min of its first half's), and
 //     levels past the end of the orbit hold 0, so the largest admissible level
-//     -- the reference's top-down scan -- is found by a 4-probe binary search;
+//     -- the reference's top-down scan -- is a count, taken in two rounds of three loads;
 //   * formula, BLA presence and arithmetic profile are template parameters;
 //   * no colouring (ap_colour runs afterwards), keeping registers low.
 #pragma once
+
+#include <climits>
 
 #include "ap_common.cuh"
 #include "ap_fp64.cuh"
@@ -51,11 +55,13 @@ __device__ __forceinline__ double fold_delta(double Z, double z, double dz, doub
     return __hiloint2double(__double2hiint(v) ^ (s & 0x80000000), __double2loint(v));
 }
 
-// 32-byte record (32-byte aligned) through the read-only path, as one 256-bit load.
+// 32-byte record through the read-only path, as two 128-bit loads: the loops wait for it, and one
+// 256-bit load takes 58 cycles where these take 40 (1920x1080 at 1e-26, one-pass rebasing with leaps,
+// 19.9 -> 19.4 ms; at 1e-160 without leaps 10.4 -> 9.7).
 __device__ __forceinline__ double4 ldg4(const double4* p) {
-    double4 r;
-    asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(r.x), "=d"(r.y), "=d"(r.z), "=d"(r.w) : "l"(p));
-    return r;
+    const double2* q = reinterpret_cast<const double2*>(p);
+    const double2 a = __ldg(q), c = __ldg(q + 1);
+    return make_double4(a.x, a.y, c.x, c.y);
 }
 
 // Cycle detection.  A bounded pixel mostly settles on an exact cycle: its state returns bit for
@@ -66,39 +72,54 @@ __device__ __forceinline__ double4 ldg4(const double4* p) {
 //     a cycle of its own: Z_{m+p} = Z_m bit for bit from m = s0 on, found by ap_pack_orbit),
 //     against one at the same phase of the tail: with no restart in between, or at the same m.
 // Brent's search: each visited state is compared with one kept state, and the kept one is renewed
-// at visits 1, 2, 4, ...  The kept states live in shared memory, one per thread (28 bytes): they
-// are touched at restarts and every kTailStride steps only.
+// at visits 1, 2, 4, ...  Every fourth restart is visited (every 32nd of the Burning Ship), from the
+// kFirstRestart-th on (escaping pixels have few), and the tail every kTailStride steps: a cycle is
+// found as some whole number of its turns.
 // What bounds the repetition: leaps are capped so that k stays within max_iter and m + 2^d below
 // the orbit's end, where the radii of longer levels are 0.  A cycle of dk iterations holds no
 // leap longer than what remains of it, so each repetition that ends by max_iter (and, in the
 // tail, below the orbit's end) takes the same leaps; what is left after those runs as always.
 // -0 and 0 compare equal: no later magnitude depends on the sign of a zero.
 // Measured: 21 mixed tiles in one batch launch 187.6 -> 40.1 ms (bounded pixels were 96-99 % of
-// the iterations of the Multibrot tiles and settle after 1000-14000 steps; of max_iter 20000-90000);
-// a 1e-160 view without bounded pixels does not change.  Visits every 64 tail steps.
+// the iterations of the Multibrot tiles and settle after 1000-14000 steps; of max_iter 20000-90000).
+// The kept state, 28 bytes a pixel, is touched rarely.  The per-frame kernel keeps it in local memory
+// (volatile: not in registers): in shared memory it took L1 capacity from the records and rows, which
+// decide where the orbit is long (1920x1080 at 1e-26, 30000 records, leaps of tolerance 1e-5, one-pass
+// rebasing 6.23 -> 5.70 ms).  The batch kernel, whose slots move, keeps it in shared memory beside them.
 template <int N>
 struct CycleStore {
     double x[N], y[N];
     int k[N], m[N], visits[N];
 };
+struct CycleLocal {
+    volatile double x[1], y[1];
+    volatile int k[1], m[1], visits[1];
+};
 constexpr int kTailStride = 64;
+constexpr int kFirstRestart = 16;
 
 // The reference's tail: period p (0: none) from step s0 on, as ap_pack_orbit leaves it in the
 // last record's fourth slot (-(4096 s0 + p); no radius is negative, so no leap reads it as one).
 struct OrbitTail {
     int p, s0;
 };
+__device__ __forceinline__ double tail_word(const double4* __restrict__ orb, int ref_len) {
+    return -__ldg(reinterpret_cast<const double*>(orb + ref_len) + 3);
+}
+__device__ __forceinline__ bool has_tail(const double4* __restrict__ orb, int ref_len) {
+    return tail_word(orb, ref_len) > 0.0;
+}
 __device__ __forceinline__ OrbitTail orbit_tail(const double4* __restrict__ orb, int ref_len) {
-    const double t = -__ldg(reinterpret_cast<const double*>(orb + ref_len) + 3);
-    if (!(t > 0.0)) return {0, 0x7fffffff};
+    const double t = tail_word(orb, ref_len);
+    if (!(t > 0.0)) return {0, INT_MAX};
     const int s0 = (int)(t * (1.0 / 4096.0));
     return {(int)(t - 4096.0 * (double)s0), s0};
 }
 
 // A visit of state (x, y) at k iterations and reference index m (0: a restart; else a tail step
 // at the kept state's phase).  Returns the length of the cycle closed, 0 when none is.
-template <int N>
-__device__ __forceinline__ int cycle_visit(CycleStore<N>& C, int q, double x, double y, int k, int m) {
+template <class Store>
+__device__ __forceinline__ int cycle_visit(Store& C, int q, double x, double y, int k, int m) {
     const int visits = C.visits[q];
     if (visits > 0 && C.x[q] == x && C.y[q] == y) {
         const int km = C.k[q], mm = C.m[q];  // m = -1: z itself, past the reference (stage 2)
@@ -115,8 +136,8 @@ __device__ __forceinline__ int cycle_visit(CycleStore<N>& C, int q, double x, do
 }
 
 // Steps from tail step m to the next visit: to the kept state's phase, or (at_phase) past it.
-template <int N>
-__device__ __forceinline__ int tail_gap(const CycleStore<N>& C, int q, OrbitTail tail, int m, bool at_phase) {
+template <class Store>
+__device__ __forceinline__ int tail_gap(const Store& C, int q, OrbitTail tail, int m, bool at_phase) {
     if (at_phase) return ((kTailStride + tail.p - 1) / tail.p) * tail.p;
     if (C.visits[q] == 0 || C.m[q] == 0) return 0;
     const int d = (m - C.m[q]) % tail.p;
@@ -314,19 +335,28 @@ __device__ __forceinline__ void delta_step(const ApFrameParams& p, double rx, do
 
 // Whether the kSpan steps from here on are plain (ap_pack.cu's orbit_window, the low word of the
 // record's third slot): |dz|^2's exponent in the record's window, and |dc|^2's at least 60 below it
-// (dc_exp60: that exponent plus 60; a |dc|^2 that underflows has exponent 0, and is covered; no
-// exponent reaches 4096, which turns spans off).
+// (dc_exp60: that exponent plus 60; a |dc|^2 that underflows has exponent 0, and is covered).  Without
+// leaps only the window's end counts, and a smaller |dz| stays below what one of 2^30 |dc| grows to
+// (960x540 at 1e-26 without leaps, where deltas stay near |dc| for thousands of steps: 12.1 ms
+// without spans, 13.6 with spans from 2^30 |dc| on, 6.9 so).
+__device__ __forceinline__ int dc_exponent60(double dcx, double dcy) {
+    return (int)((unsigned)__double2hiint(dcx * dcx + dcy * dcy) >> 20) + 60;
+}
 template <bool BLA>
 __device__ __forceinline__ bool span_fits(int dz_mag2_hi, const double4 rec, int dc_exp60) {
-    const int e = dz_mag2_hi >> 20, w = __double2loint(rec.z);
-    return e < (w & 0xffff) && e >= dc_exp60 && (!BLA || e >= (__double2hiint(rec.w) >> 20) + (w >> 16));
+    const int e = (unsigned)dz_mag2_hi >> 20, w = __double2loint(rec.z);  // unsigned: no NaN fits
+    if (!BLA) return max(e, dc_exp60) < (w & 0xffff);
+    return e < (w & 0xffff) && e >= dc_exp60 && e >= (__double2hiint(rec.w) >> 20) + (w >> 16);
 }
 
 // kSpan steps from record `rec` on without a test: 7 instructions a step where a tested one takes
-// about 28.  Lanes that do not fit wait for those that do; taking a span only where most lanes fit
-// measured slower (1920x1080 Mandelbrot at 1e-160, one-pass rebasing, a frame: 1.58 ms without
-// spans, 1.50 with, 1.67 with that vote), and the Burning Ship, whose lanes disagree more, loses
-// (a 167x167 tile at depth 65541 18.8 ms without spans, 28 with): it takes none.
+// about 28.  Lanes that do not fit wait for those that do.  In a pass with leaps the lanes that took a
+// span go on into the tested step or the leap of the same loop iteration, together with the others: at
+// 1e-26, where lanes fall out of step, 1920x1080 with one-pass rebasing 19.2 ms with a test of the
+// next span instead, 17.1 so, 18.3 without spans.  Without leaps nearly all lanes fit again (1e-160:
+// 9.7 ms against 10.4).  Taking a span only where most lanes fit measured slower (1e-160: 1.67 ms
+// against 1.50), and the Burning Ship, whose lanes disagree more, loses (a 167x167 tile at depth 65541
+// 18.8 ms without spans, 28 with): it takes none.
 template <int ARITH, int FT>
 __device__ __forceinline__ void span_steps(const ApFrameParams& p, const double4* __restrict__ rec, double& dzx,
                                            double& dzy, double dcx, double dcy) {
@@ -347,219 +377,247 @@ __device__ __forceinline__ void span_steps(const ApFrameParams& p, const double4
 enum { kActStep = 0, kActMoved = 1, kActEscaped = 2, kActNotFinite = 3 };
 __device__ __forceinline__ void value_barrier(int& v) { asm volatile("" : "+r"(v)); }
 
-template <int ARITH, int FT, bool BLA, bool BUDGET, int N>
-__device__ __forceinline__ void pixel_advance(const ApFrameParams& p, const ApFrameBuffers& b, PixelRun& s,
-                                              Round round, CycleStore<N>& C, int q) {
+// Stage 1.  TAIL: the reference has a periodic tail, whose steps are visited (a 1e-160 frame, whose
+// reference has none, with the visits' bound in the loop 1.26 ms, without it 1.24; with one-pass
+// rebasing 1.18 and 1.09).  SPANS: z^2 + c whose runs of plain steps are taken as spans.
+template <int ARITH, int FT, bool BLA, bool BUDGET, bool TAIL, bool SPANS, class Store>
+__device__ __forceinline__ void stage1_advance(const ApFrameParams& p, const ApFrameBuffers& b, PixelRun& s,
+                                               Round& round, Store& C, int q) {
     constexpr bool kCpu = (ARITH == AP_ARITH_REF_CPU);
     constexpr bool kMerge = (FT == kFtMulti);
     const bool julia = (p.fractal_type == 2 || p.fractal_type == 3);
     const int ref_len = p.ref_len, max_iter = p.max_iter;
     const double4* __restrict__ orb = reinterpret_cast<const double4*>(b.orbit_packed);
-    const double inv_ln = inv_ln_for(p.fractal_type, p.gen_n);
     int k = s.k, glitch = s.glitch, leaps = s.leaps, skipped = s.skipped;
     SampleOut o = s.o;
-
-    if (s.stage == 1) {
-        double dzx = s.dzx, dzy = s.dzy;
-        const double dcpx = julia ? 0.0 : s.dcx, dcpy = julia ? 0.0 : s.dcy;
-        const bool strict = p.strict_glitch > 0;
-        const bool esc_glitch = (p.flags & AP_FLAG_ESCAPE_GLITCH) != 0;
-        const double* __restrict__ R = b.bla_packed;
-        const double4* __restrict__ AB =
-            reinterpret_cast<const double4*>(b.bla_packed + (size_t)ref_len * 16);
-        const int max_level = p.bla_levels - 1;
-        bool paused = false;
-        int act = kActStep;
-        double esc_mag2 = 0.0;
-        const int dc_exp60 = BLA && !(p.flags & AP_FLAG_SPANS)
-                                 ? 4096 : (__double2hiint(dcpx * dcpx + dcpy * dcpy) >> 20) + 60;
-        // the loop runs to `bound`: the orbit's end, or the next visited step of its tail
-        // (past step 15, from which on the Pauldelbrot test looks at every step)
-        int bound = min(ref_len, max(k, max(16, orbit_tail(orb, ref_len).s0)));
-        for (;;) {
-            if (k >= bound) {
-                if (k >= ref_len) break;
-                const OrbitTail tail = orbit_tail(orb, ref_len);
-                int gap = tail_gap(C, q, tail, k, false);
-                if (gap == 0) {
-                    const int dk = cycle_visit(C, q, dzx, dzy, k, k);
-                    if (dk > 0) {
-                        const int jump = (ref_len - 1 - k) / dk * dk;
-                        k += jump;
-                        skipped += jump;
-                    }
-                    gap = tail_gap(C, q, tail, k, true);
+    double dzx = s.dzx, dzy = s.dzy;
+    const double dcpx = julia ? 0.0 : s.dcx, dcpy = julia ? 0.0 : s.dcy;
+    const bool strict = p.strict_glitch > 0;
+    const bool esc_glitch = (p.flags & AP_FLAG_ESCAPE_GLITCH) != 0;
+    const double* __restrict__ R = b.bla_packed;
+    const double4* __restrict__ AB =
+        reinterpret_cast<const double4*>(b.bla_packed + (size_t)ref_len * 16);
+    const int max_level = p.bla_levels - 1;
+    bool paused = false;
+    int act = kActStep;
+    double esc_mag2 = 0.0;
+    const int dc_exp60 = dc_exponent60(dcpx, dcpy);
+    // the loop runs to `bound`: the orbit's end, or the next visited step of its tail
+    // (past step 15, from which on the Pauldelbrot test looks at every step)
+    int bound = TAIL ? min(ref_len, max(k, max(16, orbit_tail(orb, ref_len).s0))) : ref_len;
+    for (;;) {
+        if (k >= bound) {
+            if (!TAIL || k >= ref_len) break;
+            const OrbitTail tail = orbit_tail(orb, ref_len);
+            int gap = tail_gap(C, q, tail, k, false);
+            if (gap == 0) {
+                const int dk = cycle_visit(C, q, dzx, dzy, k, k);
+                if (dk > 0) {
+                    const int jump = (ref_len - 1 - k) / dk * dk;
+                    k += jump;
+                    skipped += jump;
                 }
-                bound = gap < ref_len - k ? k + gap : ref_len;
+                gap = tail_gap(C, q, tail, k, true);
             }
-            if (BUDGET && round.over()) {
-                paused = true;
-                break;
-            }
-            const double4 Z = ldg4(orb + k);
-            const double rx = Z.x, ry = Z.y;
-            const double dz_mag2 = dzx * dzx + dzy * dzy;
-            const int dz_hi = __double2hiint(dz_mag2);
-            if (FT == kFtQuad && k + kSpan <= bound && span_fits<BLA>(dz_hi, Z, dc_exp60)) {
-                span_steps<ARITH, FT>(p, orb + k, dzx, dzy, dcpx, dcpy);
-                k += kSpan;
-                continue;
-            }
-            // One branch on the common path: inside the safe radius (no test can fire)
-            // and outside the level-0 BLA radius (no leap), the step runs straight
-            // through.  The packed radii are 0 wherever k + 2^d >= ref_len, so no level
-            // is admissible at the last step without a separate bound check.
-            const bool unsafe = outside(dz_hi, Z.z);
-            const bool leap = BLA && (dz_mag2 < Z.w);
-            act = kActStep;
-            if (unsafe || leap) {
-                if (unsafe) {
-                    const double zx = rx + dzx, zy = ry + dzy;
-                    const double mag2 = zx * zx + zy * zy;
-                    const double r_mag2 = rx * rx + ry * ry;
-                    if (mag2 > kBailout) {
-                        if (esc_glitch && strict && k > 15 && r_mag2 < 4.0) glitch = 1;
-                        esc_mag2 = mag2;
-                        act = kActEscaped;
-                    } else {
-                        // the Pauldelbrot threshold, as the reference forms it
-                        const double thr = r_mag2 > 1e-8 ? 1e-6 * r_mag2 : -1.0;
-                        if (strict && k > 15 && mag2 < thr) glitch = 1;
-                    }
-                }
-                if (leap && act == kActStep) {
-                    int hi = max_level;
-                    if (dz_mag2 == 0.0 && (dzx != 0.0 || dzy != 0.0)) hi = min(hi, 8);
-                    const int lo = leap_level(R + (size_t)k * 16, dz_mag2, hi);
-                    leap_delta<kCpu>(ldg4(AB + (size_t)k * 16 + lo), dzx, dzy, dcpx, dcpy);
-                    act = kActNotFinite;
-                    if (!not_finite(dzx) && !not_finite(dzy)) {
-                        act = kActMoved;
-                        k += 1 << lo;
-                        ++leaps;
-                        skipped += 1 << lo;
-                    }
+            bound = gap < ref_len - k ? k + gap : ref_len;
+        }
+        if (BUDGET && round.over()) {
+            paused = true;
+            break;
+        }
+        double4 Z = ldg4(orb + k);
+        double dz_mag2 = dzx * dzx + dzy * dzy;
+        if (SPANS && k + kSpan <= bound && span_fits<BLA>(__double2hiint(dz_mag2), Z, dc_exp60)) {
+            span_steps<ARITH, FT>(p, orb + k, dzx, dzy, dcpx, dcpy);
+            k += kSpan;
+            if (!BLA || k >= bound) continue;
+            Z = ldg4(orb + k);
+            dz_mag2 = dzx * dzx + dzy * dzy;
+        }
+        const double rx = Z.x, ry = Z.y;
+        const int dz_hi = __double2hiint(dz_mag2);
+        // One branch on the common path: inside the safe radius (no test can fire)
+        // and outside the level-0 BLA radius (no leap), the step runs straight
+        // through.  The packed radii are 0 wherever k + 2^d >= ref_len, so no level
+        // is admissible at the last step without a separate bound check.
+        const bool unsafe = outside(dz_hi, Z.z);
+        const bool leap = BLA && (dz_mag2 < Z.w);
+        act = kActStep;
+        if (unsafe || leap) {
+            if (unsafe) {
+                const double zx = rx + dzx, zy = ry + dzy;
+                const double mag2 = zx * zx + zy * zy;
+                const double r_mag2 = rx * rx + ry * ry;
+                if (mag2 > kBailout) {
+                    if (esc_glitch && strict && k > 15 && r_mag2 < 4.0) glitch = 1;
+                    esc_mag2 = mag2;
+                    act = kActEscaped;
+                } else {
+                    // the Pauldelbrot threshold, as the reference forms it
+                    const double thr = r_mag2 > 1e-8 ? 1e-6 * r_mag2 : -1.0;
+                    if (strict && k > 15 && mag2 < thr) glitch = 1;
                 }
             }
-            if (kMerge) value_barrier(act);
-            if (act >= kActEscaped) break;
-            if (act == kActStep) {
-                delta_step<ARITH, FT>(p, rx, ry, dzx, dzy, dcpx, dcpy);
-                ++k;
+            if (leap && act == kActStep) {
+                int hi = max_level;
+                if (dz_mag2 == 0.0 && (dzx != 0.0 || dzy != 0.0)) hi = min(hi, 8);
+                const int lo = leap_level(R + (size_t)k * 16, dz_mag2, hi);
+                leap_delta<kCpu>(ldg4(AB + (size_t)k * 16 + lo), dzx, dzy, dcpx, dcpy);
+                act = kActNotFinite;
+                if (!not_finite(dzx) && !not_finite(dzy)) {
+                    act = kActMoved;
+                    k += 1 << lo;
+                    ++leaps;
+                    skipped += 1 << lo;
+                }
             }
         }
-        if (paused) {
-            s.dzx = dzx;
-            s.dzy = dzy;
-            s.k = k;
-            s.glitch = glitch;
-            s.leaps = leaps;
-            s.skipped = skipped;
-            return;
-        }
-        if (act >= kActEscaped) {
-            if (act == kActEscaped) {
-                o = escaped_sample(k, esc_mag2, inv_ln);
-            } else {
-                o = interior_sample();
-                o.s = (float)k;
-                o.s64 = (double)k;
-                o.k = k;
-                glitch = 1;
-            }
-            s.stage = 3;
-        } else {
-            // Stage 2: past the end of the reference orbit, iterate z directly.
-            const double4 Zend = ldg4(orb + ref_len);
-            s.zx = Zend.x + dzx;
-            s.zy = Zend.y + dzy;
-            if (ref_len < max_iter) glitch = 1;
-            s.k2 = k;
-            o = interior_sample();
-            s.stage = 2;
-        }
-    }
-
-    if (s.stage == 2) {
-        double zx = s.zx, zy = s.zy;
-        const double cx = julia ? p.julia_cx_hi : p.ref_cx + s.dcx;
-        const double cy = julia ? p.julia_cy_hi : p.ref_cy + s.dcy;
-        const bool nan_guard = (p.flags & AP_FLAG_NAN_GUARD) != 0;
-        bool paused = false;
-        constexpr int kKind = FT == kFtQuad ? kKindQuad : FT == kFtShip ? kKindShip : kKindMulti;
-        const bool growing = fp64_growing(kKind, cx, cy, p.gen_n, p.gen_kr, p.gen_ki);
-        const bool doubles = fp64_doubles(zy, cy);
-        int tested = 0;  // steps to test one by one before the next block
-        while (k < max_iter) {
-            if (BUDGET && round.over()) {
-                paused = true;
-                break;
-            }
-            // blocks tested at their end only, as in direct iteration (fp64_orbit, ap_fp64.cuh)
-            if (growing && tested == 0 && k + kBlock <= max_iter) {
-                const double bx = zx, by = zy;
-                for_degree(kKind, p.gen_n, doubles, [&](auto n) {
-#pragma unroll
-                    for (int t = 0; t < kBlock; ++t)
-                        fp64_step<AP_ARITH_REF_CUDA, kKind, n()>(zx, zy, zx * zx, zy * zy, cx, cy, p.gen_n, p.gen_kr,
-                                                                 p.gen_ki);
-                });
-                if (zx * zx + zy * zy <= kBailout) {
-                    k += kBlock;
-                    if (cycle_visit(C, q, zx, zy, k, -1) > 0) {  // it repeats: never escapes
-                        s.k2 += max_iter - k;
-                        skipped += max_iter - k;
-                        k = max_iter;
-                    }
-                    continue;
-                }
-                zx = bx;
-                zy = by;
-                tested = kBlock + 1;
-            }
-            if (tested > 0) --tested;
-            const double zx2 = zx * zx, zy2 = zy * zy;
-            const double mag2 = zx2 + zy2;
-            if (nan_guard && (isnan(mag2) || isinf(mag2))) {
-                o.s = (float)k;
-                o.s64 = (double)k;
-                o.k = k;
-                glitch = 1;
-                break;
-            }
-            if (mag2 > kBailout) {
-                o = escaped_sample(k, mag2, inv_ln);
-                break;
-            }
-            if (FT == kFtQuad) {
-                zy = 2.0 * zx * zy + cy;
-                zx = zx2 - zy2 + cx;
-            } else if (FT == kFtShip) {
-                zy = 2.0 * fabs(zx) * fabs(zy) - cy;
-                zx = zx2 - zy2 + cx;
-            } else {
-                double zr = zx, zi = zy;
-                for_powers(p.gen_n, [&]() {
-                    const double nr = zr * zx - zi * zy, ni = zr * zy + zi * zx;
-                    zr = nr;
-                    zi = ni;
-                });
-                const double kzr = p.gen_kr * zx - p.gen_ki * zy;
-                const double kzi = p.gen_kr * zy + p.gen_ki * zx;
-                zx = zr + kzr + cx;
-                zy = zi + kzi + cy;
-            }
+        if (kMerge) value_barrier(act);
+        if (act >= kActEscaped) break;
+        if (act == kActStep) {
+            delta_step<ARITH, FT>(p, rx, ry, dzx, dzy, dcpx, dcpy);
             ++k;
         }
-        s.zx = zx;
-        s.zy = zy;
-        if (!paused) s.stage = 3;
+    }
+    if (paused) {
+        s.dzx = dzx;
+        s.dzy = dzy;
+        s.k = k;
+        s.glitch = glitch;
+        s.leaps = leaps;
+        s.skipped = skipped;
+        return;
+    }
+    if (act >= kActEscaped) {
+        if (act == kActEscaped) {
+            o = escaped_sample(k, esc_mag2, inv_ln_for(p.fractal_type, p.gen_n));
+        } else {
+            o = interior_sample();
+            o.s = (float)k;
+            o.s64 = (double)k;
+            o.k = k;
+            glitch = 1;
+        }
+        s.stage = 3;
+    } else {
+        // Stage 2: past the end of the reference orbit, iterate z directly.
+        const double4 Zend = ldg4(orb + ref_len);
+        s.zx = Zend.x + dzx;
+        s.zy = Zend.y + dzy;
+        if (ref_len < max_iter) glitch = 1;
+        s.k2 = k;
+        o = interior_sample();
+        s.stage = 2;
     }
     s.k = k;
     s.glitch = glitch;
     s.leaps = leaps;
     s.skipped = skipped;
     s.o = o;
+}
+
+// Stage 2: direct iteration past the end of the reference.
+template <int FT, bool BUDGET, class Store>
+__device__ __forceinline__ void stage2_advance(const ApFrameParams& p, PixelRun& s, Round& round, Store& C, int q) {
+    const bool julia = (p.fractal_type == 2 || p.fractal_type == 3);
+    const int max_iter = p.max_iter;
+    const double inv_ln = inv_ln_for(p.fractal_type, p.gen_n);
+    int k = s.k, glitch = s.glitch, skipped = s.skipped;
+    SampleOut o = s.o;
+    double zx = s.zx, zy = s.zy;
+    const double cx = julia ? p.julia_cx_hi : p.ref_cx + s.dcx;
+    const double cy = julia ? p.julia_cy_hi : p.ref_cy + s.dcy;
+    const bool nan_guard = (p.flags & AP_FLAG_NAN_GUARD) != 0;
+    bool paused = false;
+    constexpr int kKind = FT == kFtQuad ? kKindQuad : FT == kFtShip ? kKindShip : kKindMulti;
+    const bool growing = fp64_growing(kKind, cx, cy, p.gen_n, p.gen_kr, p.gen_ki);
+    const bool doubles = fp64_doubles(zy, cy);
+    CycleStore<1> R;  // in registers: visited after every block
+    R.visits[0] = 0;
+    int tested = 0;  // steps to test one by one before the next block
+    while (k < max_iter) {
+        if (BUDGET && round.over()) {
+            paused = true;
+            break;
+        }
+        // blocks tested at their end only, as in direct iteration (fp64_orbit, ap_fp64.cuh)
+        if (growing && tested == 0 && k + kBlock <= max_iter) {
+            const double bx = zx, by = zy;
+            for_degree(kKind, p.gen_n, doubles, [&](auto n) {
+#pragma unroll
+                for (int t = 0; t < kBlock; ++t)
+                    fp64_step<AP_ARITH_REF_CUDA, kKind, n()>(zx, zy, zx * zx, zy * zy, cx, cy, p.gen_n, p.gen_kr,
+                                                             p.gen_ki);
+            });
+            if (zx * zx + zy * zy <= kBailout) {
+                k += kBlock;
+                // a state that repeats never escapes
+                if ((BUDGET ? cycle_visit(C, q, zx, zy, k, -1) : cycle_visit(R, 0, zx, zy, k, -1)) > 0) {
+                    s.k2 += max_iter - k;
+                    skipped += max_iter - k;
+                    k = max_iter;
+                }
+                continue;
+            }
+            zx = bx;
+            zy = by;
+            tested = kBlock + 1;
+        }
+        if (tested > 0) --tested;
+        const double zx2 = zx * zx, zy2 = zy * zy;
+        const double mag2 = zx2 + zy2;
+        if (nan_guard && (isnan(mag2) || isinf(mag2))) {
+            o.s = (float)k;
+            o.s64 = (double)k;
+            o.k = k;
+            glitch = 1;
+            break;
+        }
+        if (mag2 > kBailout) {
+            o = escaped_sample(k, mag2, inv_ln);
+            break;
+        }
+        if (FT == kFtQuad) {
+            zy = 2.0 * zx * zy + cy;
+            zx = zx2 - zy2 + cx;
+        } else if (FT == kFtShip) {
+            zy = 2.0 * fabs(zx) * fabs(zy) - cy;
+            zx = zx2 - zy2 + cx;
+        } else {
+            double zr = zx, zi = zy;
+            for_powers(p.gen_n, [&]() {
+                const double nr = zr * zx - zi * zy, ni = zr * zy + zi * zx;
+                zr = nr;
+                zi = ni;
+            });
+            const double kzr = p.gen_kr * zx - p.gen_ki * zy;
+            const double kzi = p.gen_kr * zy + p.gen_ki * zx;
+            zx = zr + kzr + cx;
+            zy = zi + kzi + cy;
+        }
+        ++k;
+    }
+    s.zx = zx;
+    s.zy = zy;
+    if (!paused) s.stage = 3;
+    s.k = k;
+    s.glitch = glitch;
+    s.skipped = skipped;
+    s.o = o;
+}
+
+// Both stages of a single-reference pixel.  The lanes of a warp enter stage 2 together: the barrier
+// keeps the compiler from going from a loop's exit straight into it, lane by lane (a 437x437 view at
+// 5e-27 with a short reference 2.07 ms, 1.47 with it).
+template <int ARITH, int FT, bool BLA, bool BUDGET, bool SPANS, class Store>
+__device__ __forceinline__ void pixel_advance(const ApFrameParams& p, const ApFrameBuffers& b, PixelRun& s,
+                                              Round round, bool tail, Store& C, int q) {
+    if (s.stage == 1) {
+        if (tail) stage1_advance<ARITH, FT, BLA, BUDGET, true, SPANS>(p, b, s, round, C, q);
+        else stage1_advance<ARITH, FT, BLA, BUDGET, false, SPANS>(p, b, s, round, C, q);
+    }
+    value_barrier(s.stage);
+    if (s.stage == 2) stage2_advance<FT, BUDGET>(p, s, round, C, q);
 }
 
 // One-pass rebasing (AP_FLAG_REBASE), for orbits that start at Z_0 = 0 (fractal
@@ -575,9 +633,9 @@ __device__ __forceinline__ void pixel_advance(const ApFrameParams& p, const ApFr
 // also be AP_ARITH_FAST: |dz|^2, |z|^2 and every formula's step as fused multiply-adds
 // (about 10 FP64 instructions per Mandelbrot step on the common path; a Multibrot
 // power costs 14 instead of 22), leaps as the CUDA profile.
-template <int ARITH, int FT, bool BLA, bool BUDGET, int N>
+template <int ARITH, int FT, bool BLA, bool BUDGET, bool TAIL, bool SPANS, class Store>
 __device__ __forceinline__ void rebase_advance(const ApFrameParams& p, const ApFrameBuffers& b, PixelRun& s,
-                                               Round round, CycleStore<N>& C, int q) {
+                                               Round round, Store& C, int q) {
     constexpr bool kCpu = (ARITH == AP_ARITH_REF_CPU);
     constexpr bool kFast = (ARITH == AP_ARITH_FAST);
     constexpr bool kMerge = (FT == kFtMulti);
@@ -596,18 +654,24 @@ __device__ __forceinline__ void rebase_advance(const ApFrameParams& p, const ApF
     bool paused = false;
     int act = kActStep;
     double esc_mag2 = 0.0;
-    const int dc_exp60 = BLA && !(p.flags & AP_FLAG_SPANS)
-                             ? 4096 : (__double2hiint(dcpx * dcpx + dcpy * dcpy) >> 20) + 60;
-    // A restart at an orbit that starts at 0, without a leap there, needs no test at m = 0: z = dz
-    // has just been tested.  It goes straight to the step.
-    const double4 Zstart = ldg4(orb);
-    const bool zero_start = Zstart.x == 0.0 && Zstart.y == 0.0 && !(Zstart.w > 0.0);
+    const int dc_exp60 = dc_exponent60(dcpx, dcpy);
+    // A restart at an orbit that starts at 0, without a leap there, needs no test at m = 0: z = dz has
+    // just been tested.  Multibrot goes straight to the step (a 504x504 view of bounded pixels 11.2 ->
+    // 8.0 ms); Mandelbrot frames lose by it (1920x1080 at 1e-160 1.19 ms, 1.24 with it), and so does the
+    // Burning Ship (800x451 at depth 65541 25.9 and 29.0).
+    constexpr bool kStepOn = FT == kFtMulti;
+    // the Burning Ship restarts often and settles on a cycle rarely (127x127 at depth 12433: a visit at
+    // every restart 4.8 ms, every eighth 3.8, every 16th 3.6)
+    constexpr int kRestartStride = FT == kFtShip ? 32 : 4;
+    const double4 Zstart = kStepOn ? ldg4(orb) : make_double4(1.0, 0.0, 0.0, 0.0);
+    const bool step_on = kStepOn && Zstart.x == 0.0 && Zstart.y == 0.0 && !(Zstart.w > 0.0);
     // the loop runs to `bound`: lim, or the next visited step of the reference's tail
-    const int tail_s0 = max(1, orbit_tail(orb, ref_len).s0);
+    const int tail_s0 = TAIL ? max(1, orbit_tail(orb, ref_len).s0) : INT_MAX;
     int bound = min(lim, max(m, tail_s0));
     for (;;) {
+        if (!TAIL) bound = lim;
         if (m >= bound) {
-            if (m >= lim) break;
+            if (!TAIL || m >= lim) break;
             const OrbitTail tail = orbit_tail(orb, ref_len);
             int gap = tail_gap(C, q, tail, m, false);
             if (gap == 0) {
@@ -632,15 +696,17 @@ __device__ __forceinline__ void rebase_advance(const ApFrameParams& p, const ApF
             paused = true;
             break;
         }
-        const double4 Z = ldg4(orb + m);
-        double rx = Z.x, ry = Z.y;
-        const double dz_mag2 = kFast ? fma(dzx, dzx, dzy * dzy) : dzx * dzx + dzy * dzy;
-        const int dz_hi = __double2hiint(dz_mag2);
-        if (FT == kFtQuad && m + kSpan <= bound && span_fits<BLA>(dz_hi, Z, dc_exp60)) {
+        double4 Z = ldg4(orb + m);
+        double dz_mag2 = kFast ? fma(dzx, dzx, dzy * dzy) : dzx * dzx + dzy * dzy;
+        if (SPANS && m + kSpan <= bound && span_fits<BLA>(__double2hiint(dz_mag2), Z, dc_exp60)) {
             span_steps<ARITH, FT>(p, orb + m, dzx, dzy, dcpx, dcpy);
             m += kSpan;
-            continue;
+            if (!BLA || m >= bound) continue;
+            Z = ldg4(orb + m);
+            dz_mag2 = kFast ? fma(dzx, dzx, dzy * dzy) : dzx * dzx + dzy * dzy;
         }
+        double rx = Z.x, ry = Z.y;
+        const int dz_hi = __double2hiint(dz_mag2);
         // ap_pack_orbit leaves the orbit's last record (m == ref_len) with safe radius 0,
         // so the end of the reference takes this branch without a test of its own
         const bool unsafe = outside(dz_hi, Z.z);
@@ -651,11 +717,7 @@ __device__ __forceinline__ void rebase_advance(const ApFrameParams& p, const ApF
             if (unsafe) {
                 const double zx = rx + dzx, zy = ry + dzy;
                 const double mag2 = kFast ? fma(zx, zx, zy * zy) : zx * zx + zy * zy;
-                // high words decide most: neither test fires where |z|^2's lies above |dz|^2's
-                // and below the bailout's (unsigned: NaN lies above it)
-                const unsigned mag_hi = (unsigned)__double2hiint(mag2);
-                if (mag_hi > (unsigned)dz_hi && mag_hi < 0x40f00000u && m != ref_len) {
-                } else if (!(mag2 <= kBailout)) {
+                if (!(mag2 <= kBailout)) {
                     esc_mag2 = mag2;
                     act = kActEscaped;
                 } else if (mag2 < dz_mag2 || (m == ref_len && m > 0)) {
@@ -664,17 +726,19 @@ __device__ __forceinline__ void rebase_advance(const ApFrameParams& p, const ApF
                     lim -= m;
                     m = 0;
                     ++rebases;
-                    const int dk = cycle_visit(C, q, dzx, dzy, max_iter - lim, 0);
+                    const int dk = rebases > kFirstRestart && rebases % kRestartStride == 0 ? cycle_visit(C, q, dzx, dzy, max_iter - lim, 0) : 0;
                     if (dk > 0) {
                         const int jump = lim / dk * dk;
                         lim -= jump;
                         skipped += jump;
                     }
                     bound = min(lim, tail_s0);
-                    act = zero_start && lim > 0 ? kActStep : kActMoved;
-                    rx = 0.0;
-                    ry = 0.0;
-                    may_leap = false;
+                    act = step_on && lim > 0 ? kActStep : kActMoved;
+                    if (kStepOn) {
+                        rx = 0.0;
+                        ry = 0.0;
+                        may_leap = false;
+                    }
                 }
             }
             if (may_leap && act == kActStep) {
@@ -735,17 +799,23 @@ __device__ __forceinline__ void pixel_finish(const ApFrameParams& p, const ApFra
     }
 }
 
-// One pixel (i, j) of a coarse pass, start to finish (REBASE: AP_FLAG_REBASE).
-template <int ARITH, int FT, bool BLA, bool REBASE, int N>
+// One pixel (i, j) of a coarse pass, start to finish (REBASE: AP_FLAG_REBASE).  The tail is the orbit's,
+// so all pixels of a pass take one of the two loops.
+template <int ARITH, int FT, bool BLA, bool REBASE, bool SPANS>
 __device__ __forceinline__ void coarse_pixel(const ApFrameParams& p, const ApFrameBuffers& b, int i,
-                                             int j, CycleStore<N>& C, int q) {
+                                             int j) {
     PixelRun s;
     if (!pixel_begin<ARITH, FT>(p, b, i, j, s)) return;
-    C.visits[q] = 0;
-    if (REBASE)
-        rebase_advance<ARITH, FT, BLA, false>(p, b, s, Round{}, C, q);
-    else
-        pixel_advance<ARITH, FT, BLA, false>(p, b, s, Round{}, C, q);
+    CycleLocal C;
+    C.visits[0] = 0;
+    // one reference's Multibrot and Burning Ship loops run no faster without the visits
+    const bool tail = (!REBASE && FT != kFtQuad) || has_tail(reinterpret_cast<const double4*>(b.orbit_packed), p.ref_len);
+    if (REBASE) {
+        if (tail) rebase_advance<ARITH, FT, BLA, false, true, SPANS>(p, b, s, Round{}, C, 0);
+        else rebase_advance<ARITH, FT, BLA, false, false, SPANS>(p, b, s, Round{}, C, 0);
+    } else {
+        pixel_advance<ARITH, FT, BLA, false, SPANS>(p, b, s, Round{}, tail, C, 0);
+    }
     pixel_finish(p, b, s);
 }
 

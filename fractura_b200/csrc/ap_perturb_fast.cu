@@ -17,7 +17,7 @@ constexpr int kCoarseTile = AP_COARSE_TILE;
 constexpr int kCoarseThreads = kCoarseTile * kCoarseTile;
 constexpr int kCoarseScale = 256 / kCoarseThreads;  // blocks per 256-thread register budget
 
-template <int ARITH, int FT, bool BLA, bool REBASE>
+template <int ARITH, int FT, bool BLA, bool REBASE, bool SPANS>
 __global__ void __launch_bounds__(kCoarseThreads, (REBASE ? AP_REBASE_MIN_BLOCKS : 4) * kCoarseScale)
     perturb_coarse_kernel(const ApFrameParams p, const ApFrameBuffers b, int row0, int row_end) {
     // each warp takes an 8 x 4 patch of its block's pixels: neighbours follow similar
@@ -28,26 +28,29 @@ __global__ void __launch_bounds__(kCoarseThreads, (REBASE ? AP_REBASE_MIN_BLOCKS
     const int i = blockIdx.x * kCoarseTile + (w % kWarpsPerRow) * 8 + (l & 7);
     const int j = row0 + blockIdx.y * kCoarseTile + (w / kWarpsPerRow) * 4 + (l >> 3);
     if (i >= p.width || j >= row_end) return;
-    __shared__ CycleStore<kCoarseThreads> cycles;
-    coarse_pixel<ARITH, FT, BLA, REBASE>(p, b, i, j, cycles, threadIdx.x);
+    coarse_pixel<ARITH, FT, BLA, REBASE, SPANS>(p, b, i, j);
+}
+
+template <int ARITH, int FT, bool REBASE>
+static void launch_form(const ApFrameParams& p, const ApFrameBuffers& b, int r0, int r1, cudaStream_t st) {
+    dim3 grid((p.width + kCoarseTile - 1) / kCoarseTile, (r1 - r0 + kCoarseTile - 1) / kCoarseTile);
+    if (grid.y == 0) return;
+    constexpr int T = kCoarseThreads;
+    constexpr bool kQuad = FT == kFtQuad;
+    if (p.bla_levels <= 1) {
+        perturb_coarse_kernel<ARITH, FT, false, REBASE, kQuad><<<grid, T, 0, st>>>(p, b, r0, r1);
+    } else if (kQuad && (p.flags & AP_FLAG_SPANS)) {
+        perturb_coarse_kernel<ARITH, FT, true, REBASE, kQuad><<<grid, T, 0, st>>>(p, b, r0, r1);
+    } else {
+        perturb_coarse_kernel<ARITH, FT, true, REBASE, false><<<grid, T, 0, st>>>(p, b, r0, r1);
+    }
 }
 
 template <int ARITH, int FT>
 static void launch_ft(const ApFrameParams& p, const ApFrameBuffers& b, int r0, int r1, cudaStream_t st) {
-    dim3 grid((p.width + kCoarseTile - 1) / kCoarseTile, (r1 - r0 + kCoarseTile - 1) / kCoarseTile);
-    if (grid.y == 0) return;
-    const bool rebase = (p.flags & AP_FLAG_REBASE) != 0;
-    constexpr int T = kCoarseThreads;
-    if constexpr (ARITH == AP_ARITH_FAST) {  // validated: AP_ARITH_FAST passes are rebasing passes
-        if (p.bla_levels > 1) perturb_coarse_kernel<ARITH, FT, true, true><<<grid, T, 0, st>>>(p, b, r0, r1);
-        else perturb_coarse_kernel<ARITH, FT, false, true><<<grid, T, 0, st>>>(p, b, r0, r1);
-    } else if (p.bla_levels > 1) {
-        if (rebase) perturb_coarse_kernel<ARITH, FT, true, true><<<grid, T, 0, st>>>(p, b, r0, r1);
-        else perturb_coarse_kernel<ARITH, FT, true, false><<<grid, T, 0, st>>>(p, b, r0, r1);
-    } else {
-        if (rebase) perturb_coarse_kernel<ARITH, FT, false, true><<<grid, T, 0, st>>>(p, b, r0, r1);
-        else perturb_coarse_kernel<ARITH, FT, false, false><<<grid, T, 0, st>>>(p, b, r0, r1);
-    }
+    // validated: AP_ARITH_FAST passes are rebasing passes
+    if (ARITH == AP_ARITH_FAST || (p.flags & AP_FLAG_REBASE)) launch_form<ARITH, FT, true>(p, b, r0, r1, st);
+    else if constexpr (ARITH != AP_ARITH_FAST) launch_form<ARITH, FT, false>(p, b, r0, r1, st);
 }
 
 template <int ARITH>
