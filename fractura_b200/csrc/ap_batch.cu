@@ -22,6 +22,7 @@
 // that start together, share orbit records and branch alike.  Nothing waits on
 // anything outside the block: a block whose slots are empty once the queue has run
 // out exits.
+#include "ap_batch_map.cuh"
 #include "ap_coarse.cuh"
 #include "ap_fe32.cuh"
 
@@ -296,10 +297,9 @@ __device__ __noinline__ bool slot_begin(const ApTileDesc* __restrict__ t, int ti
 
 // Pixel u of the batch (patches of 256 pixels, numbered tile after tile; row-major in a
 // patch) -> its tile and its (i, j); false when it falls outside the tile.  Within a tile the
-// queue runs through the groups of 32 pixels in a scattered order (a multiplier coprime to
-// their number): the long-lived pixels of a tile lie together, and blocks that took them as
-// they lie kept a few SMs busy long after the others had run out of work (one 504x504 Multibrot
-// n = 5 tile 18.7 ms, 12.2 scattered).
+// queue runs through the groups of 32 pixels in a scattered order (batch_scatter): the long-lived
+// pixels of a tile lie together, and blocks that took them as they lie kept a few SMs busy long after
+// the others had run out of work (one 504x504 Multibrot n = 5 tile 18.7 ms, 12.2 scattered).
 __device__ __forceinline__ bool batch_pixel_at(const ApTileDesc* __restrict__ tiles,
                                                const int64_t* __restrict__ first, int n, int patch_w,
                                                int patch_h, long long u, int* tile, int* i, int* j) {
@@ -314,11 +314,8 @@ __device__ __forceinline__ bool batch_pixel_at(const ApTileDesc* __restrict__ ti
     *tile = lo;
     const ApTileDesc* t = tiles + lo;
     const long long patches = first[lo + 1] - first[lo];
-    const unsigned groups = (unsigned)(patches * 8);  // below 2^31 (a tile has fewer than 2^31 pixels)
-    unsigned g = (unsigned)((item - first[lo]) * 8) + (unsigned)(q >> 5);
-    if (patches % 7919) g = (unsigned)(g * 7919ull % groups);  // 7919 is an odd prime
-    const long long local = g >> 3;
-    const int w = (int)(g & 7) * 32 + (q & 31);
+    int w;
+    const long long local = batch_scatter(patches, item - first[lo], q, &w);
     const int px = (t->p.width + patch_w - 1) / patch_w;
     *i = (int)(local % px) * patch_w + w % patch_w;
     *j = (int)(local / px) * patch_h + w / patch_w;
