@@ -139,7 +139,7 @@ __global__ void __launch_bounds__(64) smooth_forward_kernel(const ApGradView v, 
                 --until_ck;
                 ++k;
             }
-            while (!done && until_ck >= kBlock && k + kBlock <= v.max_iter) {
+            while (!done && until_ck >= kBlock && v.max_iter - k >= kBlock) {
                 const C2d before = z;
 #pragma unroll
                 for (int t = 0; t < kBlock; ++t) step_f<FT>(v, z, c, z, d);
@@ -151,7 +151,7 @@ __global__ void __launch_bounds__(64) smooth_forward_kernel(const ApGradView v, 
                 until_ck -= kBlock;
                 if (z.r == kept.r && z.i == kept.i) {  // repeats: never escapes
                     const int turn = k - kept_k;
-                    for (; ckpt && slot < n_ck && k + until_ck < v.max_iter; ++slot) {
+                    for (; ckpt && slot < n_ck && until_ck < v.max_iter - k; ++slot) {
                         for (int t = until_ck % turn; t > 0; --t) step_f<FT>(v, z, c, z, d);
                         k += until_ck;
                         until_ck = v.ckpt_every;

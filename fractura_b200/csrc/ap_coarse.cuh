@@ -541,7 +541,7 @@ __device__ __forceinline__ void stage2_advance(const ApFrameParams& p, PixelRun&
             break;
         }
         // blocks tested at their end only, as in direct iteration (fp64_orbit, ap_fp64.cuh)
-        if (growing && tested == 0 && k + kBlock <= max_iter) {
+        if (growing && tested == 0 && max_iter - k >= kBlock) {
             const double bx = zx, by = zy;
             for_degree(kKind, p.gen_n, doubles, [&](auto n) {
 #pragma unroll

@@ -161,7 +161,7 @@ __device__ __forceinline__ int fp64_orbit(double zx, double zy, double cx, doubl
         const bool doubles = ARITH != AP_ARITH_REF_CPU && fp64_doubles(zy, cy);
         double sx = zx, sy = zy;  // the z that block ends are compared with
         int left = 1, window = 1;
-        while (k + kBlock <= max_iter) {
+        while (max_iter - k >= kBlock) {
             const double bx = zx, by = zy;
             auto block = [&](auto form) {
 #pragma unroll
