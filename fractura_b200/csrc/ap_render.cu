@@ -8,6 +8,7 @@
 
 #include "ap_common.cuh"
 #include "ap_fp64.cuh"
+#include "ap_samples.cuh"
 #include "ap_tiers.cuh"
 
 namespace ap {
@@ -116,18 +117,19 @@ __global__ void __launch_bounds__(32) supersample_kernel(const ApFrameParams p, 
     if (lane == 0) palette = palette_of(p, hist_colour);
     __syncwarp();
     const bool write_iter = hist_resolve ? (p.rebase_pass > 0) : ((p.flags & AP_FLAG_ITER_LAST_SUB) != 0);
-    const int f = p.factor, f2 = f * f;
+    const int f = p.factor;
+    const long long f2 = (long long)f * f, total = count * f2;
     double ra = 0.0, ga = 0.0, ba = 0.0;
     int glitches = 0, iters = 0, leaps = 0, iters2 = 0;
-    const int lo = lane * f2, hi = lo + f2;  // the owned pixel's samples
-    for (int base = 0; base < count * f2; base += 32) {
-        const int q = base + lane;
-        if (q < count * f2) {
-            const int at = list[q / f2];
+    const long long lo = lane * f2, hi = lo + f2;  // the owned pixel's samples
+    for (long long base = 0; base < total; base += 32) {
+        if (base + lane < total) {
+            int pixel, sx, sy;
+            sample_place(base + lane, f, &pixel, &sx, &sy);
+            const int at = list[pixel];
             i = i0 + (at & 7);
             j = j0 + (at >> 3);
-            const int sub = q % f2;
-            const SampleOut o = sample_at<TIER, ARITH, KIND>(p, b, (double)(i * f + sub % f), (double)(j * f + sub / f));
+            const SampleOut o = sample_at<TIER, ARITH, KIND>(p, b, (double)(i * f + sx), (double)(j * f + sy));
             double r = 0.0, g = 0.0, bb = 0.0;
             if ((double)o.s >= 0.0) colour_of(p, palette, b.lut, b.cdf, hist_colour, (double)o.s, r, g, bb);
             red[lane] = r;
@@ -137,7 +139,7 @@ __global__ void __launch_bounds__(32) supersample_kernel(const ApFrameParams p, 
             work[lane][1] = o.leaps;
             work[lane][2] = o.iters2;
             work[lane][3] = o.glitch;
-            if (write_iter && sub == f2 - 1) {
+            if (write_iter && sx == f - 1 && sy == f - 1) {
                 const size_t idx = (size_t)j * p.width + i;
                 b.iter_map[idx] = o.s;
                 if (b.kmap) b.kmap[idx] = o.k;
@@ -146,14 +148,15 @@ __global__ void __launch_bounds__(32) supersample_kernel(const ApFrameParams p, 
         }
         __syncwarp();
         if (lane < count) {
-            for (int t = max(lo, base); t < min(hi, base + 32); ++t) {
-                ra += red[t - base];
-                ga += green[t - base];
-                ba += blue[t - base];
-                iters += work[t - base][0];
-                leaps += work[t - base][1];
-                iters2 += work[t - base][2];
-                glitches += work[t - base][3] > 0 ? 1 : 0;
+            const int from = (int)(max(lo, base) - base), to = (int)(min(hi, base + 32) - base);
+            for (int t = from; t < to; ++t) {
+                ra += red[t];
+                ga += green[t];
+                ba += blue[t];
+                iters += work[t][0];
+                leaps += work[t][1];
+                iters2 += work[t][2];
+                glitches += work[t][3] > 0 ? 1 : 0;
             }
         }
         __syncwarp();
