@@ -117,55 +117,58 @@ __global__ void __launch_bounds__(32) supersample_kernel(const ApFrameParams p, 
     if (lane == 0) palette = palette_of(p, hist_colour);
     __syncwarp();
     const bool write_iter = hist_resolve ? (p.rebase_pass > 0) : ((p.flags & AP_FLAG_ITER_LAST_SUB) != 0);
-    const int f = p.factor;
-    const long long f2 = (long long)f * f, total = count * f2;
+    const int f = p.factor, rows = count * f;
     double ra = 0.0, ga = 0.0, ba = 0.0;
     int glitches = 0, iters = 0, leaps = 0, iters2 = 0;
-    const long long lo = lane * f2, hi = lo + f2;  // the owned pixel's samples
-    for (long long base = 0; base < total; base += 32) {
-        if (base + lane < total) {
-            int pixel, sx, sy;
-            sample_place(base + lane, f, &pixel, &sx, &sy);
-            const int at = list[pixel];
-            i = i0 + (at & 7);
-            j = j0 + (at >> 3);
-            const SampleOut o = sample_at<TIER, ARITH, KIND>(p, b, (double)(i * f + sx), (double)(j * f + sy));
-            double r = 0.0, g = 0.0, bb = 0.0;
-            if ((double)o.s >= 0.0) colour_of(p, palette, b.lut, b.cdf, hist_colour, (double)o.s, r, g, bb);
-            red[lane] = r;
-            green[lane] = g;
-            blue[lane] = bb;
-            work[lane][0] = o.iters;
-            work[lane][1] = o.leaps;
-            work[lane][2] = o.iters2;
-            work[lane][3] = o.glitch;
-            if (write_iter && sx == f - 1 && sy == f - 1) {
-                const size_t idx = (size_t)j * p.width + i;
-                b.iter_map[idx] = o.s;
-                if (b.kmap) b.kmap[idx] = o.k;
-                if (b.s64) b.s64[idx] = o.s64;
+    for (int row0 = 0; row0 < rows; row0 += sample_rows(f)) {
+        const int part = min(sample_rows(f), rows - row0), total = part * f;
+        // the owned pixel's samples of this part
+        const int lo = min(max(lane * f - row0, 0), part) * f, hi = min(max(lane * f + f - row0, 0), part) * f;
+        for (int base = 0; base < total; base += 32) {
+            const int q = base + lane;
+            if (q < total) {
+                int pixel, sx, sy;
+                sample_place(row0, q, f, &pixel, &sx, &sy);
+                const int at = list[pixel];
+                i = i0 + (at & 7);
+                j = j0 + (at >> 3);
+                const SampleOut o = sample_at<TIER, ARITH, KIND>(p, b, (double)(i * f + sx), (double)(j * f + sy));
+                double r = 0.0, g = 0.0, bb = 0.0;
+                if ((double)o.s >= 0.0) colour_of(p, palette, b.lut, b.cdf, hist_colour, (double)o.s, r, g, bb);
+                red[lane] = r;
+                green[lane] = g;
+                blue[lane] = bb;
+                work[lane][0] = o.iters;
+                work[lane][1] = o.leaps;
+                work[lane][2] = o.iters2;
+                work[lane][3] = o.glitch;
+                if (write_iter && sx == f - 1 && sy == f - 1) {
+                    const size_t idx = (size_t)j * p.width + i;
+                    b.iter_map[idx] = o.s;
+                    if (b.kmap) b.kmap[idx] = o.k;
+                    if (b.s64) b.s64[idx] = o.s64;
+                }
             }
-        }
-        __syncwarp();
-        if (lane < count) {
-            const int from = (int)(max(lo, base) - base), to = (int)(min(hi, base + 32) - base);
-            for (int t = from; t < to; ++t) {
-                ra += red[t];
-                ga += green[t];
-                ba += blue[t];
-                iters += work[t][0];
-                leaps += work[t][1];
-                iters2 += work[t][2];
-                glitches += work[t][3] > 0 ? 1 : 0;
+            __syncwarp();
+            if (lane < count) {
+                for (int t = max(lo, base); t < min(hi, base + 32); ++t) {
+                    ra += red[t - base];
+                    ga += green[t - base];
+                    ba += blue[t - base];
+                    iters += work[t - base][0];
+                    leaps += work[t - base][1];
+                    iters2 += work[t - base][2];
+                    glitches += work[t - base][3] > 0 ? 1 : 0;
+                }
             }
+            __syncwarp();
         }
-        __syncwarp();
     }
     if (lane < count) {
         i = i0 + (list[lane] & 7);
         j = j0 + (list[lane] >> 3);
         const size_t idx = (size_t)j * p.width + i;
-        const double inv = 1.0 / (double)f2;
+        const double inv = 1.0 / ((double)f * f);
         store_rgb(b.rgb, p.is_hdr, idx, ra * inv, ga * inv, ba * inv);
         if (kPert && b.glitch_out) b.glitch_out[idx] = glitches > 0 ? 1 : 0;
         if (b.counters) reinterpret_cast<int4*>(b.counters)[idx] = make_int4(iters, leaps, iters2, 0);

@@ -11,20 +11,18 @@
 
 namespace ap {
 
-// Sample q of pixels of f x f samples each, pixel after pixel, row after row -> its pixel and its place
-// (sx, sy) there.  64 bits where the number of a sample needs them: 32 pixels at f = 8192 have 2^31.
-AP_HOST_DEVICE void sample_place(int64_t q, int f, int* pixel, int* sx, int* sy) {
-    if (q < INT32_MAX && f <= 46340) {  // f^2 < 2^31
-        const unsigned f2 = (unsigned)f * (unsigned)f, sub = (unsigned)q % f2;
-        *pixel = (int)((unsigned)q / f2);
-        *sx = (int)(sub % (unsigned)f);
-        *sy = (int)(sub / (unsigned)f);
-    } else {
-        const int64_t f2 = (int64_t)f * f, sub = q % f2;
-        *pixel = (int)(q / f2);
-        *sx = (int)(sub % f);
-        *sy = (int)(sub / f);
-    }
+// The samples of pixels of f x f each, pixel after pixel and row after row, run in parts of whole rows whose
+// samples 31 bits number (f is below 2^25): 32 pixels at f = 8192 have 2^31 of them.
+AP_HOST_DEVICE int sample_rows(int f) {  // rows of a part
+    return (1 << 30) / f;
+}
+
+// Sample q of the part that starts at row `row0` -> its pixel and its place (sx, sy) there.
+AP_HOST_DEVICE void sample_place(int row0, int q, int f, int* pixel, int* sx, int* sy) {
+    const int row = row0 + (int)((unsigned)q / (unsigned)f);
+    *sx = (int)((unsigned)q % (unsigned)f);
+    *pixel = (int)((unsigned)row / (unsigned)f);
+    *sy = (int)((unsigned)row % (unsigned)f);
 }
 
 }  // namespace ap
