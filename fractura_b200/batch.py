@@ -62,7 +62,8 @@ class BatchConfig:
     """Launch shape of the persistent kernel: patch_w x patch_h = 256 pixels per work
     item, blocks_per_sm resident blocks of 512 threads, min_blocks = the register
     budget (4: 64 registers, 6: 42), quantum = length of a round, the time between two
-    compactions of a block's pixels (in units that grow with the pixels per thread)."""
+    compactions of a block's pixels: loop steps up to 16, above in units of 512 to 4096 clock
+    cycles that grow with the pixels per thread."""
     patch_w: int = 16
     patch_h: int = 16
     blocks_per_sm: int = 2

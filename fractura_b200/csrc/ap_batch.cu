@@ -120,7 +120,7 @@ __device__ __forceinline__ void slot_store_run(BatchSlots& S, int q, const Pixel
     S.tag[q] = (S.tag[q] & ~7) | (s.stage << 1) | (s.glitch ? 1 : 0);
 }
 
-// One round of the pixel in slot q (of tile t): loop steps up to the quantum; the
+// One round of the pixel in slot q (of tile t), until `round` is over; the
 // pixel is written out when it finishes.  Returns true when it has not finished; its
 // state is then back in slot q.  One variant per (profile, formula class, BLA,
 // rebasing): separate functions, so each keeps the register allocation it has in the
@@ -331,7 +331,7 @@ __device__ __forceinline__ int batch_class(const ApTileDesc* t) {
 }
 constexpr int kBatchClasses = 6;
 
-// Clock cycles of a round per unit of its length (`quantum`).  A short round gives the lanes of
+// Clock cycles of a round per unit of its length (`quantum`, above kRoundCheck).  A short round gives the lanes of
 // finished pixels new ones soon, a long one spends less on waiting and compacting: 512 where the
 // batch has no more than two pixels a slot, 4096 where it has sixteen (21 mixed tiles, 20 a slot:
 // 512 32.6 ms, 1024 31.5, 2048 30.2, 4096 29.2, 8192 29.6, 16384 34.6; single tiles of one or two
@@ -354,8 +354,9 @@ __global__ void __launch_bounds__(kBatchThreads, MINB * 256 / kBatchThreads) bat
     const unsigned full = 0xffffffffu;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const long long total = first[n] * 256;
-    // half the clock's range at most, so that its wrap-around is told apart
-    const unsigned span = (unsigned)min((long long)quantum * round_cycles(total), 1ll << 30);
+    // half the clock's range at most, so that its wrap-around is told apart; a short quantum is a number
+    // of loop steps (the clock is looked at after them and has passed)
+    const unsigned span = quantum <= kRoundCheck ? 0u : (unsigned)min((long long)quantum * round_cycles(total), 1ll << 30);
     if (tid == 0) {
         live_s = 0;
         drained_s = 0;

@@ -128,7 +128,9 @@ typedef struct ApFrameBuffers {
     int32_t* counters;         /* optional [H, W, 4]: work done for the pixel by this pass, summed
                                   over its sub-samples: [0] iterations stepped one at a time
                                   (direct tiers; perturbation stage 1; those of an orbit found to
-                                  repeat for ever are not run and not counted), [1] BLA leaps taken,
+                                  repeat for ever are not run and not counted; where a batch in
+                                  rounds of clock cycles notices it depends on the rounds, so
+                                  those pixels' counts vary from run to run), [1] BLA leaps taken,
                                   [2] perturbation stage-2 (direct) steps, [3] rebases
                                   (AP_FLAG_REBASE coarse passes on packed inputs; otherwise zero).  16-byte aligned;
                                   written only for pixels the pass evaluates. */
@@ -412,8 +414,8 @@ AP_API int ap_decimal_arith(int32_t op, const int64_t* a_meta, const uint64_t* a
  * tiles should come in decreasing order of expected cost.
  * ap_render_batch: renders all tiles with one persistent kernel of blocks_per_sm blocks per
  * SM that take pixels from a shared counter (device word *queue_head, reset here).  A block
- * works in rounds of a length that `quantum` scales (at least that many loop steps, up to 16, and
- * quantum x 512 to 4096 clock cycles, more with more pixels a thread): each thread runs one pixel;
+ * works in rounds: of `quantum` loop steps up to 16, and of quantum x 512 to 4096 clock cycles above
+ * (more with more pixels a thread): each thread runs one pixel;
  * the unfinished pixels are compacted into the block's first slots (shared memory) and the slots left
  * over take the next consecutive pixels of the queue with one atomicAdd.
  * tiles and first_patch are device copies of the planned arrays.  min_blocks (4 or 6) picks
