@@ -105,9 +105,13 @@ struct PlainRange {
         high = min(high, min(hx - 1u, hy - 1u));  // 0 counts as the largest
         low = min(low, min(lx - 1u, ly - 1u));
     }
+    static constexpr unsigned k181 = 0x4066a000u, kHigh = (1023u - 200u) << 20, kLow = (1023u - 700u) << 20;
     __device__ __forceinline__ bool plain() const {
-        constexpr unsigned k181 = 0x4066a000u, kHigh = (1023u - 200u) << 20, kLow = (1023u - 700u) << 20;
         return (top < k181) & (high >= kHigh - 1u) & (low >= kLow - 1u);
+    }
+    // the same without 181, for a step whose |z|^2 is tested
+    __device__ __forceinline__ bool finite() const {
+        return (top < (1023u + 400u) << 20) & (high >= kHigh - 1u) & (low >= kLow - 1u);
     }
 };
 
@@ -122,9 +126,10 @@ __device__ __forceinline__ void dd_step_general(dd& zx, dd& zy, dd zx2, dd zy2, 
     zy = SHIP ? dd_sub(two, cy) : dd_add(two, cy);
 }
 
-// The same for normalised operands in PlainRange (see dd_quad_orbit).
+// The same for normalised operands in PlainRange (see dd_quad_orbit).  Returns |z|^2 as the general
+// step's test forms it.
 template <bool SHIP>
-__device__ __forceinline__ void dd_step_plain(dd& zx, dd& zy, dd cx, dd cy) {
+__device__ __forceinline__ double dd_step_plain(dd& zx, dd& zy, dd cx, dd cy) {
     const double x2 = zx.hi + zx.hi, y2 = zy.hi + zy.hi;
     double p = zx.hi * zx.hi;
     const dd zx2 = quick_sum(p, fma(zx.hi, zx.hi, -p) + x2 * zx.lo);
@@ -142,6 +147,7 @@ __device__ __forceinline__ void dd_step_plain(dd& zx, dd& zy, dd cx, dd cy) {
     } else {
         zy = add_normalised(zxy, cy);
     }
+    return zx2.hi + zy2.hi;
 }
 
 // The orbit of z under z^2 + c (SHIP: Burning Ship), bit for bit (but for the signs of zeros, which
@@ -153,24 +159,43 @@ __device__ __forceinline__ void dd_step_plain(dd& zx, dd& zy, dd cx, dd cy) {
 //     (add_normalised; a product's correction is below 2^-50 of it): 3 operations for 6;
 //   * 2 z_x and 2 z_y are formed once for the squares' cross terms and for 2 z_x z_y
 //     (scaling by 2 commutes with every rounding that does not underflow);
-//   * while both high parts are below 181 the orbit cannot have passed the bailout, so |z|^2
-//     is formed only beside the general step, which a z takes that is near the bailout or has a
-//     high part below 2^-200 or a low part below 2^-700 (not 0), where a product could underflow.
-// The steps run in blocks whose tests are gathered into three words; where they fail, the block is
-// taken again from its start by general steps, which the lanes of a warp do together.  With a test
-// and a branch a step on all four parts of z, the chain of a lone warp waited for each: a frame that
-// leaves most of the GPU idle is bound by it (128x96 Mandelbrot at 1e-18, depth 8500, REF_CUDA: 1559 us
-// with a test a step, 1230 with blocks and a flag, 1117 with the three words; 1217 before the short
+//   * while both high parts are below 181 the orbit cannot have passed the bailout, so |z|^2 goes
+//     unformed in the blocks.  A z with a high part below 2^-200 or a low part below 2^-700 (not 0),
+//     where a product could underflow, takes the general step.
+// The first kDdLead steps are tested one by one: a shallow frame, whose pixels escape there, is bound by
+// the FP64 pipe and would run up to two blocks for nothing (1280x720 Burning Ship at 1e-20, whose pixels
+// escape after 26 steps: a frame 289 us with blocks from the first step on, 265 so).
+// Then the steps run in blocks whose tests are gathered into three words; where they fail, the block is
+// taken again from its start by tested steps, which the lanes of a warp do together.  With a test
+// and a branch a step throughout, the chain of a lone warp waited for all four parts of z: a deep frame
+// that leaves most of the GPU idle is bound by it (128x96 Mandelbrot at 1e-18, depth 8500, REF_CUDA:
+// 1559 us with a test a step, 1230 with blocks and a flag, 1117 with the three words; 1217 before the short
 // step), a large one by the FP64 pipe (960x540 20.1 -> 15.5 ms, 16.2 with a test a step; 960x540
 // Burning Ship at 2e-17, depth 6000, REF_CPU 13.1 -> 7.2 ms, 7.5 with a test a step).  Blocks of 4, 8 and
-// 16 steps: 128x96 1117, 1117 and 1093 us; 599x400 Burning Ship at depth 6000 4246, 3954 and 3981;
-// 128x96 Mandelbrot set at depth 500 161, 163 and 166.
-constexpr int kDdBlock = 8;
+// 16 steps: 128x96 1117, 1117 and 1093 us; 599x400 Burning Ship at depth 6000 4246, 3954 and 3981.
+constexpr int kDdBlock = 8, kDdLead = 32;
 // Returns the escape step, or -1.
 template <int ARITH, bool SHIP>
 __device__ __forceinline__ int dd_quad_orbit(dd zx, dd zy, const dd cx, const dd cy, int max_iter,
                                              bool normalised, double& mag2_out) {
-    for (int k = 0; k < max_iter;) {
+    int tested = kDdLead;
+    for (int k = 0; k < max_iter; tested = kDdBlock) {
+        for (const int stop = k + min(tested, max_iter - k); k < stop; ++k) {
+            PlainRange range;
+            range.add(zx, zy);
+            double mag2;
+            if (normalised && range.finite()) {
+                mag2 = dd_step_plain<SHIP>(zx, zy, cx, cy);
+            } else {
+                const dd zx2 = dd_sqr<ARITH>(zx), zy2 = dd_sqr<ARITH>(zy);
+                mag2 = zx2.hi + zy2.hi;
+                dd_step_general<ARITH, SHIP>(zx, zy, zx2, zy2, cx, cy);
+            }
+            if (mag2 > kBailout) {
+                mag2_out = mag2;
+                return k;
+            }
+        }
         while (normalised && max_iter - k >= kDdBlock) {
             const dd bx = zx, by = zy;
             PlainRange range;
@@ -185,15 +210,6 @@ __device__ __forceinline__ int dd_quad_orbit(dd zx, dd zy, const dd cx, const dd
                 break;
             }
             k += kDdBlock;
-        }
-        for (const int stop = normalised ? k + min(kDdBlock, max_iter - k) : max_iter; k < stop; ++k) {
-            const dd zx2 = dd_sqr<ARITH>(zx), zy2 = dd_sqr<ARITH>(zy);
-            const double mag2 = zx2.hi + zy2.hi;
-            if (mag2 > kBailout) {
-                mag2_out = mag2;
-                return k;
-            }
-            dd_step_general<ARITH, SHIP>(zx, zy, zx2, zy2, cx, cy);
         }
     }
     return -1;

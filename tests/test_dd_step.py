@@ -82,12 +82,12 @@ def test_device_equals_oracle_where_the_step_changes_path(case, ft, arith):
     assert np.array_equal(it.cpu().numpy().view(np.uint32), fr.iter_map.view(np.uint32))
 
 
-def plain_range(parts):
+def plain_range(parts, top=0x4066a000):
     """PlainRange of ap_dd.cuh on columns (x.hi, y.hi, x.lo, y.lo): high words, unsigned."""
     h = [(p.view(np.uint64) >> np.uint64(32)).astype(np.uint32) & np.uint32(0x7fffffff) for p in parts]
     high = np.minimum(h[0] - np.uint32(1), h[1] - np.uint32(1))
     low = np.minimum(h[2] - np.uint32(1), h[3] - np.uint32(1))
-    return ((np.maximum(h[0], h[1]) < 0x4066a000) & (high >= ((1023 - 200) << 20) - 1) & (low >= ((1023 - 700) << 20) - 1))
+    return ((np.maximum(h[0], h[1]) < top) & (high >= ((1023 - 200) << 20) - 1) & (low >= ((1023 - 700) << 20) - 1))
 
 
 def test_range_words_are_the_ranges_they_stand_for():
@@ -106,12 +106,23 @@ def test_range_words_are_the_ranges_they_stand_for():
         for q in (2, 3):
             want &= (a[q] == 0.0) | (a[q] >= 2.0 ** -700) | np.isnan(a[q])  # a NaN low part has a NaN high one
     assert np.array_equal(plain_range(grid), want)
+    with np.errstate(invalid="ignore"):  # finite(): up to 2^400
+        for q in (0, 1):
+            grid[q][a[q] == 1e300] = 2.0 ** 400
+            grid[q][a[q] == 256.0] = np.nextafter(2.0 ** 400, 0)
+        a = np.abs(np.array(grid))
+        want = np.ones(a.shape[1], bool)
+        for q in (0, 1):
+            want &= (a[q] < 2.0 ** 400) & ((a[q] == 0.0) | (a[q] >= 2.0 ** -200))
+        for q in (2, 3):
+            want &= (a[q] == 0.0) | (a[q] >= 2.0 ** -700) | np.isnan(a[q])
+    assert np.array_equal(plain_range(grid, (1023 + 400) << 20), want)
 
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("arith", [abi.AP_ARITH_REF_CPU, abi.AP_ARITH_REF_CUDA])
 @pytest.mark.parametrize("ft", [0, 1, 2])
-@pytest.mark.parametrize("max_iter", [0, 1, 7, 8, 9, 16, 17, 40, 203])
+@pytest.mark.parametrize("max_iter", [0, 1, 31, 32, 33, 39, 40, 41, 48, 203])
 def test_depths_that_end_anywhere_in_a_block(max_iter, ft, arith):
     """The whole sets (escapes at every place of a block, a zero row, bounded pixels)."""
     import oracle
