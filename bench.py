@@ -25,9 +25,9 @@ Rank 0 prints one JSON line:
             per form: G iter/s and the smooth error / escape-step agreement against the
             700-bit ground truth (tests/golden/truth_cfg3.npz); the plain form is the
             reference's (FP64 deltas, no BLA, Pauldelbrot with up to 4 rebase passes);
-  roofline  FP64 pipe of the render passes: executed FP64 operations (from the kernels'
-            work counters) / their event-timed duration, against the dependent-FMA FP64
-            peak measured in the same run;
+  roofline  FP64 pipe of the render passes: nominal FP64 operations (per step and leap of
+            the kernels' work counters) / their event-timed duration, against the
+            dependent-FMA FP64 peak measured in the same run;
   cpu_baseline  the reference's CPU path restated in C (oracle/), all host cores, full
             frames in the reference's own form (Pauldelbrot, its BLA table, orbits from
             oracle/ref_orbit.py);
@@ -59,7 +59,9 @@ import numpy as np
 ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, ROOT)
 
-# Executed FP64 operations of the perturbation loop (reference-CPU arithmetic, no fused ops):
+# Nominal FP64 operations of the perturbation loop (reference-CPU arithmetic, no fused ops), per step and
+# leap that the work counters count.  The kernels run fewer: a step inside its safe radius forms no
+# z or |z|^2, one of a span no |dz|^2 either (13), a direct step of a block no |z|^2 (5).
 #   stage-1 step: z = Z + dz (2), |z|^2 (3), Pauldelbrot test (4), BLA radius test (3),
 #                 dz' = (2Z + dz) dz + dc (13)                                        -> 25
 #   BLA leap:     z, |z|^2 (5), Pauldelbrot test (4), radius test (3), A dz + B dc (14) -> 26
@@ -81,21 +83,70 @@ FLOPS_STEP1_FEXP = 35.0
 FLOPS_STEP_REBASE = 21.0
 FLOPS_LEAP_REBASE = 22.0
 # Derivatives of the smooth value (csrc/ap_adjoint.cu), per iteration of a pixel's orbit:
-#   forward:  |z|^2 (3) + f(z) and f'(z): z^2 + c (8) and 2z (2)                       -> 13
-#             Multibrot n: z^(n-1) (6 (n-1)), z^n and P z (12), sums (4), f' (4), |z|^2 (3)
-#   adjoint:  the step and f' once more (10; Multibrot 6 (n-1) + 20), the derivatives with respect
-#             to the pixel and the parameter beside it (a fused complex multiply-add each: 6 and 8;
-#             Multibrot 8 and 8)                                                     -> 24
-FLOPS_FWD_QUAD = 13.0
+#   forward:  z^2 + c                                                                  -> 8
+#             Multibrot n: z^n and P z (6 n + 6; 18 for n = 3, which forms z^2 first), sums (4)
+#   adjoint:  the step and f' once more (10; Multibrot 4 more than the step), the derivatives with
+#             respect to the pixel and the parameter beside it (a fused complex multiply-add each:
+#             6 and 8; Multibrot 8 and 8)                                            -> 24
+FLOPS_FWD_QUAD = 8.0
 FLOPS_ADJ_QUAD = 24.0
 
 
 def flops_fwd_multi(n):
-    return 6.0 * (n - 1) + 23.0
+    return 22.0 if n == 3 else 6.0 * n + 10.0
 
 
 def flops_adj_multi(n):
-    return 6.0 * (n - 1) + 36.0
+    return flops_fwd_multi(n) + 20.0
+
+
+def forward_steps(torch, th, W, H, max_iter, fractal_type, gen_n, kmap):
+    """Steps that the derivatives' forward pass runs (smooth_forward_kernel's rule replayed): up to its escape for a
+    pixel that escapes, up to the block whose end repeats an earlier one for one that settles on a cycle."""
+    w, dev = math.exp(th[2]), kmap.device
+    h = w * H / W
+    x = (th[0] - 0.5 * w) + torch.arange(W, dtype=torch.float64, device=dev) * (w / max(1, W - 1))
+    y = (th[1] + 0.5 * h) - torch.arange(H, dtype=torch.float64, device=dev) * (h / max(1, H - 1))
+    px, py = x.expand(H, W).reshape(-1), y.reshape(H, 1).expand(H, W).reshape(-1)
+    bounded = (kmap.reshape(-1) == -1)
+    px, py = px[bounded], py[bounded]
+    if fractal_type == 2:
+        zx, zy, cx, cy = px, py, th[3], th[4]
+    else:
+        zx, zy, cx, cy = torch.zeros_like(px), torch.zeros_like(py), px, py
+    ran = torch.full_like(px, float(max_iter))
+    live = torch.ones_like(px, dtype=torch.bool)
+    kx, ky, left, window, tested, to_ckpt, block = zx, zy, 1, 1, 8, 0, 0
+    for k in range(max_iter):
+        if to_ckpt == 0:
+            to_ckpt = 1024
+        if fractal_type == 4:
+            rx, ry = zx, zy
+            for _ in range(gen_n - 1):
+                rx, ry = rx * zx - ry * zy, rx * zy + ry * zx
+            zx, zy = rx + (th[3] * zx - th[4] * zy) + cx, ry + (th[3] * zy + th[4] * zx) + cy
+        else:
+            zx, zy = zx * zx - zy * zy + cx, 2.0 * zx * zy + cy
+        to_ckpt -= 1
+        if block == 0:
+            tested -= 1
+        else:
+            block -= 1
+            if block == 0:
+                hit = live & (zx == kx) & (zy == ky)
+                ran[hit] = float(k + 1)
+                live &= ~hit
+                left -= 1
+                if left == 0:
+                    kx, ky, window = zx, zy, 2 * window
+                    left = window
+        if block == 0 and tested == 0:
+            if to_ckpt >= 16 and max_iter - (k + 1) >= 16:
+                block = 16
+            else:
+                tested = min(16, to_ckpt) + 1
+    k = kmap.reshape(-1)
+    return float(k[k > 0].sum(dtype=torch.float64) + ran.sum())
 
 
 L2_FLUSH = "flushed between timed steps (512 MiB write)"
@@ -167,8 +218,8 @@ def workload_cfg5():
                 max_iter=2000, width="3.0", dtype="f64", arith="ref_cuda", seed=20250,
                 cases=[dict(fractal_type=2, gen_n=2, theta=[0.0, 0.0, math.log(3.0), -0.8, 0.156]),
                        dict(fractal_type=4, gen_n=3, theta=[0.0, 0.0, math.log(3.0), 0.1, 0.2])],
-                form="FP64 forward with orbit checkpoints every 1024 steps, then the adjoint sweep "
-                     "(segments recomputed from checkpoints) for d loss / d(cx, cy, ln w, Re P, Im P); "
+                form="FP64 forward, then the adjoint (the orbit recomputed once, its derivatives with respect "
+                     "to the pixel and P beside it) for d loss / d(cx, cy, ln w, Re P, Im P); "
                      "Julia j=-0.8+0.156i and Multibrot n=3, k=0.1+0.2i; loss = mean squared "
                      "difference to a target at theta + N(0, 1e-3)")
 
@@ -577,7 +628,7 @@ def timed_replay(torch, _lib, ops, stream, steps, flush, record_pass=False):
 
 
 def pass_flops(torch, _lib, abi, ops, stream, H, W, strict, has_bla, direct_flops=FLOPS_DIRECT):
-    """Executed FP64 operations of every render pass in one replay, from the work counters."""
+    """Nominal FP64 operations of every render pass in one replay, from the work counters."""
     counters = torch.zeros((H, W, 4), dtype=torch.int32, device="cuda")
     f1 = 18.0 + (4.0 if strict else 0.0) + (3.0 if has_bla else 0.0)
     total = 0.0
@@ -835,7 +886,7 @@ def step_flops(fractal_type, gen_n, strict, bla, rebase=False):
 
 
 def batch_flops(torch, _lib, b, cfg):
-    """Executed FP64 operations of one batch render, from the kernel's work counters
+    """Nominal FP64 operations of one batch render, from the kernel's work counters
     (a counter-carrying copy of the descriptors, rendered once outside the timed region)."""
     from fractura_b200 import abi
     counters = []
@@ -972,9 +1023,9 @@ def batch_arm(args, wl, rank, world, local_rank, steps, headline):
 
 # ------------------------------------------------------------ adjoint arm
 def adjoint_arm(args, wl, rank, world, local_rank, steps, headline):
-    """Config 5: per step, for Julia and Multibrot n=3, the forward pass with checkpoints,
-    the loss gradient dL/ds on the device and the adjoint sweep (the autograd backward);
-    value = forward orbit iterations per second (each iteration is also swept backwards)."""
+    """Config 5: per step, for Julia and Multibrot n=3, the forward pass, the loss gradient dL/ds on the device and the
+    adjoint (the autograd backward); value = nominal orbit iterations per second (max_iter for a pixel that never
+    escapes, which the forward pass leaves at its cycle and the adjoint skips)."""
     import torch
     from fractura_b200 import _lib
     from fractura_b200 import adjoint as adj
@@ -1018,16 +1069,17 @@ def adjoint_arm(args, wl, rank, world, local_rank, steps, headline):
     stream.synchronize()
     fwd_ms = sum(e[0].elapsed_time(e[1]) for e in evs)
     adj_ms = sum(e[1].elapsed_time(e[2]) for e in evs)
-    iters = fwd_flops = adj_flops = 0.0
-    for (case, _, _), (_, k) in zip(cases, res):
-        it = nominal_iterations(k.cpu().numpy(), mi)
-        iters += it
-        if case["fractal_type"] == 4:
-            fwd_flops += flops_fwd_multi(case["gen_n"]) * it
-            adj_flops += flops_adj_multi(case["gen_n"]) * it
-        else:
-            fwd_flops += FLOPS_FWD_QUAD * it
-            adj_flops += FLOPS_ADJ_QUAD * it
+    # operations of the steps that the kernels run: the adjoint's are those of the pixels that escape in both images
+    iters = fwd_flops = adj_flops = fwd_steps = adj_steps = 0.0
+    for (case, th, tgt), (_, k) in zip(cases, res):
+        iters += nominal_iterations(k.cpu().numpy(), mi)
+        fs = forward_steps(torch, th, W, H, mi, case["fractal_type"], case["gen_n"], k)
+        ks = k[(k > 0) & (tgt >= 0)].sum(dtype=torch.float64).item()
+        fwd_steps += fs
+        adj_steps += ks
+        multi = case["fractal_type"] == 4
+        fwd_flops += (flops_fwd_multi(case["gen_n"]) if multi else FLOPS_FWD_QUAD) * fs
+        adj_flops += (flops_adj_multi(case["gen_n"]) if multi else FLOPS_ADJ_QUAD) * ks
 
     barrier(world)
     c0 = L.ap_launch_counter()
@@ -1079,12 +1131,13 @@ def adjoint_arm(args, wl, rank, world, local_rank, steps, headline):
         "config": config_of(wl, world), "form": wl["form"],
         "nominal_iterations_per_step": iters,
         "kernel_ms": {"forward": fwd_ms, "adjoint": adj_ms},
+        "steps_run": {"forward": fwd_steps, "adjoint": adj_steps},
         "flops_per_step": {"forward": fwd_flops, "adjoint": adj_flops,
                            "per_iteration": {"forward_quadratic": FLOPS_FWD_QUAD,
                                              "adjoint_quadratic": FLOPS_ADJ_QUAD,
                                              "forward_multibrot3": flops_fwd_multi(3),
                                              "adjoint_multibrot3": flops_adj_multi(3)}},
-        "roofline": {"bound": "fp64", "kernel": "smooth_adjoint_kernel (the larger of the two)",
+        "roofline": {"bound": "fp64", "kernel": "smooth_adjoint_kernel (its time is that of its longest orbits' chains)",
                      "achieved": achieved, "peak": peak64, "unit": "TFLOP/s",
                      "frac": achieved / peak64 if peak64 else None,
                      "forward_frac": (fwd_flops / (fwd_ms * 1e-3) / 1e12) / peak64 if peak64 else None,
