@@ -9,9 +9,11 @@ theta is a float64 tensor (cx, cy, ln w, Re P, Im P); P is the Julia parameter
 (fractal_type 4); Mandelbrot (0) has no P.  The forward pass is FP64 direct
 iteration on the GPU (ap_smooth_forward), which also keeps the orbit every
 CKPT_EVERY steps; the backward pass is the hand-written adjoint
-(ap_smooth_adjoint), which recomputes the orbit instead of
-storing it.  forward_mode() gives the same derivatives per pixel by
-forward-mode tangents (ap_smooth_tangent), the independent check.
+(ap_smooth_adjoint), which recomputes the orbit with its derivatives instead of
+storing it (ap_smooth_adjoint takes the kept steps, and reads none of them).
+forward_mode() gives the derivatives per pixel by forward-mode tangents
+(ap_smooth_tangent), one real parameter at a time; the check that shares no
+recurrence with either is by finite differences.
 """
 import ctypes as C
 

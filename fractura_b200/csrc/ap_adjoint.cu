@@ -15,7 +15,7 @@
 //     product dL/dtheta of the whole orbit, recomputed (no orbit is stored); one row of
 //     sums per warp of 8 x 4 pixels (deterministic, summed by the caller);
 //   ap_smooth_tangent: forward mode (one tangent per parameter carried beside z),
-//     per-pixel ds/dtheta, the independent check of the adjoint.
+//     per-pixel ds/dtheta.
 // Holomorphic steps make both sweeps complex multiplications: the adjoint multiplies by the
 // conjugates of the orbit's derivatives, the tangent by f'(z_k).
 #include "ap_common.cuh"

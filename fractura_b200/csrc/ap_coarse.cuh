@@ -146,9 +146,8 @@ __device__ __forceinline__ int tail_gap(const Store& C, int q, OrbitTail tail, i
 
 // A round of the batch kernel: it lasts until the SM's clock passes `end`, looked at every kRoundCheck
 // loop iterations (`left`, the same for all lanes of a loop), and for the first iterations in any
-// case.  Rounds counted in steps, weighted by formula, lasted as long as their block's dearest warp:
-// 44 % of the warps' time went into waiting for it (21 mixed tiles 33.3 -> 29.2 ms with the clock;
-// looking every 8, 16 or 32 iterations times alike).
+// case.  Rounds counted in steps, weighted by formula, lasted as long as their block's dearest warp
+// (21 mixed tiles 33.3 -> 29.2 ms with the clock; looking every 8, 16 or 32 iterations times alike).
 constexpr int kRoundCheck = 16;
 struct Round {
     int left;

@@ -86,9 +86,9 @@ __global__ void __launch_bounds__(kTile * kTile) render_pass_kernel(const ApFram
 // owns a pixel then adds the pixel's colours up in sample order (sy, then sx), so the sums round as
 // the sequential loop's.  Measured against a pixel per lane: 1280x720 double-double Burning Ship
 // with 2x SSAA 56.6 -> 53.1 ms with one warp a patch.  Its time was then the tail of the patches whose
-// pixels are all selected and bounded (four rounds of 20000 steps one after the other, the SMs 20 %
-// busy); with the rounds on warps of their own 53.7 -> 44.1 ms, and a 1283x721 Julia frame
-// 681 -> 645 us.
+// pixels are all selected and bounded (four rounds of 20000 steps one after the other); with the
+// rounds on warps of their own 53.7 -> 44.1 ms, and a 1283x721 Julia frame 681 -> 645 us.  A pass that
+// selects next to nothing pays for the blocks that find none (1280x720, 25 -> 75 us).
 template <int TIER, int ARITH, int KIND>
 __global__ void __launch_bounds__(32) supersample_kernel(const ApFrameParams p, const ApFrameBuffers b,
                                                          const int hist_resolve, const int share, const int shares) {
