@@ -169,8 +169,8 @@ __device__ __forceinline__ double dd_step_plain(dd& zx, dd& zy, dd cx, dd cy) {
 // taken again from its start by tested steps, which the lanes of a warp do together.  With a test
 // and a branch a step throughout, the chain of a lone warp waited for all four parts of z: a deep frame
 // that leaves most of the GPU idle is bound by it (128x96 Mandelbrot at 1e-18, depth 8500, REF_CUDA:
-// 1559 us with a test a step, 1230 with blocks and a flag, 1117 with the three words; 1217 before the short
-// step), a large one by the FP64 pipe (960x540 20.1 -> 15.5 ms, 16.2 with a test a step; 960x540
+// 1559 us with a test a step, 1230 with blocks and a flag, 1117 with the three words, 1140 with the first
+// 32 steps tested; 1217 before the short step), a large one by the FP64 pipe (960x540 20.1 -> 15.5 ms, 16.2 with a test a step; 960x540
 // Burning Ship at 2e-17, depth 6000, REF_CPU 13.1 -> 7.2 ms, 7.5 with a test a step).  Blocks of 4, 8 and
 // 16 steps: 128x96 1117, 1117 and 1093 us; 599x400 Burning Ship at depth 6000 4246, 3954 and 3981.
 constexpr int kDdBlock = 8, kDdLead = 32;
