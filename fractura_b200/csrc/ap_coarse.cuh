@@ -99,21 +99,20 @@ constexpr int kTailStride = 64;
 constexpr int kFirstRestart = 16;
 
 // The reference's tail: period p (0: none) from step s0 on, as ap_pack_orbit leaves it in the
-// last record's fourth slot (-(4096 s0 + p); no radius is negative, so no leap reads it as one).
+// last record's fourth slot (-(4096 s0 + p); no radius is negative, so no leap reads it as one),
+// where it holds at least two periods and 64 steps.
 struct OrbitTail {
     int p, s0;
 };
-__device__ __forceinline__ double tail_word(const double4* __restrict__ orb, int ref_len) {
-    return -__ldg(reinterpret_cast<const double*>(orb + ref_len) + 3);
+__device__ __forceinline__ OrbitTail orbit_tail(const double4* __restrict__ orb, int ref_len) {
+    const double t = -__ldg(reinterpret_cast<const double*>(orb + ref_len) + 3);
+    if (!(t > 0.0)) return {0, INT_MAX};
+    const int s0 = (int)(t * (1.0 / 4096.0)), p = (int)(t - 4096.0 * (double)s0);
+    if (ref_len - 1 - s0 < max(2 * p, 64)) return {0, INT_MAX};
+    return {p, s0};
 }
 __device__ __forceinline__ bool has_tail(const double4* __restrict__ orb, int ref_len) {
-    return tail_word(orb, ref_len) > 0.0;
-}
-__device__ __forceinline__ OrbitTail orbit_tail(const double4* __restrict__ orb, int ref_len) {
-    const double t = tail_word(orb, ref_len);
-    if (!(t > 0.0)) return {0, INT_MAX};
-    const int s0 = (int)(t * (1.0 / 4096.0));
-    return {(int)(t - 4096.0 * (double)s0), s0};
+    return orbit_tail(orb, ref_len).p > 0;
 }
 
 // A visit of state (x, y) at k iterations and reference index m (0: a restart; else a tail step
