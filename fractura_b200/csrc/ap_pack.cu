@@ -45,18 +45,14 @@ __device__ __forceinline__ unsigned orbit_window(const double* __restrict__ re, 
 // period p <= 4095 with Z_k = Z_{k-p} (bit for bit up to the sign of a zero) for the orbit's last 8 steps,
 // and the s0 from which on it holds for every k from s0 + p to n - 2; kept as -(4096 s0 + p) in the last
 // record (orbit_tail, ap_coarse.cuh, asks for two periods and 64 steps of it), 0 when there is none.  An
-// orbit that escaped has none (its last value tells).  Every block searches the period for itself,
-// all candidates' first values at once, and compares its share of the orbit; the largest s0 is the
-// largest word.  On one block of the packing kernel, candidates and orbit in turn, it held every frame
-// of a bounded reference up: 200000 values 306 us for both kernels, 23 so; 6000 values 17 and 16, without a
-// tail 11 and 12.5 (the second launch).
+// orbit that escaped has none (its last value tells).  One block of a launch of `blocks`: it searches the
+// period for itself, all candidates' first values at once, compares its share of the orbit and returns
+// the word of that (the largest s0 of all shares is the largest word), the same in all its threads.
 constexpr int kTailThreads = 256, kTailMaxPeriod = 4095;
-__global__ void __launch_bounds__(kTailThreads) pack_tail_kernel(const double* __restrict__ re,
-                                                                 const double* __restrict__ im, int n,
-                                                                 double4* __restrict__ out) {
+__device__ double tail_word(const double* __restrict__ re, const double* __restrict__ im, int n, int block, int blocks) {
     __shared__ int period_s, bad_s;
     const int last = n - 2;  // the record at n - 1 is the orbit's end, never a step
-    if (last < 128 || !(re[n - 1] * re[n - 1] + im[n - 1] * im[n - 1] <= kBailout)) return;
+    if (last < 128 || !(re[n - 1] * re[n - 1] + im[n - 1] * im[n - 1] <= kBailout)) return 0.0;
     const int t = threadIdx.x;
     if (t == 0) {
         period_s = kTailMaxPeriod + 1;
@@ -82,24 +78,36 @@ __global__ void __launch_bounds__(kTailThreads) pack_tail_kernel(const double* _
     }
     __syncthreads();
     const int p = period_s;
-    if (p > kTailMaxPeriod) return;
+    if (p > kTailMaxPeriod) return 0.0;
     int bad = -1;  // the largest k of this block's share with Z_k != Z_{k-p}
 #pragma unroll 4
-    for (long long k = (long long)p + blockIdx.x * kTailThreads + t; k <= last; k += gridDim.x * kTailThreads)
+    for (long long k = (long long)p + block * kTailThreads + t; k <= last; k += blocks * kTailThreads)
         if (!(re[k] == re[k - p] && im[k] == im[k - p])) bad = (int)k;
     if (bad >= 0) atomicMax(&bad_s, bad);
     __syncthreads();
-    if (t == 0) {
-        const int s0 = bad_s < 0 ? 0 : bad_s + 1 - p;
-        const double word = -(4096.0 * (double)s0 + (double)p);  // negative: the bits order by magnitude
+    const int s0 = bad_s < 0 ? 0 : bad_s + 1 - p;
+    return -(4096.0 * (double)s0 + (double)p);
+}
+
+// Long orbits (from kLongOrbit values): shared out over the blocks of a kernel of its own.  On one block of
+// the packing kernel 200000 values held every frame of a bounded reference up for 306 us (23 so), 16000
+// for 19 (19 so); a short orbit would pay for the second launch (6000 values without a tail 9 us, 12.5
+// with it; 8050 of an escaped one 6.4 and 8).
+constexpr int kLongOrbit = 1 << 14;
+__global__ void __launch_bounds__(kTailThreads) pack_tail_kernel(const double* __restrict__ re,
+                                                                 const double* __restrict__ im, int n,
+                                                                 double4* __restrict__ out) {
+    const double word = tail_word(re, im, n, blockIdx.x, gridDim.x);
+    if (threadIdx.x == 0 && word < 0.0)  // negative: the bits order by magnitude
         atomicMax(reinterpret_cast<unsigned long long*>(&out[n - 1].w), (unsigned long long)__double_as_longlong(word));
-    }
 }
 
 __global__ void __launch_bounds__(256) pack_orbit_kernel(const double* __restrict__ re,
                                                          const double* __restrict__ im, int n,
                                                          double4* __restrict__ out) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    // a short orbit's tail: the last block, which writes the last record
+    const double tail = n < kLongOrbit && blockIdx.x == gridDim.x - 1 ? tail_word(re, im, n, 0, 1) : 0.0;
     if (k >= n) return;
     const double rx = re[k], ry = im[k];
     const double r_mag2 = rx * rx + ry * ry;
@@ -117,8 +125,8 @@ __global__ void __launch_bounds__(256) pack_orbit_kernel(const double* __restric
     const int safe_hi = __double2hiint(s * s * (1.0 - 1e-12)) - 1;
     const double safe = safe_hi > 0 ? __hiloint2double(safe_hi, (int)orbit_window(re, im, k, n)) : 0.0;
     // slot 3: the level-0 BLA radius, written by ap_pack_bla (0: no leap); in the last record,
-    // which no leap starts from, the periodic tail, written by pack_tail_kernel (0: none)
-    out[k] = make_double4(rx, ry, safe, 0.0);
+    // which no leap starts from, the periodic tail (a long orbit's: by pack_tail_kernel)
+    out[k] = make_double4(rx, ry, safe, k == n - 1 ? tail : 0.0);
 }
 
 __global__ void __launch_bounds__(256) pack_bla_kernel(const double* __restrict__ T, int levels,
@@ -153,7 +161,7 @@ extern "C" int ap_pack_orbit(const double* ref_re, const double* ref_im, int32_t
     ap::pack_orbit_kernel<<<(n + 255) / 256, 256, 0, static_cast<cudaStream_t>(stream)>>>(
         ref_re, ref_im, n, reinterpret_cast<double4*>(out));
     const int rc = ap::check_launch("pack_orbit_kernel");
-    if (rc != AP_OK || n < 130) return rc;  // a tail has 64 steps at least, in an orbit of 130 values
+    if (rc != AP_OK || n < ap::kLongOrbit) return rc;
     const int blocks = (n + 2047) / 2048 < 148 ? (n + 2047) / 2048 : 148;
     ap::pack_tail_kernel<<<blocks, ap::kTailThreads, 0, static_cast<cudaStream_t>(stream)>>>(
         ref_re, ref_im, n, reinterpret_cast<double4*>(out));

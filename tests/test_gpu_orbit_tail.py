@@ -41,7 +41,7 @@ def _packed(re, im):
 
 @pytest.mark.parametrize("p,s0,n", [(1, 0, 130), (1, 60, 130), (1, 100, 400), (2, 17, 131), (3, 0, 2049), (64, 1000, 2305), (255, 7, 4097),
                                     (256, 300, 5000), (257, 2100, 9000), (4095, 0, 8193), (4095, 1, 8194), (4095, 2000, 20001),
-                                    (4096, 0, 20000), (12, 250000, 303105), (12, 303000, 303105)])
+                                    (4096, 0, 20000), (12, 5000, 16383), (12, 5000, 16384), (12, 250000, 303105), (12, 303000, 303105)])
 def test_tail_is_found(p, s0, n):
     rng = np.random.default_rng(p + s0 + n)
     re, im = rng.uniform(-1, 1, n), rng.uniform(-1, 1, n)
